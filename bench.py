@@ -102,16 +102,9 @@ def make_workload(name: str):
 # The mixed path's level-0 kernels read one coefficient-code byte per cell in
 # place of the diagonal and the three coefficient arrays.
 def kernel_bytes(name: str, w: int):
-    coded = w == 4
     table = {
         "k_advect": 18 * w + 1 + 10 * w,        # 10 scalars + u,v,w + fx,fy,fz + Pb,nu + blocked -> 10 scalars
         "k_momentum": 9 * w,                    # vel, 2 other components, fo, Pb, T, nu, p -> vel' (per face)
-        "k_gs_pre": 2 * w + 1 if coded else 6 * w,                 # r, code (diag, 3 coefficients) -> z
-        "k_gs_black": 3 * w + 4 + 1 if coded else 6.5 * w + 4,     # r, z, agg, code -> z (black)
-        "k_gs_red_dot": 3 * w + 1 if coded else 6.5 * w,           # r, z, code -> z (red), r.z
-        "k_cg_apply": 4 * w + 1 if coded else 8 * w,               # z, d, code -> d, q
-        "k_cg_update": 7 * w,                   # p, d, r, q, diag -> p, r
-        "k_res_restrict": 2 * w + 4 + 1 if coded else 6 * w + 4,   # r, z, agg, code -> level-1 b
         "k_rhs": 13 * w + 1,
         "k_heat": 8 * w + 1,
         "k_energy": 6 * w + 1,
@@ -121,44 +114,26 @@ def kernel_bytes(name: str, w: int):
         "k_turb_nu": 5 * w + 1,
         "k_velcorr": 5 * w,
         "k_stats": 4 * w + 1,
-        "k_mx_res64": 8 + 3 * w + 1,            # p64, b, code -> r, e
-        "k_mx_update": 8 + 8 + 2 * w,
     }
     return table.get(name)
 
 
-# DRAM bytes (read + write) per cell of each level-0 kernel, measured by ncu
-# (dram__bytes_read.sum + dram__bytes_write.sum of the first full-batch launch
-# on the 64-scenario batch, mixed path, divided by its 7,964,799 cells)
-NCU_BYTES_PER_CELL = {"k_gs_pre": 22.7, "k_res_restrict": 30.0, "k_gs_black": 32.3, "k_gs_red_dot": 26.8,
-                      "k_cg_apply": 25.6, "k_cg_update": 23.5, "k_mx_res64": 34.5}
-
-
-def jacobi_step_bytes(levels, iters, w: int) -> float:
-    """Algorithmic bytes of one step's coarse-level damped Jacobi sweeps
-    (k_jacobi): every scenario runs it + 1 V-cycles, each with three sweeps of
-    each level 1..L-2 (one on the way down -- the from-zero sweep is fused into
-    the restriction -- and two on the way up); a sweep of a level with n rows
-    and nnz stored off-diagonal entries reads diag, b, the input vector and
-    rowStart per row and col and val per entry and writes one value per row
-    (4w + 4 per row, 4 + w per entry); the prolongating sweep also reads agg."""
+def solve_bytes(levels, iters, w: int) -> float:
+    """Algorithmic bytes of one step's pressure solve (k_solve), the arrays its
+    passes cannot do without: per cell and CG iteration the direction update with
+    q = A d (z, half of r, d, q -> d, q) and the update (p, d, q, r -> p, r, half
+    of z); per cell and V-cycle, it + 1 of them, the four half sweeps and the
+    residual, each over one colour; and the coarse levels: per V-cycle three
+    sweeps and a restriction of each level 1..L-2 with n rows and nnz couplings
+    (their couplings are kept on chip, so only b, x and y move) and the dense
+    coarsest operator."""
     total = 0.0
     for (rows, nnz), it in zip(levels, iters):
-        per_cycle = sum(rows[l] * (12 * w + 16) + 3 * (4 + w) * nnz[l] for l in range(1, len(rows) - 1))
-        total += (it + 1) * per_cycle
+        n = rows[0]
+        per_iter = n * (12 * w + 1)
+        per_cycle = n * (6.25 * w + 8.5) + sum(10 * w * r for r in rows[1:-1]) + rows[-1] ** 2 * w
+        total += it * per_iter + (it + 1) * per_cycle
     return total
-
-
-def launched_cells(name: str, launches: int, iters, sizes) -> int:
-    """Cells processed by all launches of one kernel in one step. A scenario
-    that stopped after it CG iterations took part in it launches of q = A d and
-    of the update, and in it + 1 V-cycles (level-0 sweeps and residual);
-    every other kernel runs over every cell at each launch."""
-    if name in ("k_cg_apply", "k_cg_update"):
-        return sum(i * n for i, n in zip(iters, sizes))
-    if name in ("k_gs_pre", "k_gs_black", "k_gs_red_dot", "k_res_restrict"):
-        return sum((i + 1) * n for i, n in zip(iters, sizes))
-    return launches * sum(sizes)
 
 
 def measured_peak():
@@ -474,34 +449,23 @@ def measure(args, precision, L, world, clocks: bool):
     prof_iters = [g.stats(s)["pressure_iters"] for s in range(len(cases))]
     tot_prof = sum(p[2] for p in prof)
     w = 8 if precision == _lib.PREC_FP64 else 4
-    # the dominant kernel of the step; the coarse-level Jacobi sweeps are
-    # modelled per multigrid row, the other kernels per cell
-    modelled = [p for p in prof if kernel_bytes(p[0], w) or p[0] == "k_jacobi"]
+    # the dominant kernel of the step: the pressure solve by its own model, the
+    # others by bytes per cell
+    modelled = [p for p in prof if kernel_bytes(p[0], w) or p[0] == "k_solve"]
     top = max(modelled or prof, key=lambda p: p[2])
     per_unit = kernel_bytes(top[0], w)
     peak, peak_kind = measured_peak()
     roof = None
-    if top[0] == "k_jacobi":
-        levels = [(g.mg_levels(s), g.mg_nnz(s)) for s in range(len(cases))]
-        total = jacobi_step_bytes(levels, prof_iters, w)
-        bytes_per_launch = total / top[1]
-        achieved = bytes_per_launch / (top[2] / top[1] / 1e3) / 1e9
+    total = None
+    if top[0] == "k_solve":
+        total = solve_bytes([(g.mg_levels(s), g.mg_nnz(s)) for s in range(len(cases))], prof_iters, w)
+    elif per_unit:
+        total = per_unit * top[1] * cells
+    if total:
+        achieved = total / (top[2] / 1e3) / 1e9
         roof = {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak,
                 "traffic": None, "kernel": top[0], "kernel_share": top[2] / tot_prof,
-                "algorithmic_bytes_per_launch": bytes_per_launch, "peak_kind": peak_kind,
-                "model": "per V-cycle and level 1..L-2: rows (12w + 16) + 3 (4 + w) nnz (three sweeps)"}
-    elif per_unit:
-        # cells the kernel's launches of the profiled step processed: the CG
-        # kernels skip scenarios that have stopped iterating
-        units = launched_cells(top[0], top[1], prof_iters, [c.N for c in cases])
-        bytes_per_launch = per_unit * units / top[1]
-        achieved = bytes_per_launch / (top[2] / top[1] / 1e3) / 1e9
-        traffic = None
-        if precision == _lib.PREC_MIXED and top[0] in NCU_BYTES_PER_CELL and args.workload == "batch64":
-            traffic = NCU_BYTES_PER_CELL[top[0]] * units / top[1]
-        roof = {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak,
-                "traffic": traffic, "kernel": top[0], "kernel_share": top[2] / tot_prof,
-                "algorithmic_bytes_per_launch": bytes_per_launch, "peak_kind": peak_kind}
+                "algorithmic_bytes_per_launch": total / top[1], "peak_kind": peak_kind}
     g.close()
     sm = sorted(step_ms)
     pct = lambda q: sm[min(len(sm) - 1, int(round(q * (len(sm) - 1))))]

@@ -2,8 +2,8 @@
 // the domain tables of the launches and the launch sequence of the gas-phase
 // step (src/sim/solver.cpp:226-269). A single-scenario context is a batch of
 // one. Every kernel launch covers one domain (cells, faces of one axis, one
-// multigrid level, ...) of every scenario; the whole step is captured once as
-// a CUDA graph whose pressure-solve loops are device-side while nodes.
+// kind of boundary, ...) of every scenario; the pressure solve is one cooperative
+// launch (solve.cuh), and the whole step is captured once as a CUDA graph.
 // Instantiated per precision by engine_fp64.cu and engine_mixed.cu.
 #pragma once
 #include <array>
@@ -23,8 +23,8 @@
 #include "mixed_kernels.cuh"
 #include "radiation.cuh"
 #include "volume.cuh"
-#include "rowblock.cuh"
-#include "level0.cuh"
+#include "selftest.cuh"
+#include "solve.cuh"
 
 namespace phx {
 
@@ -41,14 +41,11 @@ namespace phx {
 // dense coarse operators up to this many unknowns (n^2 reals)
 constexpr int DENSE_MAX = 4096;
 
-enum DomId {
-    D_ONE = 0, D_CELLS, D_FX, D_FY, D_FZ, D_BX, D_BY, D_BZ, D_CZ, D_CC, D_CO_DENSE, D_CO_SERIAL, D_RB, D_QUAD, D_LEAK,
-    D_L0,                        // level-0 tiles of the mixed path: 2x2x2 blocks (level0.cuh)
-    D_L0R,                       // the same, several blocks per thread (the passes with a dot product)
-    D_LV0,                       // D_LV0 + l: rows of level l when l is not the coarsest (1 <= l < 12)
-    D_RS0 = D_LV0 + MAX_LEVELS,  // D_RS0 + l: rows of level l+1 for restriction from level l >= 1
-    D_COUNT = D_RS0 + MAX_LEVELS
-};
+enum DomId { D_ONE = 0, D_CELLS, D_FX, D_FY, D_FZ, D_BX, D_BY, D_BZ, D_CZ, D_CC, D_LEAK, D_COUNT };
+
+// widest rows the contexts take (nx); wider grids are refused
+template <class R>
+constexpr int maxRow() { return sizeof(R) == 8 ? 410 : 776; }
 
 template <class T>
 static T* carve(char*& base, size_t& off, size_t n) {
@@ -104,7 +101,6 @@ struct Scenario {
     size_t arenaBytes = 0;       // both arenas
     size_t mainBytes = 0, mgBytes = 0;
     Scn<R> h{};                  // host copy of the device descriptor
-    R* dbuf[2] = {nullptr, nullptr};
     std::string err;
 
     ~Scenario() {
@@ -136,10 +132,8 @@ struct Scenario {
         for (auto v : geo.lx) geo.anyLeak |= v != 0;
         for (auto v : geo.ly) geo.anyLeak |= v != 0;
         for (auto v : geo.lz) geo.anyLeak |= v != 0;
-        RbShapes<R> one;
-        one.add(g->nx, g->ny);
-        if (!one.finish()) {
-            err = "grid rows too long for the shared-memory tiles of the pressure kernels (nx = " + std::to_string(g->nx) + ")";
+        if (g->nx > maxRow<R>()) {
+            err = "grid rows too long for the pressure kernels (nx = " + std::to_string(g->nx) + ")";
             return PHX_ERR_UNSUPPORTED;
         }
         cfl = g->cfl; dtMaxP = g->dt_max; tol = g->tol; relTol = g->rel_tol; maxIters = g->max_iters;
@@ -203,12 +197,9 @@ struct Scenario {
 
     size_t layoutMain(char* base) {
         const int N = geo.N(), NX = geo.NX(), NY = geo.NY(), NZ = geo.NZ();
-        const int nl = (int)MG.lv.size();
-        // one reduction partial per CTA of the widest reduction domain (cells,
-        // row-block tiles, level-0 tiles)
-        int tl[D_COUNT];
-        tiles(tl);
-        const int partStride = std::max(tl[D_CELLS], std::max(tl[D_RB], tl[D_L0])) + 1;
+        // one reduction partial per CTA of the cell domain and per tile of the solve
+        const int nblk = ((geo.nx + 1) >> 1) * ((geo.ny + 1) >> 1) * ((geo.nz + 1) >> 1);
+        const int partStride = std::max((N + TPB - 1) / TPB, solveTiling<R>(nblk).nt) + 1;
         size_t off = 0;
         Scn<R>& s = h;
         s.blocked = carve<uint8_t>(base, off, N);
@@ -248,9 +239,7 @@ struct Scenario {
         for (int q = 0; q < 9; ++q) s.tmp[q] = carve<R>(base, off, N);
         s.adv = kMixed ? nullptr : carve<double>(base, off, (size_t)ADV_REC * (NX + NY + NZ));
         s.b = carve<R>(base, off, N); s.r = carve<R>(base, off, N); s.z = carve<R>(base, off, N);
-        dbuf[0] = carve<R>(base, off, N); dbuf[1] = carve<R>(base, off, N);
-        s.d = dbuf[0];
-        s.q = carve<R>(base, off, N);
+        s.d = carve<R>(base, off, N); s.q = carve<R>(base, off, N);
         s.p64 = kMixed ? carve<double>(base, off, N) : nullptr;
         s.p64prev = kMixed ? carve<double>(base, off, N) : nullptr;
         Level<R>& L0 = s.lv[0];
@@ -262,6 +251,7 @@ struct Scenario {
         s.part = carve<double>(base, off, (size_t)PS_COUNT * partStride);
         s.partStride = partStride;
         s.cnt = carve<unsigned>(base, off, PS_COUNT + 4);
+        s.teamBar = carve<unsigned>(base, off, 64);
         return off + 256;
     }
 
@@ -297,6 +287,7 @@ struct Scenario {
                 D.col = carve<int>(base, off, L.col.size() + 1);
                 D.val = carve<R>(base, off, L.val.size() + 1);
                 D.diag = carve<R>(base, off, L.n + 1);
+                D.omd = carve<R>(base, off, L.n + 1);
                 D.x = carve<R>(base, off, L.n + 1); D.y = carve<R>(base, off, L.n + 1); D.b = carve<R>(base, off, L.n + 1);
             }
             D.agg = L.agg.empty() ? nullptr : carve<int>(base, off, L.agg.size());
@@ -400,10 +391,6 @@ struct Scenario {
             s.replaceEvery = every;
         }
         s.extrap = std::getenv("PHX_NO_EXTRAP") == nullptr;   // mixed path: extrapolated initial guess
-        s.fp16Scratch = kMixed && std::getenv("PHX_FP16_SCRATCH") != nullptr;
-        s.fp16Z0 = kMixed && std::getenv("PHX_FP16_Z0") != nullptr;
-        s.tj = rowBlockRows<R>(geo.nx, geo.ny);
-        s.njb = (geo.ny + s.tj - 1) / s.tj;
         PHX_TRY(putRaw(st, s.blocked, geo.blocked.data(), N));
         PHX_TRY(put(st, s.fx, geo.fx)); PHX_TRY(put(st, s.fy, geo.fy)); PHX_TRY(put(st, s.fz, geo.fz));
         PHX_TRY(put(st, s.ax, geo.ax)); PHX_TRY(put(st, s.ay, geo.ay)); PHX_TRY(put(st, s.az, geo.az));
@@ -448,6 +435,9 @@ struct Scenario {
             PHX_TRY(putRaw(st, D.col, L.col.data(), L.col.size()));
             PHX_TRY(put(st, D.val, L.val));
             PHX_TRY(put(st, D.diag, L.diag));
+            std::vector<double> omd(L.n);
+            for (int I = 0; I < L.n; ++I) omd[I] = L.diag[I] > 0 ? OMEGA / L.diag[I] : 0.0;
+            PHX_TRY(put(st, D.omd, omd));
         }
         for (int l = 0; l < (int)MG.lv.size(); ++l) {
             const MgLevel& L = MG.lv[l];
@@ -504,10 +494,6 @@ struct Scenario {
         for (int d = 0; d < D_COUNT; ++d) t[d] = 0;
         t[D_ONE] = 1;
         t[D_CELLS] = cdiv(N, TPB);
-        t[D_RB] = cdiv(ny, rowBlockRows<R>(nx, ny)) * cdiv(nz, RB_KZ);      // row blocks x plane blocks
-        t[D_L0] = l0Tiles(nx, ny, nz, 1);
-        t[D_L0R] = l0Tiles(nx, ny, nz, l0Bpt(L0_RED));
-        t[D_QUAD] = cdiv(N, TPB * CG_QUAD);                                 // 4 cells per thread
         t[D_LEAK] = cdiv((long long)leak.size() / 4, TPB);
         t[D_FX] = cdiv(geo.NX(), TPB);
         t[D_FY] = cdiv(geo.NY(), TPB);
@@ -517,14 +503,6 @@ struct Scenario {
         t[D_BZ] = cdiv((long long)nx * ny, TPB);
         t[D_CZ] = (int)Z.closed.size();
         t[D_CC] = cdiv((long long)Z.closedCells.size(), TPB);
-        const int nl = (int)MG.lv.size();
-        const MgLevel& Lc = MG.lv[nl - 1];
-        t[D_CO_DENSE] = Lc.dense.empty() ? 0 : cdiv(Lc.n, TPB / 32);
-        t[D_CO_SERIAL] = Lc.dense.empty() ? 1 : 0;
-        for (int l = 1; l < MAX_LEVELS; ++l) {
-            t[D_LV0 + l] = (l < nl - 1) ? cdiv(MG.lv[l].n, TPB) : 0;
-            t[D_RS0 + l] = (l + 1 <= nl - 1) ? cdiv(MG.lv[l + 1].n, TPB / RRJ_LANES) : 0;   // 8 lanes per unknown
-        }
     }
 };
 
@@ -541,37 +519,17 @@ public:
     int cap = 0;                 // scenario capacity of the tables
     char* tab = nullptr;
     Scn<R>* dS = nullptr;        // descriptors
-    R** dD = nullptr;            // CG direction buffers, 2 per scenario
     int* dDomStart = nullptr;    // D_COUNT x (cap + 1)
     double* dDtMax = nullptr;    // per-scenario dtMax of the step
-    int* dLoop = nullptr;        // [0] iterations of the graph's CG while node, [1] runs of its replacement node
-    int* dTiles = nullptr;       // [D_COUNT][cap] tiles of each scenario per domain
-    int* dAStart = nullptr;      // [2][D_COUNT][cap + 1] active-tile prefixes (solving / replacing)
-    int* dATotal = nullptr;      // [2][D_COUNT]
     unsigned* dErr = nullptr;    // error word of the device side (bounded waits that ran out)
     unsigned* ownTab = nullptr;  // CTA -> (scenario, tile) of every domain (Dom::owner)
     size_t ownCap = 0;
     double* dTimes = nullptr;    // simulated time of each scenario (read-back staging)
-    int* dAllTotal = nullptr;    // the row-block tile total of the batch (every tile active), for tuning runs
-    // launch shape of a row-block kernel: dynamic shared memory, persistent grid, slot strides
-    struct RbCfg {
-        size_t smem = 0;
-        int grid = 0;
-        RbShape shape{0, 0, 0};
-    };
-    RbCfg cfgApply, cfgGs[3], cfgRes;
-    // the coded-coefficient level-0 kernels (level0.cuh) and their launch shape;
-    // PHX_L0_ROWBLOCK=1 runs level 0 on the row-block kernels instead
-    const bool l0Requested = std::getenv("PHX_L0_ROWBLOCK") == nullptr;
-    bool useL0 = false;
+    double* dMaxPart = nullptr;  // k_solve: two maxima per CTA
+    int solveGrid = 0;           // k_solve: CTAs resident at once
     bool smoothOne = false;            // mixed path: one Jacobi sweep per coarse level and leg (vcycleSweeps)
-    bool l0RedWide = false;            // the red sweep with L0_RED_WIDE blocks per thread
-    int l0grid[L0_MODES + 1] = {};     // per pass; [L0_MODES]: the wide red sweep
-    ADom adom[2][D_COUNT];
     double* hPin = nullptr;      // pinned scratch for read-backs
     Dom dom[D_COUNT];
-    int maxLevels = 0;
-    bool anyClosed = false;
     bool anyLeak = false;
     bool tablesDirty = true;
     int launches = 0;
@@ -1015,16 +973,11 @@ public:
             for (int pass = 0; pass < 2; ++pass) {
                 size_t off = 0;
                 dS = carve<Scn<R>>(base, off, cap);
-                dD = carve<R*>(base, off, 2 * cap);
                 dDomStart = carve<int>(base, off, (size_t)D_COUNT * (cap + 1));
                 dDtMax = carve<double>(base, off, cap);
-                dLoop = carve<int>(base, off, 4);
-                dTiles = carve<int>(base, off, (size_t)D_COUNT * cap);
-                dAStart = carve<int>(base, off, (size_t)2 * D_COUNT * (cap + 1));
-                dATotal = carve<int>(base, off, 2 * D_COUNT);
                 dErr = carve<unsigned>(base, off, 4);
                 dTimes = carve<double>(base, off, cap);
-                dAllTotal = carve<int>(base, off, 4);
+                dMaxPart = carve<double>(base, off, 2 * MAX_SOLVE_CTAS);
                 if (pass == 0) {
                     cudaError_t e = cudaMalloc(&tab, off + 256);
                     if (e != cudaSuccess) { tab = nullptr; err = "device allocation of the batch tables failed"; return PHX_ERR_OOM; }
@@ -1035,15 +988,11 @@ public:
         }
         std::vector<int> starts((size_t)D_COUNT * (n + 1), 0);
         std::vector<int> tilesAll((size_t)D_COUNT * cap, 0);
-        std::vector<R*> dd(2 * std::max(n, 1), nullptr);
-        maxLevels = 0;
-        anyClosed = false;
         anyLeak = false;
         {
             std::lock_guard<std::mutex> lock(vcycleMutex());
             smoothOne = kMixed && vcycleSweeps() == 1;
         }
-        RbShapes<R> shp;
         int t[D_COUNT];
         for (int s = 0; s < n; ++s) {
             Scenario<R>& S = *sc[s];
@@ -1052,15 +1001,10 @@ public:
                 starts[(size_t)d * (n + 1) + s + 1] = starts[(size_t)d * (n + 1) + s] + t[d];
                 tilesAll[(size_t)d * cap + s] = t[d];
             }
-            dd[2 * s] = S.dbuf[0];
-            dd[2 * s + 1] = S.dbuf[1];
-            maxLevels = std::max(maxLevels, (int)S.MG.lv.size());
-            anyClosed |= !S.Z.closed.empty();
             anyLeak |= !S.leak.empty();
             S.h.dtMaxArg = dDtMax + s;
             S.h.errWord = dErr;
             S.h.smooth1 = smoothOne ? 1 : 0;
-            shp.add(S.geo.nx, S.geo.ny);
         }
         // per domain, the scenario and tile of every CTA (packed 11 + 20 bits)
         size_t ownTotal = 0;
@@ -1095,219 +1039,25 @@ public:
             dom[d].owner = own.empty() ? nullptr : ownTab + ownOff;
             ownOff += (size_t)dom[d].total;
         }
-        for (int k = 0; k < 2; ++k)
-            for (int d = 0; d < D_COUNT; ++d) {
-                adom[k][d].start = dAStart + (size_t)(k * D_COUNT + d) * (cap + 1);
-                adom[k][d].total = dATotal + k * D_COUNT + d;
-                adom[k][d].nscn = n;
-            }
-        persistCtas = PERSIST_CTAS;
-        if (const char* cap = std::getenv("PHX_PERSIST_CTAS")) persistCtas = std::max(1, std::min(persistCtas, std::atoi(cap)));
-        if (n > 0) {
-            if (!shp.finish()) {
-                err = "the batch's widest grids need more shared memory than a CTA has";
-                return PHX_ERR_UNSUPPORTED;
-            }
-        }
         PHX_CK(cudaMemcpyAsync(dDomStart, starts.data(), starts.size() * sizeof(int), cudaMemcpyHostToDevice, st));
-        PHX_CK(cudaMemcpyAsync(dTiles, tilesAll.data(), tilesAll.size() * sizeof(int), cudaMemcpyHostToDevice, st));
-        if (n > 0) PHX_CK(cudaMemcpyAsync(dD, dd.data(), 2 * n * sizeof(R*), cudaMemcpyHostToDevice, st));
         tablesDirty = false;
         for (int s = 0; s < n; ++s) PHX_TRY(pushDescriptor(s, false));
-        const int allTotal = dom[D_RB].total;
-        PHX_CK(cudaMemcpyAsync(dAllTotal, &allTotal, sizeof(int), cudaMemcpyHostToDevice, st));
         PHX_CK(cudaStreamSynchronize(st));
-        if (n > 0) PHX_TRY(tuneRowBlocks(shp));
-        useL0 = false;
-        if (n > 0 && l0Requested) PHX_TRY(setupL0());
-        return PHX_OK;
+        return n > 0 ? setupSolve() : PHX_OK;
     }
 
-    // launch shape of the level-0 kernels: a persistent grid of as many CTAs
-    // as fit on the SMs
-    int setupL0() {
-        int dev = 0, sms = 0;
+    // the solve kernel's grid: every CTA resident, since its teams wait on one
+    // another. PHX_PERSIST_CTAS caps it (tests: several scenarios per CTA)
+    static constexpr int MAX_SOLVE_CTAS = 1024;
+    int setupSolve() {
+        int dev = 0, sms = 0, occ = 0;
         PHX_CK(cudaGetDevice(&dev));
         PHX_CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-        // Grid per pass: k times the resident CTAs, or (k = 0) one CTA per tile.
-        // q = A d and the red sweep end every tile with a reduction of d.q or
-        // r.z; one CTA per tile lets the SM overlap those of different tiles,
-        // which a persistent CTA runs one after the other (mixed batch of 64:
-        // 443 to 452 M cell-updates/s). The smoothing passes have no reduction
-        // and run one persistent wave. PHX_L0_WAVES="k0,k1,k2,k3,k4" (in pass
-        // order; one value sets all five) overrides this for measurements.
-        static const std::array<int, L0_MODES> waves = [] {
-            std::array<int, L0_MODES> w = {0, 1, 1, 1, 0};
-            if (const char* e = std::getenv("PHX_L0_WAVES")) {
-                int v[L0_MODES], n = 0;
-                for (const char* c = e; *c && n < L0_MODES;) {
-                    v[n++] = std::max(0, std::atoi(c));
-                    while (*c && *c != ',') ++c;
-                    if (*c == ',') ++c;
-                }
-                if (n > 0) for (int m = 0; m < L0_MODES; ++m) w[m] = v[n == 1 ? 0 : std::min(m, n - 1)];
-            }
-            return w;
-        }();
-        int residentWide = 0;   // CTAs of the four-block red sweep resident on the GPU at once
-        auto one = [&](auto kern, int mode) -> int {
-            int occ = 0;
-            PHX_CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kern, L0_THREADS, 0));
-            const int k = waves[std::min(mode, L0_MODES - 1)];
-            const int cap = persistCtas * TPB / L0_THREADS;   // PHX_PERSIST_CTAS caps every shape
-            const int resident = std::min(sms * std::max(occ, 1), cap);
-            if (mode == L0_MODES) residentWide = resident;
-            l0grid[mode] = k == 0 ? (persistCtas < PERSIST_CTAS ? cap : (1 << 30)) : resident * k;
-            return PHX_OK;
-        };
-        PHX_TRY(one(k_l0<R, L0_APPLY, 1>, L0_APPLY));
-        PHX_TRY(one(k_l0<R, L0_PRE, 1>, L0_PRE));
-        PHX_TRY(one(k_l0<R, L0_RES, 1>, L0_RES));
-        PHX_TRY(one(k_l0<R, L0_BLACK, 1>, L0_BLACK));
-        PHX_TRY(one(k_l0<R, L0_RED, 1>, L0_RED));
-        PHX_TRY(one(k_l0<R, L0_RED, L0_RED_WIDE>, L0_MODES));
-        // several blocks per thread only where the batch's wide tiles still fill
-        // every CTA slot of the GPU twice (PHX_L0_RED_WIDE=0|1 forces it)
-        static const int redWide = [] {
-            const char* e = std::getenv("PHX_L0_RED_WIDE");
-            return e ? std::atoi(e) : -1;
-        }();
-        l0RedWide = redWide >= 0 ? redWide == 1 : (long long)dom[D_L0R].total >= 2LL * residentWide;
-        useL0 = true;
-        return PHX_OK;
-    }
-
-    // a level-0 pass over the active level-0 tiles
-    template <int MODE>
-    void launchL0(const char* name, int phase) {
-        if constexpr (MODE == L0_RED) {
-            if (l0RedWide) {
-                launchL0k<MODE, L0_RED_WIDE>(name, phase, D_L0R, l0grid[L0_MODES]);
-                return;
-            }
-        }
-        launchL0k<MODE, 1>(name, phase, D_L0, l0grid[MODE]);
-    }
-    template <int MODE, int BPT>
-    void launchL0k(const char* name, int phase, int d, int gridCap) {
-        {
-            if (dom[d].total <= 0) return;
-            const int grid = std::min(dom[d].total, gridCap);
-            const Scn<R>* S = dS;
-            R* const* D = (R* const*)dD;
-            if (prof) {
-                if (evNext + 2 > (int)evPool.size()) {
-                    for (int i = 0; i < 64; ++i) { cudaEvent_t e; cudaEventCreate(&e); evPool.push_back(e); }
-                }
-                cudaEventRecord(evPool[evNext], st);
-                k_l0<R, MODE, BPT><<<grid, L0_THREADS, 0, st>>>(S, adom[0][d], D, phase);
-                cudaEventRecord(evPool[evNext + 1], st);
-                evUse.push_back({name, evNext});
-                evNext += 2;
-            } else {
-                k_l0<R, MODE, BPT><<<grid, L0_THREADS, 0, st>>>(S, adom[0][d], D, phase);
-            }
-            ++launches;
-        }
-    }
-
-    // ---- launch shapes of the row-block kernels -----------------------------------------
-    // The slot count of each kernel's staging ring (and with it how many CTAs
-    // share an SM) is tuned on the batch itself: every candidate that fits an
-    // SM's shared memory is timed on all tiles of the batch (the kernels only
-    // write scratch that the next projection recomputes), and the fastest is
-    // kept, cached per kernel and slot shape. The results do not depend on the
-    // choice. PHX_NO_AUTOTUNE=1 takes the first candidate that fits two CTAs
-    // per SM instead.
-    std::map<std::string, int> tuneCache;
-    int tuneRowBlocks(const RbShapes<R>& shp) {
-        const Scn<R>* S = dS;
-        const ADom all{dom[D_RB].start, dAllTotal, nscn()};
-        PHX_TRY(tuneRB("apply", cfgApply, k_cg_apply_rb<R>, shp.apply, 0, ApplyLayout<R>::MIN_ST,
-                       [&](const RbShape& sh, size_t smem, int grid) {
-                           k_cg_apply_rb<R><<<grid, RB_THREADS, smem, st>>>(S, all, (R* const*)dD, sh);
-                       }));
-        PHX_TRY(tuneRB("gs_pre", cfgGs[GS_PRE], k_gs_rb<R, GS_PRE>, shp.gs[GS_PRE], 0, GsLayout<R, GS_PRE>::MIN_ST,
-                       [&](const RbShape& sh, size_t smem, int grid) {
-                           k_gs_rb<R, GS_PRE><<<grid, RB_THREADS, smem, st>>>(S, all, sh, 2);
-                       }));
-        PHX_TRY(tuneRB("gs_black", cfgGs[GS_BLACK], k_gs_rb<R, GS_BLACK>, shp.gs[GS_BLACK], 0,
-                       GsLayout<R, GS_BLACK>::MIN_ST, [&](const RbShape& sh, size_t smem, int grid) {
-                           k_gs_rb<R, GS_BLACK><<<grid, RB_THREADS, smem, st>>>(S, all, sh, 2);
-                       }));
-        PHX_TRY(tuneRB("gs_red", cfgGs[GS_RED], k_gs_rb<R, GS_RED>, shp.gs[GS_RED], 0, GsLayout<R, GS_RED>::MIN_ST,
-                       [&](const RbShape& sh, size_t smem, int grid) {
-                           k_gs_rb<R, GS_RED><<<grid, RB_THREADS, smem, st>>>(S, all, sh, 2);
-                       }));
-        PHX_TRY(tuneRB("res", cfgRes, k_res_rb<R>, shp.res, shp.resTail, ResLayout<R>::MIN_ST,
-                       [&](const RbShape& sh, size_t smem, int grid) {
-                           k_res_rb<R><<<grid, RB_THREADS, smem, st>>>(S, all, sh);
-                       }));
-        return PHX_OK;
-    }
-
-    template <class K, class Launch>
-    int tuneRB(const char* name, RbCfg& c, K kern, RbShape shape, int tail, int minSt, Launch launchFn) {
-        int dev = 0, sms = 0;
-        PHX_CK(cudaGetDevice(&dev));
-        PHX_CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-        const size_t maxSmem = RB_SM_SMEM - RB_STATIC_SMEM;
-        PHX_CK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)maxSmem));
-        std::vector<int> cands;
-        for (int k = minSt; k <= RB_MAX_ST; ++k) {
-            RbShape sh = shape;
-            sh.st = k;
-            if (rbSmem(sh, tail) <= maxSmem) cands.push_back(k);
-        }
-        if (cands.empty()) {
-            err = std::string("the batch's widest grids need more shared memory than an SM has (") + name + ")";
-            return PHX_ERR_UNSUPPORTED;
-        }
-        auto gridFor = [&](size_t smem, int* grid) -> int {
-            int occ = 0;
-            PHX_CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kern, RB_THREADS, smem));
-            *grid = std::min(sms * std::max(occ, 1), persistCtas);
-            return PHX_OK;
-        };
-        // default: the deepest ring that still lets two CTAs share an SM, else one more slot than the minimum
-        int best = cands.front() + (cands.size() > 1 ? 1 : 0);
-        for (int k : cands) {
-            RbShape sh = shape;
-            sh.st = k;
-            if (rbSmem(sh, tail) <= RB_SM_SMEM / 2 - RB_STATIC_SMEM) best = k;
-        }
-        const std::string key = std::string(name) + ":" + std::to_string(shape.slot) + ":" + std::to_string(shape.ring) +
-                                ":" + std::to_string(tail);
-        auto hit = tuneCache.find(key);
-        if (hit != tuneCache.end()) {
-            best = hit->second;
-        } else if (std::getenv("PHX_NO_AUTOTUNE") == nullptr && dom[D_RB].total > 0 && cands.size() > 1) {
-            float bestMs = 1e30f;
-            for (int k : cands) {
-                RbShape sh = shape;
-                sh.st = k;
-                const size_t smem = rbSmem(sh, tail);
-                int grid = 0;
-                PHX_TRY(gridFor(smem, &grid));
-                grid = std::min(grid, dom[D_RB].total);
-                launchFn(sh, smem, grid);
-                PHX_CK(cudaEventRecord(ev[2], st));
-                launchFn(sh, smem, grid);
-                launchFn(sh, smem, grid);
-                PHX_CK(cudaEventRecord(ev[3], st));
-                PHX_CK(cudaEventSynchronize(ev[3]));
-                float ms = 0;
-                PHX_CK(cudaEventElapsedTime(&ms, ev[2], ev[3]));
-                if (ms < bestMs) { bestMs = ms; best = k; }
-            }
-            PHX_TRY(checkLaunch());
-            PHX_TRY(checkDeviceError());
-            tuneCache[key] = best;
-        }
-        shape.st = best;
-        c.shape = shape;
-        c.smem = rbSmem(shape, tail);
-        PHX_TRY(gridFor(c.smem, &c.grid));
+        PHX_CK(cudaFuncSetAttribute(k_solve<R>, cudaFuncAttributeMaxDynamicSharedMemorySize, SolveCfg<R>::POOL));
+        PHX_CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_solve<R>, SolveCfg<R>::T, SolveCfg<R>::POOL));
+        if (occ < 1) { err = "the solve kernel does not fit an SM"; return PHX_ERR_CUDA; }
+        solveGrid = std::min(sms * occ, MAX_SOLVE_CTAS);
+        if (const char* c = std::getenv("PHX_PERSIST_CTAS")) solveGrid = std::max(1, std::min(solveGrid, std::atoi(c)));
         return PHX_OK;
     }
 
@@ -1404,51 +1154,6 @@ public:
         ++launches;
     }
 
-    // persistent grid over the active tiles of domain d (solve kernels): 16 CTAs of 256
-    // threads per SM of GB300 measured best on the 64-scenario batch (8: 274.5, 12: 278.5,
-    // 16: 279.0, 32: 278.2 M cell-updates/s; a CTA per tile: 268.7)
-    static constexpr int PERSIST_CTAS = 152 * 16;
-    int persistCtas = PERSIST_CTAS;   // PHX_PERSIST_CTAS caps it (tests: many tiles per CTA)
-    template <class K, class... A>
-    void launchA(const char* name, int d, int threads, K kern, A... args) {
-        if (dom[d].total <= 0) return;
-        const int grid = std::min(dom[d].total, persistCtas);
-        if (prof) {
-            if (evNext + 2 > (int)evPool.size()) {
-                for (int i = 0; i < 64; ++i) { cudaEvent_t e; cudaEventCreate(&e); evPool.push_back(e); }
-            }
-            cudaEventRecord(evPool[evNext], st);
-            kern<<<grid, threads, 0, st>>>(args...);
-            cudaEventRecord(evPool[evNext + 1], st);
-            evUse.push_back({name, evNext});
-            evNext += 2;
-        } else {
-            kern<<<grid, threads, 0, st>>>(args...);
-        }
-        ++launches;
-    }
-
-    // persistent grid over the active row-block tiles, with the staging ring in dynamic shared memory
-    template <class K, class... A>
-    void launchRB(const char* name, const RbCfg& c, K kern, A... args) {
-        if (dom[D_RB].total <= 0) return;
-        const int grid = std::min(dom[D_RB].total, c.grid);
-        const size_t rbSmem = c.smem;
-        if (prof) {
-            if (evNext + 2 > (int)evPool.size()) {
-                for (int i = 0; i < 64; ++i) { cudaEvent_t e; cudaEventCreate(&e); evPool.push_back(e); }
-            }
-            cudaEventRecord(evPool[evNext], st);
-            kern<<<grid, RB_THREADS, rbSmem, st>>>(args...);
-            cudaEventRecord(evPool[evNext + 1], st);
-            evUse.push_back({name, evNext});
-            evNext += 2;
-        } else {
-            kern<<<grid, RB_THREADS, rbSmem, st>>>(args...);
-        }
-        ++launches;
-    }
-
     // the device error word: a bounded wait inside a kernel that ran out
     int checkDeviceError() {
         if (!dErr) return PHX_OK;
@@ -1459,33 +1164,12 @@ public:
             // report once and clear, so that the context stays usable
             PHX_CK(cudaMemsetAsync(dErr, 0, sizeof(unsigned), st));
             PHX_CK(cudaStreamSynchronize(st));
-            err = (w & 3u) ? "a staged shared-memory copy did not arrive within its time limit; the step's results are "
-                             "not valid (device error word " + std::to_string(w) + ")"
-                           : "a bounded device wait ran out (self-test, device error word " + std::to_string(w) + ")";
+            err = (w & ERR_TEAM_WAIT) ? "a CTA of the pressure solve waited too long for its team; the step's results are not "
+                             "valid (device error word " + std::to_string(w) + ")"
+                                        : "a bounded device wait ran out (self-test, device error word " + std::to_string(w) + ")";
             return PHX_ERR_TIMEOUT;
         }
         return PHX_OK;
-    }
-
-    ActiveTables activeTables() const {
-        ActiveTables t;
-        t.tiles = dTiles;
-        t.astart = dAStart;
-        t.atotal = dATotal;
-        t.nscn = nscn();
-        t.cap = cap;
-        t.ndom = D_COUNT;
-        // the domains of the solve's persistent kernels (kind 0: solving, kind 1: replacing)
-        int n = 0;
-        auto add = [&](int kind, int d) { if (n < 32) t.list[n++] = (short)(kind * D_COUNT + d); };
-        add(0, D_CELLS); add(0, D_CZ); add(0, D_RB); add(0, D_L0); add(0, D_L0R); add(0, D_QUAD); add(0, D_CO_DENSE); add(0, D_CO_SERIAL);
-        for (int l = 1; l < maxLevels - 1 && l < MAX_LEVELS; ++l) { add(0, D_LV0 + l); add(0, D_RS0 + l); }
-        add(1, D_CELLS); add(1, D_CZ);
-        t.nlist = n;
-        return t;
-    }    void rebuildActive() {
-        k_active<R><<<1, 256, 0, st>>>(dS, activeTables());
-        ++launches;
     }
 
     int collectProfile() {
@@ -1567,95 +1251,47 @@ public:
             launch("k_leak_finish", D_CZ, TPB, k_leak_finish<R>, (const Scn<R>*)dS, dom[D_CZ]);
         }
     }
-    // one V-cycle z = M r (src/sim/pressure_mg.cpp:270-300) closed by the
-    // last red half sweep with r.z; phase 0: before the CG loop, 1: inside
-    // it, 2: a bare V-cycle
-    void vcycle(int phase) {
+    // the whole pressure solve in one cooperative launch (solve.cuh)
+    int launchSolve(int vcycleOnly) {
+        SolveArgs a;
+        a.nscn = nscn();
+        a.cap = maxItersAll() + 2;
+        a.vcycleOnly = vcycleOnly;
+        a.maxPart = dMaxPart;
+        cudaLaunchConfig_t cfg = {};
+        cfg.gridDim = dim3((unsigned)solveGrid);
+        cfg.blockDim = dim3(SolveCfg<R>::T);
+        cfg.dynamicSmemBytes = SolveCfg<R>::POOL;
+        cfg.stream = st;
+        cudaLaunchAttribute at;
+        at.id = cudaLaunchAttributeCooperative;
+        at.val.cooperative = 1;
+        cfg.attrs = &at;
+        cfg.numAttrs = 1;
         const Scn<R>* S = dS;
-        if (useL0) {
-            launchL0<L0_PRE>("k_gs_pre", phase);
-            launchL0<L0_RES>("k_res_restrict", phase);
-        } else {
-            launchRB("k_gs_pre", cfgGs[GS_PRE], k_gs_rb<R, GS_PRE>, S, adom[0][D_RB], cfgGs[GS_PRE].shape, phase);
-            launchRB("k_res_restrict", cfgRes, k_res_rb<R>, S, adom[0][D_RB], cfgRes.shape);
-        }
-        // down: level 1's first Jacobi sweep; then per level its second sweep (not
-        // in the one-sweep schedule) and its residual restricted to level l+1 with
-        // l+1's first sweep; up: per level the prolongating sweep and (two-sweep
-        // schedule) a plain one
-        if (!useL0) launchA("k_jacobi", D_LV0 + 1, TPB, k_jacobi<R>, S, adom[0][D_LV0 + 1], 1, 0);
-        for (int l = 1; l < maxLevels - 1; ++l) {
-            if (!smoothOne) launchA("k_jacobi", D_LV0 + l, TPB, k_jacobi<R>, S, adom[0][D_LV0 + l], l, 1);
-            launchA("k_res_restrict_jac0", D_RS0 + l, TPB, k_res_restrict_jac0<R>, S, adom[0][D_RS0 + l], l);
-        }
-        launchA("k_coarse_dense", D_CO_DENSE, TPB, k_coarse_dense<R>, S, adom[0][D_CO_DENSE]);
-        launchA("k_coarse_serial", D_CO_SERIAL, 32, k_coarse_serial<R>, S, adom[0][D_CO_SERIAL]);
-        for (int l = maxLevels - 2; l >= 1; --l) {
-            if (smoothOne) {
-                launchA("k_jacobi", D_LV0 + l, TPB, k_jacobi<R>, S, adom[0][D_LV0 + l], l, 3);
-            } else {
-                launchA("k_jacobi", D_LV0 + l, TPB, k_jacobi<R>, S, adom[0][D_LV0 + l], l, 2);
-                launchA("k_jacobi", D_LV0 + l, TPB, k_jacobi<R>, S, adom[0][D_LV0 + l], l, 1);
+        int e0 = -1;
+        if (prof) {
+            if (evNext + 2 > (int)evPool.size()) {
+                for (int i = 0; i < 64; ++i) { cudaEvent_t e; cudaEventCreate(&e); evPool.push_back(e); }
             }
+            e0 = evNext;
+            evNext += 2;
+            cudaEventRecord(evPool[e0], st);
         }
-        if (useL0) {
-            launchL0<L0_BLACK>("k_gs_black", phase);
-            launchL0<L0_RED>("k_gs_red_dot", phase);
-        } else {
-            launchRB("k_gs_black", cfgGs[GS_BLACK], k_gs_rb<R, GS_BLACK>, S, adom[0][D_RB], cfgGs[GS_BLACK].shape, phase);
-            launchRB("k_gs_red_dot", cfgGs[GS_RED], k_gs_rb<R, GS_RED>, S, adom[0][D_RB], cfgGs[GS_RED].shape, phase);
+        PHX_CK(cudaLaunchKernelEx(&cfg, k_solve<R>, S, a));
+        if (prof) {
+            cudaEventRecord(evPool[e0 + 1], st);
+            evUse.push_back({"k_solve", e0});
         }
-    }
-    // all scenarios' flag in slot `slot` set?
-    int readAll(int slot, bool& all) {
-        const int n = nscn();
-        for (int s = 0; s < n; ++s)
-            PHX_CK(cudaMemcpyAsync(hPin + 16 + s % 4000, sc[s]->h.sv + slot, sizeof(double), cudaMemcpyDeviceToHost, st));
-        PHX_CK(cudaStreamSynchronize(st));
-        all = true;
-        for (int s = 0; s < n; ++s) all &= hPin[16 + s % 4000] != 0;
+        ++launches;
         return PHX_OK;
     }
-    // Solver::project: right-hand side, first V-cycle and CG set-up
-    void projectPrelude() {
+    // right-hand side (and the mixed path's initial guess), then the solve
+    int solveStage() {
         const Scn<R>* S = dS;
-        launch("k_reset", D_ONE, 32, k_reset<R>, S, dom[D_ONE], 0);
-        rebuildActive();
+        if (kMixed) launch("k_mx_extrap", D_CELLS, TPB, k_mx_extrap<R>, S, dom[D_CELLS]);
         launch("k_rhs", D_CELLS, TPB, k_rhs<R>, S, dom[D_CELLS]);
-        vcycle(0);
-    }
-    // one CG iteration (src/sim/gasphase.cpp:605-625). The mixed path can
-    // replace the recursive residual by the FP64 one before preconditioning,
-    // so its first red half sweep runs after that.
-    // The CG iteration in three parts: q = A d and the update; the mixed path's
-    // residual replacement (in the step graph, a conditional node that runs it
-    // only on iterations where some scenario replaces); the preconditioner.
-    void cgIterUpdate(cudaGraphConditionalHandle repl, int setCond) {
-        const Scn<R>* S = dS;
-        if (useL0) {
-            launchA("k_l0_dupdate", D_QUAD, TPB, k_l0_dupdate<R>, S, adom[0][D_QUAD], (R* const*)dD);
-            launchL0<L0_APPLY>("k_cg_apply", 1);
-        } else launchRB("k_cg_apply", cfgApply, k_cg_apply_rb<R>, S, adom[0][D_RB], (R* const*)dD, cfgApply.shape);
-        launchA("k_cg_update", D_QUAD, TPB, k_cg_update<R>, S, adom[0][D_QUAD], (R* const*)dD, repl,
-                (const int*)adom[1][D_CELLS].total, dLoop + 1, setCond);
-        if (kMixed && anyClosed) launchA("k_mx_zone_center", D_CZ, TPB, k_mx_zone_center<R>, S, adom[0][D_CZ], 0);
-    }
-    void cgIterReplace() {
-        const Scn<R>* S = dS;
-        launchA("k_mx_update", D_CELLS, TPB, k_mx_update<R>, S, adom[1][D_CELLS], 1);
-        launchA("k_mx_res64", D_CELLS, TPB, k_mx_res64<R>, S, adom[1][D_CELLS], 1);
-        launchA("k_mx_zone_proj", D_CZ, TPB, k_mx_zone_proj<R>, S, adom[1][D_CZ], 1);
-    }
-    void cgIterPrecondition() {
-        const Scn<R>* S = dS;
-        vcycle(1);
-        if (kMixed && anyClosed) launchA("k_mx_zone_center", D_CZ, TPB, k_mx_zone_center<R>, S, adom[0][D_CZ], 1);
-    }
-    // one CG iteration (src/sim/gasphase.cpp:605-625), launched kernel by kernel
-    void cgIteration() {
-        cgIterUpdate(cudaGraphConditionalHandle{}, 0);
-        if (kMixed) cgIterReplace();
-        cgIterPrecondition();
+        return launchSolve(0);
     }
     // zone mean removal and velocity correction (:629-676)
     void projectEpilogue() {
@@ -1666,41 +1302,14 @@ public:
         launch("k_velcorr", D_FY, TPB, k_velcorr<R>, S, dom[D_FY], 1);
         launch("k_velcorr", D_FZ, TPB, k_velcorr<R>, S, dom[D_FZ], 2);
     }
-    // ---- mixed path: the FP32 CG starts from the FP64 residual b - A p64 ---------------
-    void mixedPrelude() {
-        const Scn<R>* S = dS;
-        launch("k_reset", D_ONE, 32, k_reset<R>, S, dom[D_ONE], 0);
-        rebuildActive();
-        launch("k_mx_extrap", D_CELLS, TPB, k_mx_extrap<R>, S, dom[D_CELLS]);
-        launch("k_rhs", D_CELLS, TPB, k_rhs<R>, S, dom[D_CELLS]);
-        launchA("k_mx_res64", D_CELLS, TPB, k_mx_res64<R>, S, adom[0][D_CELLS], 0);
-        launchA("k_mx_zone_proj", D_CZ, TPB, k_mx_zone_proj<R>, S, adom[0][D_CZ], 0);
-        vcycle(0);
-        if (anyClosed) launchA("k_mx_zone_center", D_CZ, TPB, k_mx_zone_center<R>, S, adom[0][D_CZ], 1);
-    }
-    void mixedEpilogue() {
-        launch("k_mx_final", D_CELLS, TPB, k_mx_final<R>, dS, dom[D_CELLS]);
-    }
-
     int maxItersAll() const {
         int m = 0;
         for (auto& S : sc) m = std::max(m, S->maxIters);
         return m;
     }
 
-    // host-driven CG loop: the stop test is read back after every iteration
     int stProject() {
-        if (kMixed) mixedPrelude();
-        else projectPrelude();
-        const int maxIt = maxItersAll();
-        bool done = false;
-        PHX_TRY(readAll(SV_DONE, done));
-        for (int it = 0; !done && it <= maxIt + 1; ++it) {
-            rebuildActive();
-            cgIteration();
-            PHX_TRY(readAll(SV_DONE, done));
-        }
-        if (kMixed) mixedEpilogue();
+        PHX_TRY(solveStage());
         projectEpilogue();
         return PHX_OK;
     }
@@ -1726,13 +1335,12 @@ public:
         return PHX_OK;
     }
 
-    // ---- captured step graph: the CG loops are device-side while nodes ---------------
+    // ---- captured step graph -----------------------------------------------------------
     cudaGraph_t graph = nullptr;
     cudaGraphExec_t gexec = nullptr;
-    cudaGraphConditionalHandle cgHandle{};
-    int outerKernels = 0, bodyKernels = 0, replKernels = 0;
+    int graphKernels = 0;        // kernel nodes of the step graph
     // the step runs as one CUDA graph; PHX_NO_GRAPH=1 launches the same kernels
-    // one by one (kernels inside conditional graphs cannot be profiled by ncu)
+    // one by one
     bool useGraph = std::getenv("PHX_NO_GRAPH") == nullptr;
 
     void destroyGraph() {
@@ -1742,34 +1350,11 @@ public:
         graph = nullptr;
     }
 
-    // add a conditional node (while or if) after the current capture position of
-    // st (which captures into graph g); capture continues after it
-    int addConditional(cudaGraph_t g, cudaGraphConditionalHandle handle, cudaGraphConditionalNodeType type,
-                       cudaGraph_t* body) {
-        cudaStreamCaptureStatus cs;
-        const cudaGraphNode_t* deps = nullptr;
-        size_t ndeps = 0;
-        PHX_CK(cudaStreamGetCaptureInfo(st, &cs, nullptr, nullptr, &deps, nullptr, &ndeps));
-        cudaGraphNodeParams cp = {};
-        cp.type = cudaGraphNodeTypeConditional;
-        cp.conditional.handle = handle;
-        cp.conditional.type = type;
-        cp.conditional.size = 1;
-        cudaGraphNode_t cond;
-        PHX_CK(cudaGraphAddNode(&cond, g, deps, nullptr, ndeps, &cp));
-        *body = cp.conditional.phGraph_out[0];
-        PHX_CK(cudaStreamUpdateCaptureDependencies(st, &cond, nullptr, 1, cudaStreamSetCaptureDependencies));
-        return PHX_OK;
-    }
-
     int buildGraph() {
         destroyGraph();
         std::vector<Scn<R>> saved;
         for (auto& S : sc) saved.push_back(S->h);
-        const int n = nscn();
         PHX_CK(cudaGraphCreate(&graph, 0));
-        // conditional handles are created before the capture of the graph that holds their node
-        PHX_CK(cudaGraphConditionalHandleCreate(&cgHandle, graph, 0, 0));
         PHX_CK(cudaStreamBeginCaptureToGraph(st, graph, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal));
         launches = 0;
         stBegin(true, 0.0);
@@ -1779,44 +1364,13 @@ public:
         stEnergy();
         stMomentum();
         stLeakage();
-        if (kMixed) mixedPrelude();
-        else projectPrelude();
-        cudaMemsetAsync(dLoop, 0, 2 * sizeof(int), st);
-        const int capIt = maxItersAll() + 2;
-        k_cg_cond<R><<<1, 256, 0, st>>>(dS, n, cgHandle, dLoop, capIt, activeTables(), 1);
-        ++launches;
-        cudaGraph_t body = nullptr;
-        PHX_TRY(addConditional(graph, cgHandle, cudaGraphCondTypeWhile, &body));
-        if (kMixed) mixedEpilogue();
-        projectEpilogue();
+        PHX_TRY(stProject());
         stAdvect();
         stEnd();
-        cudaGraph_t outGraph = nullptr;
-        PHX_CK(cudaStreamEndCapture(st, &outGraph));
-        outerKernels = launches;
-        // the loop body; the mixed path's residual replacement is a conditional
-        // node of it, set by k_cg_update on each iteration
-        cudaGraphConditionalHandle replHandle{};
-        cudaGraph_t replBody = nullptr;
-        if (kMixed) PHX_CK(cudaGraphConditionalHandleCreate(&replHandle, body, 0, 0));
-        PHX_CK(cudaStreamBeginCaptureToGraph(st, body, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal));
-        launches = 0;
-        cgIterUpdate(replHandle, kMixed ? 1 : 0);
-        if (kMixed) PHX_TRY(addConditional(body, replHandle, cudaGraphCondTypeIf, &replBody));
-        cgIterPrecondition();
-        k_cg_cond<R><<<1, 256, 0, st>>>(dS, n, cgHandle, dLoop, capIt, activeTables(), 1);
-        ++launches;
-        PHX_CK(cudaStreamEndCapture(st, &body));
-        bodyKernels = launches;
-        replKernels = 0;
-        if (kMixed) {
-            PHX_CK(cudaStreamBeginCaptureToGraph(st, replBody, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal));
-            launches = 0;
-            cgIterReplace();
-            PHX_CK(cudaStreamEndCapture(st, &replBody));
-            replKernels = launches;
-        }
-        for (int s = 0; s < n; ++s) sc[s]->h = saved[s];
+        cudaGraph_t done = nullptr;
+        PHX_CK(cudaStreamEndCapture(st, &done));
+        graphKernels = launches;
+        for (int s = 0; s < nscn(); ++s) sc[s]->h = saved[s];
         PHX_CK(cudaGraphInstantiate(&gexec, graph, 0));
         return checkLaunch();
     }
@@ -1826,15 +1380,6 @@ public:
         PHX_TRY(setDtMax(dtMax, per));
         PHX_CK(cudaGraphLaunch(gexec, st));
         swapHost(1 | 2 | 4);
-        return PHX_OK;
-    }
-
-    // kernels the last graph step ran: the outer nodes plus the loop body per iteration
-    int graphLaunchCount(int* out) {
-        int lc[2] = {0, 0};
-        PHX_CK(cudaMemcpyAsync(lc, dLoop, 2 * sizeof(int), cudaMemcpyDeviceToHost, st));
-        PHX_CK(cudaStreamSynchronize(st));
-        *out = outerKernels + bodyKernels * std::max(0, lc[0] - 1) + replKernels * lc[1];
         return PHX_OK;
     }
 
@@ -1900,9 +1445,8 @@ public:
         Scenario<R>& S = *sc[0];
         const int N = S.geo.N();
         PHX_TRY(S.put(st, S.h.r, std::vector<double>(r, r + N)));
-        launch("k_reset", D_ONE, 32, k_reset<R>, (const Scn<R>*)dS, dom[D_ONE], 2);
-        rebuildActive();
-        vcycle(2);
+        launch("k_reset", D_ONE, 32, k_reset<R>, (const Scn<R>*)dS, dom[D_ONE]);
+        PHX_TRY(launchSolve(1));
         PHX_TRY(checkLaunch());
         return getReal(S.h.z, N, z);
     }
@@ -2084,10 +1628,7 @@ public:
         return PHX_OK;
     }
     int lastLaunches() const override {
-        if (useGraph && gexec) {
-            int k = 0;
-            if (const_cast<Ctx*>(this)->graphLaunchCount(&k) == PHX_OK) return k;
-        }
+        if (useGraph && gexec) return graphKernels;
         return launches;
     }
 
@@ -2112,13 +1653,7 @@ public:
             float ms = 0;
             PHX_CK(cudaEventElapsedTime(&ms, ev[0], ev[1]));
             total += ms;
-            if (useGraph) {
-                int k = 0;
-                PHX_TRY(graphLaunchCount(&k));
-                nl += k;
-            } else {
-                nl += launches;
-            }
+            nl += useGraph ? graphKernels : launches;
         }
         if (totalMs) *totalMs = total;
         if (launchesOut) *launchesOut = nl;

@@ -84,12 +84,10 @@ enum Slot {
     SV_DTMAX_ARG = 0, SV_DT, SV_TIME, SV_MAXVEL, SV_MAXNU, SV_MAXDIV,
     SV_RZ, SV_ALPHA, SV_BETA, SV_RMAX, SV_BMAX, SV_IT, SV_DONE, SV_DQ,
     SV_PITERS, SV_PRES, SV_PREL, SV_HRR, SV_MAXGAST, SV_BURNING, SV_FUELIN, SV_FUELBURNED, SV_FUELINDOMAIN,
-    SV_INV, SV_ACTIVE,
-    // mixed path: FP64 refinement loop around the FP32 inner CG
-    SV_R64MAX, SV_R0MAX, SV_OUTER, SV_ODONE, SV_ITTOT, SV_REPL,
+    SV_INV,
     SV_HAVEPREV,                 // mixed path: p64prev holds the previous step's pressure
     SV_SRC_MF = 32,              // MAX_SRC injection amounts of this step (-1 = inactive)
-    SV_BREAK = SV_SRC_MF + MAX_SRC,   // mixed path: 1 after a CG breakdown (next update skipped), 2 restart pending
+    SV_WITERS = SV_SRC_MF + MAX_SRC,                     // iterations of the last solve (SV_PITERS), fixed for the coming one: its team's weight
     SV_COUNT = 64
 };
 
@@ -129,6 +127,7 @@ struct Level {
     const int *rowStart, *col;   // couplings (off-diagonal, positive), coarse levels
     const R* val;
     const R* diag;
+    const R* omd;                // omega / diag (0 without a diagonal): the damped Jacobi factor
     const int* agg;              // unknown -> unknown of the next coarser level (nullptr at the coarsest)
     const int *childStart, *child;   // next coarser unknown -> its unknowns here, ascending
     R *x, *y, *b;                // iterate, Jacobi scratch, right-hand side
@@ -142,7 +141,7 @@ struct Scn {
     // row length dvA, plane size dvB, rows per plane dY
     DivU dvA[3], dvB[3];
     int dY[3];
-    DivU dvL0[2];                // 2x2x2 blocks of the mixed path's level-0 kernels: blocks per row, per plane
+    DivU dvL0[2];                // 2x2x2 blocks of the pressure solve: blocks per row, per plane
     double dx, ox, oy, oz;
     double cfl, dtMaxP, tol, relTol;
     const double* dtMaxArg;      // this step's dtMax argument (one slot per scenario of the batch)
@@ -159,7 +158,7 @@ struct Scn {
     const R *a0x, *a0y, *a0z;    // the same with wind-inflow boundary faces closed (multigrid level 0)
     const uint8_t *lx, *ly, *lz; // crack faces (null when there are none)
     const R* diag;               // level-0 diagonal
-    const unsigned char* code0;  // mixed path: level-0 coefficient code per cell (level0.cuh)
+    const unsigned char* code0;  // level-0 coefficient code per cell (level0.cuh)
     const int* zone;
     const uint8_t* zoneOpen;
     int nZones, nClosed;
@@ -193,20 +192,17 @@ struct Scn {
     int replaceEvery;            // mixed path: iterations between FP64 residual replacements
     int extrap;                  // mixed path: start the solve from 2 p(n) - p(n-1) (PHX_NO_EXTRAP=1: from p(n))
     double* p64prev;             // mixed path: the previous step's pressure (FP64)
-    int fp16Scratch;             // mixed path: Jacobi scratch rounded to FP16 (an accuracy study; off by default)
-    int fp16Z0;                  // mixed path: level-0 smoother output z rounded to FP16 (an accuracy study; off by default)
     int nLevels;
     int smooth1;                 // mixed path: one damped Jacobi sweep per coarse level on each leg
                                  // of the V-cycle (the reference: two, src/sim/pressure_mg.cpp:281-297)
     Level<R> lv[MAX_LEVELS];
-    // row-block tiles of the level-0 pressure kernels: tj rows x RB_KZ planes, njb blocks along y
-    int tj, njb;
-    unsigned* errWord;           // the context's error word (a bounded wait that ran out sets bit 0)
+    unsigned* errWord;           // the context's error word (a bounded wait that ran out sets a bit)
     // scalars and reductions
     double* sv;
     double* part;                // PS_COUNT x partStride
     int partStride;
     unsigned* cnt;               // last-CTA counters, one per reduction kind
+    unsigned* teamBar;           // arrivals at the solve's team barrier; zeroed by k_begin and k_reset
 };
 
 // CTA -> (scenario, tile) over a domain
@@ -216,36 +212,6 @@ struct Dom {
     int total;                   // CTAs of the launch
     const unsigned* owner;       // [total] scenario << 20 | tile of each CTA (null: search the prefix)
 };
-
-// the same over the scenarios still active in a solve: the prefix and the
-// total live in device memory and are rebuilt between iterations, so a
-// persistent grid loops over the tiles of unfinished scenarios only
-struct ADom {
-    const int* start;            // [nscn + 1], zero-width for finished scenarios
-    const int* total;
-    int nscn;
-};
-
-// binary search in a shared-memory copy of an active prefix
-__device__ __forceinline__ void locateShared(const int* st, int nscn, int b, int& s, int& tile) {
-    int lo = 0, hi = nscn - 1;
-    while (lo < hi) {
-        int mid = (lo + hi + 1) >> 1;
-        if (st[mid] <= b) lo = mid; else hi = mid - 1;
-    }
-    s = lo;
-    tile = b - st[lo];
-}
-
-__device__ __forceinline__ void locate(const ADom& d, int b, int& s, int& tile) {
-    int lo = 0, hi = d.nscn - 1;
-    while (lo < hi) {
-        int mid = (lo + hi + 1) >> 1;
-        if (d.start[mid] <= b) lo = mid; else hi = mid - 1;
-    }
-    s = lo;
-    tile = b - d.start[lo];
-}
 
 __device__ __forceinline__ void locate(const Dom& d, int b, int& s, int& tile) {
     if (d.owner) {   // one load instead of a search through the prefix

@@ -1,0 +1,1093 @@
+// The pressure solve as one cooperative kernel: the multigrid-preconditioned
+// CG of every scenario of a context (src/sim/gasphase.cpp:551-626 with the
+// V-cycle of src/sim/pressure_mg.cpp:193-300), from the first residual to the
+// accepted pressure.
+//
+// Why one kernel. A CG iteration is 12 to 18 short passes. Launched one by one
+// from a graph's while node each cost about 6 us on a single building whatever
+// its size (a launch, a chain of dependent loads for its tables and
+// descriptor, and a drained GPU); a team barrier costs 1.0 us between 2 CTAs
+// and 1.2 to 1.5 us between 152 with stores in flight, and tables, scalars and
+// coarse rows stay on the SM. Measured, ms per step, launches / this kernel:
+// 36x24x24 room 2.17 / 1.06 in FP64 and 1.13 / 0.55 mixed, 72x52x44 house
+// 6.8 / 4.3 and 2.77 / 1.30, 1.3 M cells mixed 5.66 / 4.1, 24 houses of 2.9 M
+// cells mixed 8.1 / 5.9.
+//
+// What bounds it. One building: latency. Per pass a barrier, one L2 round trip
+// (286 cycles) and the pass's own instructions, 2 to 3 us together; per
+// reduction a chain of FP64 additions (72 cycles each) and one division (570).
+// Large batches: instruction issue in FP32, the FP64 pipe (a warp's
+// instruction takes it about 19 cycles) in FP64.
+//
+// Teams. The CTAs of the grid are divided into one team per scenario, in
+// proportion to the scenario's work (cells times the iterations of its last
+// solve), at least one CTA each. A team runs its scenario's passes one after
+// the other with a barrier of its own between them, so a scenario never waits
+// for another one's iterations and a stopped scenario costs nothing. With more
+// scenarios than CTAs a team is one CTA that takes several scenarios in turn.
+// Every CTA of a team keeps the scenario's scalars in shared memory and
+// computes alpha, beta and the stop test itself from the passes' partial sums,
+// in one fixed order, so all of them take the same decisions.
+//
+// Sums: a scenario's partial sums and the order they are added in follow from
+// its size alone (SolveTiling). Neither depends on the teams, so a scenario's
+// result is the same bits alone, in any batch and with any number of CTAs.
+//
+// Waits: a team barrier gives up after TEAM_WAIT_CYCLES, records it in the
+// context's error word and ends the kernel; the launch is cooperative, so all
+// CTAs of a team are resident.
+#pragma once
+#include "mixed_kernels.cuh"
+
+namespace phx {
+
+constexpr long long TEAM_WAIT_CYCLES = 4000000000LL;       // about two seconds
+constexpr unsigned ERR_TEAM_WAIT = 8u;                     // error-word bit
+
+template <class R>
+struct SolveCfg {
+    static constexpr int T = sizeof(R) == 8 ? 512 : 1024;  // threads per CTA
+    static constexpr int POOL = 98304;                     // shared memory for the coarse rows, bytes
+};
+
+// How a scenario's pairs are walked: a warp takes 8 consecutive 2x2x2 blocks (four
+// lanes a block) at a time; `warps` warps side by side are a tile, which walks
+// `reps` such groups. A tile's dot product is one partial sum. The shape follows
+// from the scenario's size alone, so its sums do not depend on the team.
+// FP32: a tile is always the 32 blocks of four warps, whose products are added in
+// the order of one thread per block (the block's cells in ascending order, then
+// a warp's shuffle tree), four tiles to a sum that reaches FP64.
+struct SolveTiling {
+    int warps, reps, nt;
+};
+template <class R>
+__host__ __device__ inline SolveTiling solveTiling(int nblk) {
+    const int groups = (nblk + 7) / 8;
+    SolveTiling t;
+    t.reps = 1;
+    if (sizeof(R) == 4) {
+        t.warps = 4;
+    } else {
+        t.warps = groups <= 512 ? 1 : groups <= 4096 ? 4 : 8;
+        while (groups / (t.warps * t.reps) >= 4096) t.reps *= 2;
+    }
+    const int per = t.warps * t.reps;
+    t.nt = (groups + per - 1) / per;
+    return t;
+}
+
+struct SolveArgs {
+    int nscn;
+    int cap;                 // iterations after which the loop ends whatever the flags say
+    int vcycleOnly;          // 1: one V-cycle z = M r without the CG (phx_precondition)
+    double* maxPart;         // 2 per CTA: max |r| of the recursion, max |r| of the FP64 residual
+};
+
+// Passes over level 0. A thread owns a pair of cells along x, one red (i + j + k
+// even) and one black; every pass relaxes or applies the stencil to one colour
+// and reads the other colour's neighbours.
+enum {
+    PASS_APPLY = 0,          // q = A z + beta q, d = z + beta d, d.q
+    PASS_UPDATE,             // p += alpha d, r -= alpha q, max|r|; red z = r / diag
+    PASS_RED0,               // red z = r / diag
+    PASS_BLACK0,             // black z from its red neighbours: the pre-smoothing pair from x = 0
+    PASS_RES,                // residual restricted to level 1, level 1's first Jacobi sweep
+    PASS_BLACK,              // black sweep after the prolongation
+    PASS_RED                 // red sweep, r.z
+};
+
+template <class R>
+struct SolveBufs {
+    R *p, *r, *z, *q, *d;    // d: the direction (FP32: the previous one, dNew the one being formed)
+    R* dNew;
+    R alpha, beta;
+    bool haveD;              // d and q hold the previous direction and its product
+};
+
+// a pair's values at c0, c0 + 1: one vector access where rows have even length
+template <class R, bool EVEN>
+__device__ __forceinline__ void pairLoad(const R* a, int c0, bool on1, R& v0, R& v1) {
+    if constexpr (EVEN) {
+        using V = typename std::conditional<sizeof(R) == 4, float2, double2>::type;
+        const V v = *reinterpret_cast<const V*>(a + c0);
+        v0 = v.x;
+        v1 = v.y;
+    } else {
+        v0 = a[c0];
+        v1 = a[on1 ? c0 + 1 : c0];
+    }
+}
+template <class R, bool EVEN>
+__device__ __forceinline__ void pairStore(R* a, int c0, bool on1, R v0, R v1) {
+    if constexpr (EVEN) {
+        using V = typename std::conditional<sizeof(R) == 4, float2, double2>::type;
+        V v;
+        v.x = v0;
+        v.y = v1;
+        *reinterpret_cast<V*>(a + c0) = v;
+    } else {
+        a[c0] = v0;
+        if (on1) a[c0 + 1] = v1;
+    }
+}
+
+// the right-hand side of level-1 unknown `at` (none: -1) and, unless level 1 is the
+// coarsest, its first damped Jacobi sweep from x = 0. Every lane writes its
+// cells' aggregates; the lanes of one aggregate write the same value.
+template <class R>
+__device__ __forceinline__ void restrictTo(const Scn<R>& g, int at, R value) {
+    if (at < 0) return;
+    const Level<R>& L = g.lv[1];
+    L.b[at] = value;
+    if (g.nLevels > 2) L.y[at] = jacobiValue(value, R(0), L.diag[at], L.omd[at]);
+}
+
+// One pass over the pair of thread-index q (block q / 4, row and plane of the
+// block by q % 4). All loads are issued unconditionally at clamped places and
+// used through the cell's code, so one memory latency covers them. Cells
+// without a diagonal hold 0 in z, d, q and r.
+//
+// FP64: terms of the reference's passes that are known by construction are not
+// evaluated. After the pre-smoothing pair a black cell's residual is zero and a
+// red cell's is the sum of its black neighbours (its z is r / diag); after the
+// last red half sweep (A z)_red = r_red; and q = A d follows d's recurrence
+// (q = A z + beta q), so no neighbour's d is needed. FP32 evaluates every term:
+// dropping them moved the rounding of its recursion, and with it iteration
+// counts and the pressure's FP32 noise.
+// dot (FP64) or t0, t1 (FP32) take the pair's terms of the pass's dot product.
+template <class R, int MODE, bool EVEN>
+__device__ __forceinline__ void solvePair(const Scn<R>& g, const SolveBufs<R>& B, int q, int nblk, double& dot, F2& t0,
+                                          F2& t1, R& rmax, bool writeZ) {
+    using T = R;
+    const int nx = g.nx, ny = g.ny, nz = g.nz, sxy = nx * ny;
+    const int blk = min(q >> 2, nblk - 1), sub = q & 3;
+    const int bz = (int)divU((unsigned)blk, g.dvL0[1]);
+    const int rem = blk - bz * (int)g.dvL0[1].d;
+    const int by = (int)divU((unsigned)rem, g.dvL0[0]);
+    const int i0 = 2 * (rem - by * (int)g.dvL0[0].d);
+    const int dj = sub & 1, dk = sub >> 1;
+    const int j = 2 * by + dj, k = 2 * bz + dk;
+    const bool live = (q >> 2) < nblk && j < ny && k < nz;
+    if (MODE != PASS_RES && !live) return;
+    const int c0 = live ? i0 + nx * j + sxy * k : 0;
+    const bool on1 = live && (EVEN || i0 + 1 < nx);
+    const int ro = dj ^ dk;                                  // the red cell of the pair: c0 + ro
+    const bool rOn = ro ? on1 : live, bOn = ro ? live : on1;
+    const int cr = rOn ? c0 + ro : c0, cb = bOn ? c0 + 1 - ro : c0;
+    const unsigned char* cf = g.code0;
+    auto diagOf = [&](int c, unsigned cd) -> T { return (cd & CODE_GENERAL) ? g.diag[c] : codeDiag<T>(cd); };
+
+    if constexpr (MODE == PASS_UPDATE) {
+        T p0, p1, d0, d1, q0, q1, r0, r1;
+        pairLoad<T, EVEN>(B.p, c0, on1, p0, p1);
+        pairLoad<T, EVEN>(sizeof(R) == 4 ? B.dNew : B.d, c0, on1, d0, d1);
+        pairLoad<T, EVEN>(B.q, c0, on1, q0, q1);
+        pairLoad<T, EVEN>(B.r, c0, on1, r0, r1);
+        const unsigned cd = cf[cr];
+        p0 = madd(p0, B.alpha, d0);
+        r0 = madd(r0, -B.alpha, q0);
+        p1 = madd(p1, B.alpha, d1);
+        r1 = madd(r1, -B.alpha, q1);
+        rmax = mx(rmax, (T)fabs(r0));
+        if (on1) rmax = mx(rmax, (T)fabs(r1));
+        pairStore<T, EVEN>(B.p, c0, on1, p0, p1);
+        pairStore<T, EVEN>(B.r, c0, on1, r0, r1);
+        if (writeZ && rOn) {
+            const T dg = diagOf(cr, cd);
+            B.z[cr] = dg <= T(0) ? T(0) : l0Div(ro ? r1 : r0, cd, dg);
+        }
+        return;
+    }
+    if constexpr (MODE == PASS_RED0) {
+        if (rOn) {
+            const unsigned cd = cf[cr];
+            const T rv = B.r[cr], dg = diagOf(cr, cd);
+            B.z[cr] = dg <= T(0) ? T(0) : l0Div(rv, cd, dg);
+        }
+        return;
+    }
+    if constexpr (sizeof(R) == 4 && (MODE == PASS_APPLY || MODE == PASS_RES)) {
+        // FP32: both cells of the pair with all their neighbours; q is A d itself and
+        // the residual keeps every term (their rounding is what the FP32 recursion
+        // is built on: the forms below, exact in real numbers, would let it drift)
+        auto value = [&](int at) -> T {
+            const T zv = B.z[at];
+            if (MODE == PASS_APPLY && B.haveD) return zv + B.beta * B.d[at];
+            return zv;
+        };
+        auto pair = [&](int at, T& v0, T& v1) {
+            pairLoad<T, EVEN>(B.z, at, on1, v0, v1);
+            if (MODE == PASS_APPLY && B.haveD) {
+                T e0, e1;
+                pairLoad<T, EVEN>(B.d, at, on1, e0, e1);
+                v0 = v0 + B.beta * e0;
+                v1 = v1 + B.beta * e1;
+            }
+        };
+        T v0, v1, ym0, ym1, yp0, yp1, zm0, zm1, zp0, zp1;
+        const int c1 = on1 ? c0 + 1 : c0;
+        const T xm = value(live && i0 > 0 ? c0 - 1 : c0), xp = value(live && i0 + 2 < nx ? c0 + 2 : c0);
+        pair(c0, v0, v1);
+        pair(live && j > 0 ? c0 - nx : c0, ym0, ym1);
+        pair(live && j < ny - 1 ? c0 + nx : c0, yp0, yp1);
+        pair(live && k > 0 ? c0 - sxy : c0, zm0, zm1);
+        pair(live && k < nz - 1 ? c0 + sxy : c0, zp0, zp1);
+        const unsigned cd0 = cf[c0], cd1 = cf[c1];
+        const L0Nb<T> n0{xm, v1, ym0, yp0, zm0, zp0}, n1{v0, xp, ym1, yp1, zm1, zp1};
+        L0Coef<T> g0{}, g1{};
+        if (live && (cd0 & CODE_GENERAL)) g0 = l0General(g, i0, j, k);
+        if (on1 && (cd1 & CODE_GENERAL)) g1 = l0General(g, i0 + 1, j, k);
+        const T dg0 = (cd0 & CODE_GENERAL) ? g0.dg : codeDiag<T>(cd0), dg1 = (cd1 & CODE_GENERAL) ? g1.dg : codeDiag<T>(cd1);
+        if constexpr (MODE == PASS_APPLY) {
+            T w0 = T(0), w1 = T(0);
+            if (dg0 > T(0)) w0 = l0Sum<-1>(dg0 * v0, cd0, g0, n0, i0, j, k, nx, ny, nz);
+            if (on1 && dg1 > T(0)) w1 = l0Sum<-1>(dg1 * v1, cd1, g1, n1, i0 + 1, j, k, nx, ny, nz);
+            pairStore<T, EVEN>(B.dNew, c0, on1, v0, v1);
+            pairStore<T, EVEN>(B.q, c0, on1, w0, w1);
+            t0 = f2prod(w0, v0);
+            t1 = on1 ? f2prod(w1, v1) : F2{0.f, 0.f};
+        } else {
+            T r0, r1;
+            pairLoad<T, EVEN>(B.r, c0, on1, r0, r1);
+            const int* af = g.lv[0].agg;
+            const int a0 = live ? af[c0] : -1, a1 = on1 ? af[c1] : -1;
+            T s0 = T(0), s1 = T(0);
+            if (a0 >= 0) s0 = l0Sum<1>(r0 - dg0 * v0, cd0, g0, n0, i0, j, k, nx, ny, nz);
+            if (a1 >= 0) s1 = l0Sum<1>(r1 - dg1 * v1, cd1, g1, n1, i0 + 1, j, k, nx, ny, nz);
+            // the block's cells in ascending order over its four lanes
+            T acc0 = T(0), acc1 = T(0);
+#pragma unroll
+            for (int l = 0; l < 4; ++l) {
+                const int b0 = __shfl_sync(0xffffffffu, a0, l, 4), b1 = __shfl_sync(0xffffffffu, a1, l, 4);
+                const T e0 = __shfl_sync(0xffffffffu, s0, l, 4), e1 = __shfl_sync(0xffffffffu, s1, l, 4);
+                if (b0 >= 0 && b0 == a0) acc0 = acc0 + e0;
+                if (b1 >= 0 && b1 == a0) acc0 = acc0 + e1;
+                if (b0 >= 0 && b0 == a1) acc1 = acc1 + e0;
+                if (b1 >= 0 && b1 == a1) acc1 = acc1 + e1;
+            }
+            restrictTo(g, a0, acc0);
+            if (a1 != a0) restrictTo(g, a1, acc1);
+        }
+        return;
+    }
+    // the cell this pass computes (o: its place in the pair) and its neighbours of
+    // the other colour
+    constexpr bool kRed = MODE == PASS_RES || MODE == PASS_RED;
+    const int o = kRed ? ro : 1 - ro;
+    const int c = kRed ? cr : cb, cIn = kRed ? cb : cr;
+    const bool cOn = kRed ? rOn : bOn, inOn = kRed ? bOn : rOn;
+    const bool hx = o ? i0 + 2 < nx : i0 > 0;
+    const int nb[5] = {hx ? (o ? c + 1 : c - 1) : c, j > 0 ? c - nx : c, j < ny - 1 ? c + nx : c,
+                       k > 0 ? c - sxy : c, k < nz - 1 ? c + sxy : c};
+    const T* z = B.z;
+    T v[5], vIn;
+    vIn = z[cIn];
+#pragma unroll
+    for (int f = 0; f < 5; ++f) v[f] = z[live ? nb[f] : 0];
+    const unsigned cd = cf[c];
+    if constexpr (MODE == PASS_BLACK) {   // red neighbours: z plus the prolongated correction
+        const int* af = g.lv[0].agg;
+        const T* x1 = g.lv[1].x;
+        int ag[5], agIn;
+        agIn = af[cIn];
+#pragma unroll
+        for (int f = 0; f < 5; ++f) ag[f] = af[nb[f]];
+        T xv[5], xIn;
+        xIn = x1[max(agIn, 0)];
+#pragma unroll
+        for (int f = 0; f < 5; ++f) xv[f] = x1[max(ag[f], 0)];
+        vIn = agIn >= 0 ? (T)(vIn + xIn) : vIn;
+#pragma unroll
+        for (int f = 0; f < 5; ++f) v[f] = ag[f] >= 0 ? (T)(v[f] + xv[f]) : v[f];
+    }
+    L0Nb<T> n;
+    n.xm = o ? vIn : v[0];
+    n.xp = o ? v[0] : vIn;
+    n.ym = v[1];
+    n.yp = v[2];
+    n.zm = v[3];
+    n.zp = v[4];
+    auto sum = [&](auto sign, T start, L0Coef<T>& gen) -> T {
+        if (cd & CODE_GENERAL) gen = l0General(g, i0 + o, j, k);
+        return l0Sum<decltype(sign)::value>(start, cd, gen, n, i0 + o, j, k, nx, ny, nz);
+    };
+    using Plus = std::integral_constant<int, 1>;
+    using Minus = std::integral_constant<int, -1>;
+    L0Coef<T> gen{};
+    if constexpr (MODE == PASS_APPLY) {
+        T z0, z1, d0 = T(0), d1 = T(0), q0 = T(0), q1 = T(0);
+        const T zc = z[c], rr = B.r[cr];
+        if (B.haveD) {
+            pairLoad<T, EVEN>(B.d, c0, on1, d0, d1);
+            pairLoad<T, EVEN>(B.q, c0, on1, q0, q1);
+        }
+        const T zr = rOn ? vIn : T(0), zb = bOn ? zc : T(0);
+        z0 = ro ? zb : zr;
+        z1 = ro ? zr : zb;
+        T wb = T(0);
+        if (cOn) {
+            const T dg = diagOf(c, cd);
+            if (dg > T(0)) wb = sum(Minus{}, dg * zb, gen);
+        }
+        const T wr = rOn ? rr : T(0);
+        T w0 = ro ? wb : wr, w1 = ro ? wr : wb;
+        if (B.haveD) {
+            z0 = madd(z0, B.beta, d0);
+            z1 = madd(z1, B.beta, d1);
+            w0 = madd(w0, B.beta, q0);
+            w1 = madd(w1, B.beta, q1);
+        }
+        pairStore<T, EVEN>(B.d, c0, on1, z0, z1);
+        pairStore<T, EVEN>(B.q, c0, on1, w0, w1);
+        dot = fma((double)w0, (double)z0, dot);
+        if (on1) dot = fma((double)w1, (double)z1, dot);
+    } else if constexpr (MODE == PASS_BLACK0 || MODE == PASS_BLACK) {
+        const T rv = B.r[c];
+        if (cOn) {
+            const T dg = diagOf(c, cd);
+            T zc = T(0);
+            if (dg > T(0)) zc = l0Div(sum(Plus{}, rv, gen), cd, dg);
+            B.z[c] = zc;
+        }
+    } else if constexpr (MODE == PASS_RED) {
+        const T rv = B.r[c], rb = B.r[cIn];
+        if (cOn) {
+            const T dg = diagOf(c, cd);
+            T zc = T(0);
+            if (dg > T(0)) zc = l0Div(sum(Plus{}, rv, gen), cd, dg);
+            B.z[c] = zc;
+            if constexpr (sizeof(R) == 4) (o ? t1 : t0) = f2prod(rv, zc);
+            else dot = fma(rv, zc, dot);
+        }
+        if (inOn) {
+            if constexpr (sizeof(R) == 4) (o ? t0 : t1) = f2prod(rb, vIn);
+            else dot = fma(rb, vIn, dot);
+        }
+    } else {   // PASS_RES: the four lanes of a block hold its red cells in ascending order
+        const int* af = g.lv[0].agg;
+        const int a = cOn ? af[c] : -1, ab = inOn ? af[cIn] : -1;
+        T res = T(0);
+        if (a >= 0) res = sum(Plus{}, T(0), gen);
+        T acc = T(0), accB = T(0);
+        const bool apart = __any_sync(0xffffffffu, ab >= 0 && ab != a);   // pieces of a block that are not joined
+#pragma unroll
+        for (int l = 0; l < 4; ++l) {
+            const int al = __shfl_sync(0xffffffffu, a, l, 4);
+            const T rl = __shfl_sync(0xffffffffu, res, l, 4);
+            if (al >= 0 && al == a) acc = acc + rl;
+            if (apart && al >= 0 && al == ab) accB = accB + rl;
+        }
+        restrictTo(g, a, acc);
+        if (ab != a) restrictTo(g, ab, accB);
+    }
+}
+
+// ---- team barrier ---------------------------------------------------------------
+struct Team {
+    unsigned* bar;           // arrivals since the start of the solve
+    unsigned* errWord;
+    unsigned target;
+    int size, rank, first;   // CTAs, this CTA's place, the team's first CTA
+};
+
+// every thread of every CTA of the team calls it; false: the wait ran out and
+// the kernel has to end. *gaveUp is shared memory, 0 at first.
+__device__ __forceinline__ bool teamSync(Team& t, volatile int* gaveUp) {
+    __syncthreads();
+    if (t.size == 1) return true;
+    t.target += (unsigned)t.size;
+    if (threadIdx.x == 0) {
+        asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(t.bar) : "memory");
+        unsigned seen;
+        asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(seen) : "l"(t.bar) : "memory");
+        if ((int)(seen - t.target) < 0) {
+            const long long t0 = clock64();
+            do {
+                asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(seen) : "l"(t.bar) : "memory");
+                if (clock64() - t0 > TEAM_WAIT_CYCLES) {
+                    atomicOr(t.errWord, ERR_TEAM_WAIT);
+                    *gaveUp = 1;
+                    break;
+                }
+            } while ((int)(seen - t.target) < 0);
+        }
+    }
+    __syncthreads();
+    return *gaveUp == 0;
+}
+
+// ---- sums ----------------------------------------------------------------------
+__device__ __forceinline__ F2 f2Load(const double* p) {
+    const float2 v = *reinterpret_cast<const float2*>(p);
+    return F2{v.x, v.y};
+}
+__device__ __forceinline__ void f2Store(double* p, F2 v) { *reinterpret_cast<float2*>(p) = make_float2(v.hi, v.lo); }
+// a float as a double by its bits (a conversion instruction takes some hundred
+// cycles here); zeros and numbers below the normal range take the conversion
+__device__ __forceinline__ double widen(float f) {
+    const unsigned b = __float_as_uint(f), e = b & 0x7f800000u;
+    if (e == 0u || e == 0x7f800000u) return (double)f;
+    return __hiloint2double((int)((b & 0x80000000u) | (((b & 0x7fffffffu) >> 3) + 0x38000000u)), (int)(b << 29));
+}
+__device__ __forceinline__ double warpSumAll(double v) {   // the same value in every lane
+    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    return v;
+}
+// FP32: the sum of a scenario's nt tiles, four to a CTA-sized group whose sum is
+// rounded to FP64, in every lane of warp 0. The orders are those of a 128-thread
+// CTA per 128 blocks and one such CTA over their sums.
+__device__ __forceinline__ double teamTotalF2(const double* part, int nt, double* sh) {
+    const int tid = (int)threadIdx.x, n4 = (nt + 3) / 4;
+    if (tid < 128) {
+        double acc = 0;
+        for (int i = tid; i < n4; i += 128) {
+            F2 w[4];
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+                w[e] = F2{0.f, 0.f};
+                if (4 * i + e < nt) {
+                    const float2 v = __ldcg(reinterpret_cast<const float2*>(part + 4 * i + e));
+                    w[e] = F2{v.x, v.y};
+                }
+            }
+            const F2 v = f2add(f2add(w[0], w[2]), f2add(w[1], w[3]));
+            acc += widen(v.hi) + widen(v.lo);
+        }
+        acc = warpSum(acc);
+        if ((tid & 31) == 0) sh[tid >> 5] = acc;
+    }
+    __syncthreads();
+    return (sh[0] + sh[2]) + (sh[1] + sh[3]);
+}
+// The sum of a scenario's nt partials, in every lane of warp 0; the whole CTA
+// calls it and may read what other warps wrote to shared memory before the call.
+// Up to 512 partials warp 0 adds alone, beyond that eight warps add 256 columns
+// first. What counts here is the chain of FP64 instructions (an addition takes
+// some hundred cycles, an FP32-to-FP64 conversion more): the loads of sixteen
+// values are in flight together, and they are added as a tree.
+__device__ __forceinline__ double teamTotal(const double* part, int nt, double* sh256) {
+    const int tid = (int)threadIdx.x;
+    double acc = 0;
+    const int step = nt > 512 ? 256 : 32;
+    if (tid < step) {
+        for (int i0 = tid; i0 < nt; i0 += 16 * step) {
+            double v[16];
+#pragma unroll
+            for (int e = 0; e < 16; ++e) {
+                const int i = i0 + e * step;
+                v[e] = i < nt ? __ldcg(part + i) : 0.0;
+            }
+#pragma unroll
+            for (int e = 0; e < 16; e += 4)
+                if ((i0 & ~31) + e * step < nt) acc += (v[e] + v[e + 1]) + (v[e + 2] + v[e + 3]);
+        }
+        if (step == 256) sh256[tid] = acc;
+    }
+    __syncthreads();
+    if (tid < 32) {
+        if (step == 256) {
+            double v[8];
+#pragma unroll
+            for (int w = 0; w < 8; ++w) v[w] = sh256[w * 32 + tid];
+            acc = ((v[0] + v[1]) + (v[2] + v[3])) + ((v[4] + v[5]) + (v[6] + v[7]));
+        }
+        acc = warpSumAll(acc);
+    }
+    return acc;
+}
+
+// The maximum of non-negative values through their bit patterns, in integer
+// instructions (a NaN never enters: the callers' mx drops it)
+__device__ __forceinline__ float warpMaxPos(float v) {
+    return __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(v)));
+}
+__device__ __forceinline__ double warpMaxPos(double v) {
+    const unsigned long long b = (unsigned long long)__double_as_longlong(v);
+    const unsigned hi = (unsigned)(b >> 32), mhi = __reduce_max_sync(0xffffffffu, hi);
+    const unsigned mlo = __reduce_max_sync(0xffffffffu, hi == mhi ? (unsigned)b : 0u);
+    return __longlong_as_double((long long)(((unsigned long long)mhi << 32) | mlo));
+}
+// CTA-wide max of non-negative values into *dst (this CTA's slot)
+template <class V>
+__device__ __forceinline__ void ctaMaxStore(double* dst, V v, V* sh) {
+    v = warpMaxPos(v);
+    const int w = (int)(threadIdx.x >> 5), l = (int)(threadIdx.x & 31), nw = (int)(blockDim.x >> 5);
+    if (l == 0) sh[w] = v;   // the previous call's reader is past a team barrier
+    __syncthreads();
+    if (w == 0) {
+        const V x = warpMaxPos(l < nw ? sh[l] : V(0));
+        if (l == 0) *dst = (double)x;
+    }
+}
+
+// ---- coarse rows in shared memory ---------------------------------------------
+// A warp's rows of a coarse level are the same in every V-cycle, so their
+// couplings are kept in the CTA's shared memory, transposed over the lanes: a
+// sweep then waits for one memory latency (its neighbours' values) instead of
+// three (row start, column, value). Rows that do not fit the pool, or have more
+// than ROW_WIDEST couplings, are read from the level's arrays every time.
+constexpr int ROW_WIDEST = 24, ROW_CHUNKS = 2;
+struct RowSet {
+    int off;                 // words from the pool's start; -1: not kept
+    int width;               // couplings of the longest row
+};
+template <class R>
+struct RowView {
+    const R* diag;           // [32]: the diagonal; FP64 sweeps (toNext): omega / diagonal
+    const R* val;            // [width][32]
+    const int *own, *col, *next;   // [32], [width][32] each
+};
+template <class R>
+__device__ __forceinline__ RowView<R> rowView(const unsigned* pool, const RowSet& s) {
+    RowView<R> v;
+    v.diag = reinterpret_cast<const R*>(pool + s.off);
+    v.val = v.diag + 32;
+    v.own = reinterpret_cast<const int*>(v.val + 32 * s.width);
+    v.col = v.own + 32;
+    v.next = v.col + 32 * s.width;
+    return v;
+}
+// keep row I of level l in lane's column of a new set (I < 0: none): diagonal, the
+// row's aggregate (toNext) or the row itself, couplings, their columns and
+// (toNext) their aggregates. Short rows end in couplings of 0 to the row itself.
+template <class R>
+__device__ __forceinline__ void keepRows(const Level<R>& L, int I, bool toNext, unsigned* pool, int* used, int words,
+                                         RowSet* out) {
+    const int lane = (int)(threadIdx.x & 31);
+    const int q0 = I >= 0 ? L.rowStart[I] : 0, n = I >= 0 ? L.rowStart[I + 1] - q0 : 0;
+    RowSet s;
+    s.width = __reduce_max_sync(0xffffffffu, n);
+    constexpr int RW = (int)sizeof(R) / 4;
+    const int need = 32 * ((1 + s.width) * RW + 1 + s.width * (toNext ? 2 : 1));
+    int off = -1;
+    if (lane == 0 && s.width <= ROW_WIDEST) {
+        off = atomicAdd(used, need);
+        if (off + need > words) off = -1;
+    }
+    s.off = __shfl_sync(0xffffffffu, off, 0);
+    if (s.off >= 0) {
+        const RowView<R> v = rowView<R>(pool, s);
+        const_cast<R*>(v.diag)[lane] = I < 0 ? R(0) : toNext && sizeof(R) == 8 ? L.omd[I] : L.diag[I];
+        const_cast<int*>(v.own)[lane] = I < 0 ? -1 : toNext ? L.agg[I] : I;
+        for (int e = 0; e < s.width; ++e) {
+            const int col = e < n ? L.col[q0 + e] : max(I, 0);
+            const_cast<R*>(v.val)[32 * e + lane] = e < n ? L.val[q0 + e] : R(0);
+            const_cast<int*>(v.col)[32 * e + lane] = col;
+            if (toNext) const_cast<int*>(v.next)[32 * e + lane] = L.agg[col];
+        }
+    }
+    if (lane == 0) *out = s;
+}
+// jacobiRow for a kept row
+template <class R>
+__device__ __forceinline__ void jacobiKept(const Scn<R>& g, const RowView<R>& v, int width, int I, int l, int mode) {
+    using T = R;
+    const Level<R>& L = g.lv[l];
+    if (I >= L.n) return;
+    const int lane = (int)(threadIdx.x & 31);
+    const bool toX = mode == 1 || mode == 3, prolong = mode == 2 || mode == 3;
+    const R* in = toX ? L.y : L.x;
+    const R* xc = g.lv[l + 1].x;
+    R* out = toX ? L.x : L.y;
+    T s = L.b[I], xI = in[I];
+    T cI = T(0);
+    if (prolong) cI = xc[v.own[lane]];
+    for (int e0 = 0; e0 < width; e0 += 8) {
+        T x[8], c[8];
+#pragma unroll
+        for (int e = 0; e < 8; ++e) {
+            const int at = 32 * min(e0 + e, width - 1) + lane;
+            x[e] = in[v.col[at]];
+            if (prolong) c[e] = xc[v.next[at]];
+        }
+#pragma unroll
+        for (int e = 0; e < 8; ++e)
+            if (e0 + e < width) s = madd(s, v.val[32 * (e0 + e) + lane], prolong ? x[e] + c[e] : x[e]);
+    }
+    if (prolong) xI = xI + cI;
+    out[I] = jacobiValue(s, xI, v.diag[lane], v.diag[lane]);
+}
+// resRestrictJac0Warp for kept rows: lane c of the eight lanes of unknown J has J's
+// child c
+template <class R>
+__device__ __forceinline__ void resRestrictKept(const Scn<R>& g, const RowView<R>& v, int width, int jBase, int l) {
+    using T = R;
+    const Level<R>& L = g.lv[l];
+    const Level<R>& C = g.lv[l + 1];
+    const int lane = (int)(threadIdx.x & 31), J = jBase + lane / RRJ_LANES;
+    const R* it = g.smooth1 ? L.y : L.x;
+    const int I = v.own[lane];
+    const T dg = v.diag[lane];
+    T bI = T(0), xI = T(0);
+    if (I >= 0) { bI = L.b[I]; xI = it[I]; }
+    T s = madd(bI, -dg, xI);
+    for (int e0 = 0; e0 < width; e0 += 8) {
+        T x[8];
+#pragma unroll
+        for (int e = 0; e < 8; ++e) x[e] = it[v.col[32 * min(e0 + e, width - 1) + lane]];
+#pragma unroll
+        for (int e = 0; e < 8; ++e) if (e0 + e < width) s = madd(s, v.val[32 * (e0 + e) + lane], x[e]);
+    }
+    if (!(dg > 0)) s = T(0);
+    const unsigned valid = __ballot_sync(0xffffffffu, I >= 0);
+    const int lane0 = lane & ~(RRJ_LANES - 1);
+    T acc = T(0);
+#pragma unroll
+    for (int q = 0; q < RRJ_LANES; ++q) {
+        const T rq = __shfl_sync(0xffffffffu, s, lane0 + q);
+        if ((valid >> (lane0 + q)) & 1u) acc = acc + rq;
+    }
+    if (J < C.n && lane == lane0) {
+        C.b[J] = acc;
+        if (l + 1 < g.nLevels - 1) C.y[J] = jacobiValue(acc, T(0), C.diag[J], C.omd[J]);
+    }
+}
+
+// ---- teams ------------------------------------------------------------------------
+// CTAs per scenario: the smallest bound on work / CTAs that the grid can meet
+// (bisection on the bound), at least one CTA and at most one per tile. One
+// warp; every CTA computes the same division.
+template <class R>
+__device__ void divideTeams(const Scn<R>* S, int n, int G, int* first) {
+    __shared__ float work[MAX_BATCH];
+    __shared__ int most[MAX_BATCH];
+    for (int s = threadIdx.x; s < n; s += blockDim.x) {
+        const Scn<R>& g = S[s];
+        const int nblk = (int)g.dvL0[1].d * ((g.nz + 1) >> 1);
+        const SolveTiling tl = solveTiling<R>(nblk);
+        most[s] = tl.warps == 1 ? (tl.nt + 1) / 2 : tl.nt;
+        work[s] = (float)nblk * (float)(g.sv[SV_WITERS] + 2.0);
+    }
+    __syncthreads();
+    if (threadIdx.x < 32) {
+        auto ctas = [&](int s, float bound) { return min(most[s], max(1, (int)ceilf(work[s] / bound))); };
+        float hi = 0;
+        for (int s = threadIdx.x; s < n; s += 32) hi = fmaxf(hi, work[s]);
+        hi = warpMax(hi);
+        float lo = 0;
+        for (int it = 0; it < 20; ++it) {
+            const float mid = 0.5f * (lo + hi);
+            int sum = 0;
+            for (int s = threadIdx.x; s < n; s += 32) sum += mid > 0 ? ctas(s, mid) : most[s];
+            sum = __reduce_add_sync(0xffffffffu, sum);
+            if (sum <= G) hi = mid; else lo = mid;
+        }
+        int base = 0;
+        for (int s0 = 0; s0 < n; s0 += 32) {
+            const int s = s0 + (int)threadIdx.x;
+            int v = s < n ? (hi > 0 ? ctas(s, hi) : 1) : 0;
+            for (int o = 1; o < 32; o <<= 1) {
+                const int u = __shfl_up_sync(0xffffffffu, v, o);
+                if ((int)threadIdx.x >= o) v += u;
+            }
+            if (s < n) first[s + 1] = base + v;
+            base += __shfl_sync(0xffffffffu, v, 31);
+        }
+        if (threadIdx.x == 0) first[0] = 0;
+    }
+    __syncthreads();
+}
+
+// ---- the kernel ----------------------------------------------------------------------
+template <class R>
+__global__ void __launch_bounds__(SolveCfg<R>::T, 1)
+k_solve(const Scn<R>* __restrict__ S, SolveArgs a) {
+    using T = R;
+    constexpr int TH = SolveCfg<R>::T;
+    constexpr bool kMixed = sizeof(R) == 4;
+    __shared__ __align__(16) unsigned long long graw[sizeof(Scn<R>) / 8];
+    extern __shared__ __align__(16) unsigned pool[];
+    __shared__ CgState cg;
+    __shared__ double shSum[256], shZone[8], shMax[2];
+    __shared__ RowSet rowsJ[MAX_LEVELS][TH / 32][ROW_CHUNKS], rowsR[MAX_LEVELS][TH / 32][ROW_CHUNKS];
+    __shared__ int poolUsed;
+    __shared__ double shDot[2][TH];   // the tiles' dot products, by turns
+    __shared__ double shMx[32];
+    __shared__ int first[MAX_BATCH + 1];
+    __shared__ int gaveUp;
+    static_assert(sizeof(Scn<R>) % 8 == 0, "descriptors are copied as 8-byte words");
+    const int tid = (int)threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int G = (int)gridDim.x, b = (int)blockIdx.x;
+    if (tid == 0) gaveUp = 0;
+    Team team;
+    int s = b, sStep = G;
+    team.size = 1; team.rank = 0; team.first = b; team.target = 0; team.bar = nullptr; team.errWord = nullptr;
+    if (a.nscn <= G) {
+        divideTeams(S, a.nscn, G, first);
+        s = a.nscn;
+        for (int q = 0; q < a.nscn; ++q)
+            if (b >= first[q] && b < first[q + 1]) { s = q; break; }
+        if (s >= a.nscn) return;   // no work for this CTA
+        sStep = a.nscn;
+        team.first = first[s];
+        team.size = first[s + 1] - first[s];
+        team.rank = b - team.first;
+    }
+    const Scn<R>& g = *reinterpret_cast<const Scn<R>*>(graw);
+    for (; s < a.nscn; s += sStep) {
+        __syncthreads();
+        {   // the scenario's descriptor and scalars
+            const unsigned long long* src = reinterpret_cast<const unsigned long long*>(S + s);
+            for (int i = tid; i < (int)(sizeof(Scn<R>) / 8); i += TH) graw[i] = src[i];
+            __syncthreads();
+            if (tid == 0) {
+                const double* sv = g.sv;
+                cg.rz = 1;   // not yet known: a divisor whose quotient is not used
+                cg.alpha = cg.beta = cg.dq = 0;
+                cg.rmax = sv[SV_RMAX];
+                cg.r64max = 0;
+                cg.pres = sv[SV_PRES];
+                cg.prel = sv[SV_PREL];
+                cg.tol = g.tol;
+                cg.relTol = g.relTol;
+                cg.inv = sv[SV_INV];
+                cg.bmax = sv[SV_BMAX];
+                cg.relStop = g.relTol > 0 ? g.relTol * cg.bmax : -1.0;
+                cg.relStop2 = 2.0 * cg.relStop;
+                cg.tolHalf = 0.5 * g.tol;
+                cg.haveB = cg.bmax > 0;
+                cg.haveRel = g.relTol > 0;
+                cg.it = cg.done = cg.repl = cg.brk = 0;
+                poolUsed = 0;
+            }
+            team.bar = g.teamBar;
+            team.errWord = g.errWord;
+            __syncthreads();
+        }
+        const int N = g.N, nl = g.nLevels;
+        const int nblk = (int)g.dvL0[1].d * ((g.nz + 1) >> 1);
+        const SolveTiling tl = solveTiling<R>(nblk);
+        const int nt = tl.nt;
+        const int t0 = (int)((long long)nt * team.rank / team.size), t1 = (int)((long long)nt * (team.rank + 1) / team.size);
+        const int rank = team.rank, size = team.size;
+        double* const partDq = g.part + (size_t)PS_DQ * g.partStride;
+        double* const partRz = g.part + (size_t)PS_RZ * g.partStride;
+        double* const maxR = a.maxPart + 2 * b;
+        const bool closed = kMixed && g.nClosed > 0;
+        SolveBufs<R> B;
+        B.p = g.p; B.z = g.z; B.q = g.q; B.r = g.r; B.d = g.d;
+        B.dNew = nullptr; B.alpha = T(0); B.beta = T(0); B.haveD = false;
+
+#define PHX_TEAM_SYNC() do { if (!teamSync(team, &gaveUp)) return; } while (0)
+        // one pass over the team's tiles
+        const int slot = warp / tl.warps, slots = TH / 32 / tl.warps, wt = warp - slot * tl.warps;
+        int turn = 0;
+        auto pairs = [&](auto mode, auto even, double* part, T& rm, bool writeZ) {
+            constexpr int MODE = decltype(mode)::value;
+            constexpr bool kDot = MODE == PASS_APPLY || MODE == PASS_RED;
+            for (int t = t0 + slot; t < t1; t += slots) {
+                double dot = 0;
+                F2 e0{0.f, 0.f}, e1{0.f, 0.f};
+                for (int q = 0; q < tl.reps; ++q)
+                    solvePair<R, MODE, decltype(even)::value>(g, B, ((t * tl.reps + q) * tl.warps + wt) * 32 + lane, nblk,
+                                                              dot, e0, e1, rm, writeZ);
+                if constexpr (kDot && kMixed) {
+                    // a block's eight terms in ascending order over its four lanes, the
+                    // 32 blocks of the tile by one warp
+                    F2 acc = f2add(e0, e1);
+#pragma unroll
+                    for (int l = 1; l < 4; ++l) {
+                        const F2 before{__shfl_sync(0xffffffffu, acc.hi, l - 1, 4), __shfl_sync(0xffffffffu, acc.lo, l - 1, 4)};
+                        const F2 next = f2add(f2add(before, e0), e1);
+                        if ((lane & 3) == l) acc = next;
+                    }
+                    double* const sh = shDot[turn] + 32 * slot;
+                    turn ^= 1;
+                    if ((lane & 3) == 3) f2Store(sh + wt * 8 + (lane >> 2), acc);
+                    asm volatile("bar.sync %0, 128;" ::"r"(slot + 1) : "memory");
+                    if (wt == 0) {
+                        acc = warpSum(f2Load(sh + lane));
+                        if (lane == 0) f2Store(part + t, acc);
+                    }
+                } else if constexpr (kDot) {
+                    if (tl.warps > 1) {   // the tile's first warp adds the warps' lanes
+                        double* const sh = shDot[turn];
+                        turn ^= 1;
+                        sh[tid] = dot;
+                        asm volatile("bar.sync %0, %1;" ::"r"(slot + 1), "r"(tl.warps * 32) : "memory");
+                        if (wt == 0)
+                            for (int w = 1; w < tl.warps; ++w) dot += sh[tid + 32 * w];
+                    }
+                    if (wt == 0) {
+                        dot = warpSumAll(dot);
+                        if (lane == 0) part[t] = dot;
+                    }
+                }
+            }
+        };
+        auto pass = [&](auto mode, double* part, T& rm, bool writeZ) {
+            if (g.nx & 1) pairs(mode, std::false_type{}, part, rm, writeZ);
+            else pairs(mode, std::true_type{}, part, rm, writeZ);
+        };
+#define PHX_PASS(m, part, rm, wz) pass(std::integral_constant<int, m>{}, part, rm, wz)
+        // rows of a coarse level: a warp takes 32 consecutive rows, warps round-robin over the team
+        const int gw = warp * size + rank, nw = (TH / 32) * size;
+        for (int l = 1; l < nl - 1; ++l)
+            for (int m = 0; m < ROW_CHUNKS; ++m) {
+                const Level<R>& L = g.lv[l];
+                const Level<R>& C = g.lv[l + 1];
+                const int chunk = gw + m * nw, I = chunk * 32 + lane;
+                if (lane == 0) rowsJ[l][warp][m].off = rowsR[l][warp][m].off = -1;
+                __syncwarp();
+                if (chunk * 32 < L.n)
+                    keepRows(L, I < L.n ? I : -1, true, pool, &poolUsed, SolveCfg<R>::POOL / 4, &rowsJ[l][warp][m]);
+                if (chunk * (32 / RRJ_LANES) < C.n) {
+                    const int J = chunk * (32 / RRJ_LANES) + lane / RRJ_LANES, c = lane % RRJ_LANES;
+                    const int e0 = J < C.n ? L.childStart[J] : 0, nch = J < C.n ? L.childStart[J + 1] - e0 : 0;
+                    if (__reduce_max_sync(0xffffffffu, nch) <= RRJ_LANES)
+                        keepRows(L, c < nch ? L.child[e0 + c] : -1, false, pool, &poolUsed, SolveCfg<R>::POOL / 4,
+                                 &rowsR[l][warp][m]);
+                }
+                __syncwarp();
+            }
+        auto jacobiLevel = [&](int l, int mode) {
+            const int n = g.lv[l].n;
+            for (int m = 0, i = gw * 32; i < n; ++m, i += nw * 32) {
+                const RowSet rs = m < ROW_CHUNKS ? rowsJ[l][warp][m] : RowSet{-1, 0};
+                if (rs.off >= 0) jacobiKept(g, rowView<R>(pool, rs), rs.width, i + lane, l, mode);
+                else jacobiRow(g, i + lane, l, mode);
+            }
+        };
+        auto restrictLevel = [&](int l) {
+            constexpr int PER = 32 / RRJ_LANES;
+            for (int m = 0, j = gw * PER; j < g.lv[l + 1].n; ++m, j += nw * PER) {
+                const RowSet rs = m < ROW_CHUNKS ? rowsR[l][warp][m] : RowSet{-1, 0};
+                if (rs.off >= 0) resRestrictKept(g, rowView<R>(pool, rs), rs.width, j, l);
+                else resRestrictJac0Warp(g, j, l);
+            }
+        };
+        // the cells of the grid, elementwise
+        auto cells = [&](auto f) {
+            for (int c = rank * TH + tid; c < N; c += size * TH) f(c);
+        };
+        // sums over a closed zone by the first 256 threads (the order of a 256-thread CTA)
+        auto zoneMean = [&](int zi, const R* v) -> double {
+            const int e0 = g.closedStart[zi], e1 = g.closedStart[zi + 1];
+            double acc = 0;
+            if (tid < TPB)
+                for (int e = e0 + tid; e < e1; e += TPB) acc += (double)v[g.closedCells[e]];
+            acc = warpSum(acc);
+            __syncthreads();
+            if (lane == 0 && warp < 8) shZone[warp] = acc;
+            __syncthreads();
+            const double sum = ((shZone[0] + shZone[4]) + (shZone[2] + shZone[6])) +
+                               ((shZone[1] + shZone[5]) + (shZone[3] + shZone[7]));
+            return e1 > e0 ? sum / (double)(e1 - e0) : 0.0;
+        };
+        auto zoneCenter = [&](R* v) {
+            for (int zi = rank; zi < g.nClosed; zi += size) {
+                const double mean = zoneMean(zi, v);
+                for (int e = g.closedStart[zi] + tid; e < g.closedStart[zi + 1]; e += TH) {
+                    const int c = g.closedCells[e];
+                    if (g.diag[c] > 0) v[c] = (R)((double)v[c] - mean);
+                }
+            }
+        };
+        // mixed path: r = b - A p64 in FP64 (k_mx_res64's expressions), p = 0; closed
+        // zones: the zone mean of r removed
+        auto residual64 = [&](double& rm) {
+            const int nx = g.nx, ny = g.ny, nz = g.nz, sxy = nx * ny;
+            const double* x = g.p64;
+            cells([&](int c) {
+                // every load up front at clamped places; a coded cell's coefficients are 0 or 1
+                const unsigned cd = g.code0[c];
+                const double x0 = x[c], xm = x[max(c - 1, 0)], xp = x[min(c + 1, N - 1)], ym = x[max(c - nx, 0)],
+                             yp = x[min(c + nx, N - 1)], zm = x[max(c - sxy, 0)], zp = x[min(c + sxy, N - 1)];
+                const double bc = (double)g.b[c];
+                double r = 0;
+                if (!(cd & CODE_GENERAL)) {
+                    const int cnt = __popc(cd & 63u) + (cd >> 7);
+                    double acc = __dmul_rn((double)cnt, x0);
+                    acc -= (cd & 1u) ? xm : 0.0;
+                    acc -= (cd & 2u) ? xp : 0.0;
+                    acc -= (cd & 4u) ? ym : 0.0;
+                    acc -= (cd & 8u) ? yp : 0.0;
+                    acc -= (cd & 16u) ? zm : 0.0;
+                    acc -= (cd & 32u) ? zp : 0.0;
+                    r = cnt > 0 ? bc - acc : 0.0;
+                } else {
+                    const double dg = (double)g.diag[c];
+                    int i, j, k;
+                    ijkOf(g, 0, c, i, j, k);
+                    const int fx0 = i + (nx + 1) * (j + ny * k), fy0 = i + nx * (j + (ny + 1) * k);
+                    double acc = dg * x0;
+                    if (i > 0) acc -= (double)g.a0x[fx0] * xm;
+                    if (i < nx - 1) acc -= (double)g.a0x[fx0 + 1] * xp;
+                    if (j > 0) acc -= (double)g.a0y[fy0] * ym;
+                    if (j < ny - 1) acc -= (double)g.a0y[fy0 + nx] * yp;
+                    if (k > 0) acc -= (double)g.a0z[c] * zm;
+                    if (k < nz - 1) acc -= (double)g.a0z[c + sxy] * zp;
+                    if (dg > 0) r = bc - acc;
+                }
+                B.r[c] = (R)r;
+                g.p[c] = 0;
+                const int z = g.nClosed > 0 ? g.zone[c] : -1;
+                if (!(z >= 0 && !g.zoneOpen[z])) rm = mx(rm, fabs(r));
+            });
+        };
+        auto zoneProject = [&](double& rm) {
+            for (int zi = rank; zi < g.nClosed; zi += size) {
+                const double mean = zoneMean(zi, B.r);
+                for (int e = g.closedStart[zi] + tid; e < g.closedStart[zi + 1]; e += TH) {
+                    const int c = g.closedCells[e];
+                    if (g.diag[c] > 0) {
+                        const R v = (R)((double)B.r[c] - mean);
+                        B.r[c] = v;
+                        rm = fmax(rm, fabs((double)v));
+                    }
+                }
+            }
+        };
+
+        if (kMixed && !a.vcycleOnly) {
+            double rm = 0;
+            residual64(rm);
+            if (closed) {
+                PHX_TEAM_SYNC();
+                zoneProject(rm);
+            }
+            ctaMaxStore(maxR + 1, rm, shMx);
+            PHX_TEAM_SYNC();
+        }
+
+        T none = T(0);
+        for (int phase = a.vcycleOnly ? 2 : 0, loop = 0;; phase = 1, ++loop) {
+            bool haveRed = false;   // the update has set the red cells of z
+            if (phase == 1) {
+                B.beta = (T)cg.beta;
+                B.haveD = cg.it > 0;
+                if (kMixed) {   // the neighbours' previous d is read: two buffers by turns
+                    B.d = cg.it & 1 ? g.tmp[0] : g.d;
+                    B.dNew = cg.it & 1 ? g.d : g.tmp[0];
+                }
+                PHX_PASS(PASS_APPLY, partDq, none, false);
+                PHX_TEAM_SYNC();
+                const double total = kMixed ? teamTotalF2(partDq, nt, shSum) : teamTotal(partDq, nt, shSum);
+                if (tid == 0) {
+                    cg.dq = total;
+                    if (cg.brk == 1) {   // the iteration after a breakdown: no update, then a restart
+                        cg.alpha = 0;
+                        cg.brk = 2;
+                    } else if (total <= 0) {
+                        cg.done = 1;
+                    } else {
+                        cg.alpha = cg.rz / total;
+                    }
+                }
+                __syncthreads();
+                if (cg.done != 0) break;
+                B.alpha = (T)cg.alpha;
+                const bool repl = kMixed && cg.repl != 0;
+                haveRed = !repl && !closed;
+                T rm = T(0);
+                PHX_PASS(PASS_UPDATE, nullptr, rm, haveRed);
+                ctaMaxStore(maxR, rm, reinterpret_cast<T*>(shMx));
+                PHX_TEAM_SYNC();
+                if (closed) {
+                    zoneCenter(B.r);
+                    PHX_TEAM_SYNC();
+                }
+                if (repl) {
+                    cells([&](int c) { if (g.diag[c] > 0) g.p64[c] += (double)g.p[c]; });
+                    PHX_TEAM_SYNC();
+                    double rm64 = 0;
+                    residual64(rm64);
+                    if (closed) {
+                        PHX_TEAM_SYNC();
+                        zoneProject(rm64);
+                    }
+                    ctaMaxStore(maxR + 1, rm64, shMx);
+                    PHX_TEAM_SYNC();
+                }
+            }
+            // the V-cycle z = M r
+            if (!haveRed) {
+                PHX_PASS(PASS_RED0, nullptr, none, true);
+                PHX_TEAM_SYNC();
+            }
+            PHX_PASS(PASS_BLACK0, nullptr, none, true);
+            PHX_TEAM_SYNC();
+            PHX_PASS(PASS_RES, nullptr, none, true);
+            PHX_TEAM_SYNC();
+            for (int l = 1; l < nl - 1; ++l) {
+                if (!g.smooth1) {
+                    jacobiLevel(l, 1);
+                    PHX_TEAM_SYNC();
+                }
+                restrictLevel(l);
+                PHX_TEAM_SYNC();
+            }
+            if (g.lv[nl - 1].dense) {
+                for (int row = gw; row < g.lv[nl - 1].n; row += nw) coarseDenseRow(g, row);
+            } else if (rank == 0) {
+                coarseSerialTile(g);
+            }
+            PHX_TEAM_SYNC();
+            for (int l = nl - 2; l >= 1; --l) {
+                if (g.smooth1) {
+                    jacobiLevel(l, 3);
+                } else {
+                    jacobiLevel(l, 2);
+                    PHX_TEAM_SYNC();
+                    jacobiLevel(l, 1);
+                }
+                PHX_TEAM_SYNC();
+            }
+            PHX_PASS(PASS_BLACK, nullptr, none, true);
+            PHX_TEAM_SYNC();
+            PHX_PASS(PASS_RED, partRz, none, true);
+            if (phase == 2) return;
+            PHX_TEAM_SYNC();
+            // r.z, the maxima, beta and the stop test
+            if (warp >= TH / 32 - 2) {   // the maxima of the recursion and of the FP64 residual
+                const int which = warp - (TH / 32 - 2);
+                const double* mp = a.maxPart + 2 * team.first + which;
+                double m = 0;
+                for (int i = lane; i < size; i += 32) m = mx(m, __ldcg(mp + 2 * i));
+                m = warpMaxPos(m);
+                if (lane == 0) shMax[which] = m;
+            }
+            const double total = kMixed ? teamTotalF2(partRz, nt, shSum + 4) : teamTotal(partRz, nt, shSum);
+            if (warp == 0) {
+                const double rmax = phase == 1 ? shMax[0] : cg.rmax;
+                const double r64 = kMixed && (phase == 0 || cg.repl != 0) ? shMax[1] : 0.0;
+                const CgTests ts = cgTests(cg, total, rmax, r64);
+                if (lane == 0) {
+                    closeCgIteration(g, cg, phase, total, ts);
+                    if (loop >= a.cap) cg.done = 1;
+                }
+            }
+            if (closed) {
+                zoneCenter(B.z);
+                PHX_TEAM_SYNC();
+            }
+            __syncthreads();
+            if (cg.done != 0) break;
+        }
+        // mixed path: p64 += e and its FP32 copy (written before the team's last barrier)
+        if (kMixed)
+            cells([&](int c) {
+                double v = g.p64[c];
+                if (g.diag[c] > 0) v += (double)g.p[c];
+                g.p64[c] = v;
+                g.p[c] = (R)v;
+            });
+        if (rank == 0 && tid == 0) {
+            double* sv = g.sv;
+            sv[SV_RZ] = cg.rz;
+            sv[SV_ALPHA] = cg.alpha;
+            sv[SV_BETA] = cg.beta;
+            sv[SV_DQ] = cg.dq;
+            sv[SV_RMAX] = 0;
+            sv[SV_IT] = sv[SV_PITERS] = cg.it;
+            sv[SV_DONE] = 1;
+            sv[SV_PRES] = cg.pres;
+            sv[SV_PREL] = cg.prel;
+            if (kMixed) sv[SV_HAVEPREV] = 1;
+        }
+#undef PHX_PASS
+#undef PHX_TEAM_SYNC
+    }
+}
+
+}  // namespace phx

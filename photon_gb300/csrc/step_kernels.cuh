@@ -73,7 +73,6 @@ __device__ bool lastCtaSum(const Scn<R>& g, int slot, int tile, int ntiles, V vT
 }
 
 __device__ __forceinline__ int ntilesOf(const Dom& d, int s) { return __ldg(d.start + s + 1) - __ldg(d.start + s); }
-__device__ __forceinline__ int ntilesOf(const ADom& d, int s) { return d.start[s + 1] - d.start[s]; }
 
 // ---------------------------------------------------------------------------
 // Solver::stableDt (src/sim/gasphase.cpp:63-70) and the injection amounts of
@@ -124,6 +123,8 @@ __global__ void k_begin(const Scn<R>* __restrict__ S, Dom dom, int computeDt, do
         sv[SV_SRC_MF + q] = mf;
     }
     sv[SV_FUELIN] = fuelIn;
+    sv[SV_WITERS] = sv[SV_PITERS];
+    *g.teamBar = 0;
     // reductions of this step start from their neutral values
     sv[SV_MAXNU] = 0;
     sv[SV_MAXDIV] = 0;
