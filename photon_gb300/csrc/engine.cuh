@@ -237,7 +237,7 @@ struct Scenario {
         s.hrr = carve<R>(base, off, N); s.massSrc = carve<R>(base, off, N);
         s.lit = carve<uint8_t>(base, off, N); s.lit2 = carve<uint8_t>(base, off, N); s.pilot = carve<uint8_t>(base, off, N);
         for (int q = 0; q < 9; ++q) s.tmp[q] = carve<R>(base, off, N);
-        s.adv = kMixed ? nullptr : carve<double>(base, off, (size_t)ADV_REC * (NX + NY + NZ));
+        s.rho = kMixed ? nullptr : carve<R>(base, off, N);
         s.b = carve<R>(base, off, N); s.r = carve<R>(base, off, N); s.z = carve<R>(base, off, N);
         s.d = carve<R>(base, off, N); s.q = carve<R>(base, off, N);
         s.p64 = kMixed ? carve<double>(base, off, N) : nullptr;
@@ -1154,6 +1154,15 @@ public:
         ++launches;
     }
 
+    // the same with every CTA's tile split over `split` smaller CTAs
+    template <class K, class... A>
+    void launchSplit(const char* name, int d, int split, int threads, K kern, A... args) {
+        const int total = dom[d].total;
+        dom[d].total = total * split;
+        launch(name, d, threads, kern, args...);
+        dom[d].total = total;
+    }
+
     // the device error word: a bounded wait inside a kernel that ran out
     int checkDeviceError() {
         if (!dErr) return PHX_OK;
@@ -1226,12 +1235,11 @@ public:
         launch("k_turb_nu", D_CELLS, TPB, k_turb_nu<R>, S, dom[D_CELLS]);
     }
     void stHeat() {
-        if (!kMixed) {   // FP64: each interior face's conductive flux once
-            launch("k_heat_faces", D_FX, TPB, k_heat_faces<R>, (const Scn<R>*)dS, dom[D_FX], 0);
-            launch("k_heat_faces", D_FY, TPB, k_heat_faces<R>, (const Scn<R>*)dS, dom[D_FY], 1);
-            launch("k_heat_faces", D_FZ, TPB, k_heat_faces<R>, (const Scn<R>*)dS, dom[D_FZ], 2);
-        }
         launch("k_heat", D_CELLS, TPB, k_heat<R>, (const Scn<R>*)dS, dom[D_CELLS]);
+    }
+    // FP64, a stage on its own: the density the full step's earlier kernels leave behind
+    void stDensity() {
+        if (!kMixed) launch("k_rho", D_CELLS, TPB, k_rho<R>, (const Scn<R>*)dS, dom[D_CELLS]);
     }
     void stEnergy() { launch("k_energy", D_CELLS, TPB, k_energy<R>, (const Scn<R>*)dS, dom[D_CELLS]); }
     void stMomentum() {
@@ -1314,12 +1322,7 @@ public:
         return PHX_OK;
     }
     void stAdvect() {
-        if (!kMixed) {
-            launch("k_adv_faces", D_FX, TPB, k_adv_faces<R>, (const Scn<R>*)dS, dom[D_FX], 0);
-            launch("k_adv_faces", D_FY, TPB, k_adv_faces<R>, (const Scn<R>*)dS, dom[D_FY], 1);
-            launch("k_adv_faces", D_FZ, TPB, k_adv_faces<R>, (const Scn<R>*)dS, dom[D_FZ], 2);
-        }
-        launch("k_advect", D_CELLS, TPB, kMixed ? k_advect<R> : k_advect_2cta<R>, (const Scn<R>*)dS, dom[D_CELLS]);
+        launchSplit("k_advect", D_CELLS, TPB / ADV_TPB<R>, ADV_TPB<R>, k_advect<R>, (const Scn<R>*)dS, dom[D_CELLS]);
         swapBoth(4);
     }
     void stEnd() {
@@ -1424,12 +1427,12 @@ public:
         case PHX_STAGE_BEGIN: PHX_TRY(setDtMax(arg, nullptr)); stBegin(true, 0.0); break;
         case PHX_STAGE_COMBUSTION: stBegin(false, arg); stCombustion(); break;
         case PHX_STAGE_TURBULENCE: stTurbulence(); break;
-        case PHX_STAGE_HEAT: stBegin(false, arg); stHeat(); break;
+        case PHX_STAGE_HEAT: stBegin(false, arg); stDensity(); stHeat(); break;
         case PHX_STAGE_ENERGY: stBegin(false, arg); stEnergy(); break;
-        case PHX_STAGE_MOMENTUM: stBegin(false, arg); stMomentum(); break;
+        case PHX_STAGE_MOMENTUM: stBegin(false, arg); stDensity(); stMomentum(); break;
         case PHX_STAGE_LEAKAGE: stBegin(false, arg); stLeakage(); break;
         case PHX_STAGE_PROJECT: stBegin(false, arg); PHX_TRY(stProject()); break;
-        case PHX_STAGE_ADVECT: stBegin(false, arg); stAdvect(); break;
+        case PHX_STAGE_ADVECT: stBegin(false, arg); stDensity(); stAdvect(); break;
         case PHX_STAGE_END: stBegin(false, arg); stEnd(); break;
         default: err = "unknown stage"; return PHX_ERR_INVALID;
         }

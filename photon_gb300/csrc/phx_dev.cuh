@@ -70,10 +70,6 @@ template <class R>
 __host__ __device__ __forceinline__ constexpr double tStoredFromKd(double t) { return sizeof(R) == 4 ? t - K_T0 : t; }
 template <class R>
 __host__ __device__ __forceinline__ constexpr double tKFromStoredd(double s) { return sizeof(R) == 4 ? K_T0 + s : s; }
-// per-face transport record: upwind density, the 10 limited face values, and
-// the diffusion terms of the 9 species for the momentum-free and the mass form
-constexpr int ADV_RUP = 0, ADV_FACE = 1, ADV_DQ = ADV_FACE + NSC, ADV_MQ = ADV_DQ + NSC - 1,
-              ADV_REC = ADV_MQ + NSC - 1;
 constexpr int MAX_SRC = 16;      // burners + ignitions per scenario
 constexpr int MAX_LEVELS = 12;   // multigrid levels (the reference's cap)
 constexpr int TPB = 256;         // threads per CTA of the cell/face kernels
@@ -183,8 +179,7 @@ struct Scn {
     R *p, *S, *nu, *Pb, *Q, *Qr, *hrr, *massSrc;
     uint8_t *lit, *lit2, *pilot;
     R* tmp[9];                   // turbulence: cell-centre velocities and filter passes
-    double* adv;                 // FP64 path: per-face transport records (ADV_REC arrays over the
-                                 // NX + NY + NZ faces, x faces first), k_adv_faces -> k_advect
+    R* rho;                      // FP64 path: gas density of the current T and Pb (k_turb_nu, k_energy; null: mixed)
     // pressure solve
     R *b, *r, *z, *d, *q;
     double* p64;                 // mixed path: FP64 pressure; the FP32 iterate p holds the part not yet folded in
