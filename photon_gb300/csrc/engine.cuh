@@ -41,7 +41,8 @@ namespace phx {
 // dense coarse operators up to this many unknowns (n^2 reals)
 constexpr int DENSE_MAX = 4096;
 
-enum DomId { D_ONE = 0, D_CELLS, D_FX, D_FY, D_FZ, D_BX, D_BY, D_BZ, D_CZ, D_CC, D_LEAK, D_COUNT };
+// D_FACES, D_BND: the tiles of the x, then the y, then the z faces (boundary sides)
+enum DomId { D_ONE = 0, D_CELLS, D_FACES, D_BND, D_CZ, D_CC, D_LEAK, D_COUNT };
 
 // widest rows the contexts take (nx); wider grids are refused
 template <class R>
@@ -250,6 +251,7 @@ struct Scenario {
         s.sv = carve<double>(base, off, SV_COUNT);
         s.part = carve<double>(base, off, (size_t)PS_COUNT * partStride);
         s.partStride = partStride;
+        s.windU = carve<double>(base, off, geo.nz);
         s.cnt = carve<unsigned>(base, off, PS_COUNT + 4);
         s.teamBar = carve<unsigned>(base, off, 64);
         return off + 256;
@@ -495,12 +497,8 @@ struct Scenario {
         t[D_ONE] = 1;
         t[D_CELLS] = cdiv(N, TPB);
         t[D_LEAK] = cdiv((long long)leak.size() / 4, TPB);
-        t[D_FX] = cdiv(geo.NX(), TPB);
-        t[D_FY] = cdiv(geo.NY(), TPB);
-        t[D_FZ] = cdiv(geo.NZ(), TPB);
-        t[D_BX] = cdiv((long long)ny * nz * 2, TPB);
-        t[D_BY] = cdiv((long long)nx * nz * 2, TPB);
-        t[D_BZ] = cdiv((long long)nx * ny, TPB);
+        t[D_FACES] = cdiv(geo.NX(), TPB) + cdiv(geo.NY(), TPB) + cdiv(geo.NZ(), TPB);
+        t[D_BND] = cdiv(2LL * ny * nz, TPB) + cdiv(2LL * nx * nz, TPB) + cdiv((long long)nx * ny, TPB);
         t[D_CZ] = (int)Z.closed.size();
         t[D_CC] = cdiv((long long)Z.closedCells.size(), TPB);
     }
@@ -1042,6 +1040,7 @@ public:
         PHX_CK(cudaMemcpyAsync(dDomStart, starts.data(), starts.size() * sizeof(int), cudaMemcpyHostToDevice, st));
         tablesDirty = false;
         for (int s = 0; s < n; ++s) PHX_TRY(pushDescriptor(s, false));
+        if (n > 0) k_wind<R><<<dom[D_ONE].total, 128, 0, st>>>(dS, dom[D_ONE]);
         PHX_CK(cudaStreamSynchronize(st));
         return n > 0 ? setupSolve() : PHX_OK;
     }
@@ -1222,16 +1221,19 @@ public:
     void stBegin(bool computeDt, double dt) {
         launch("k_begin", D_ONE, 32, k_begin<R>, (const Scn<R>*)dS, dom[D_ONE], computeDt ? 1 : 0, dt);
     }
-    void stCombustion() {
+    // Stages. In the full step the double buffers are exchanged by kernels that do not
+    // read them (turbulence: the burning flags; energy: the velocities, ahead of
+    // momentum; the end of the step: the scalars); a stage on its own (alone) does it
+    // by k_swap, so that its result is in place when it returns.
+    void stCombustion(bool alone) {
         launch("k_combust", D_CELLS, TPB, k_combust<R>, (const Scn<R>*)dS, dom[D_CELLS]);
-        swapBoth(1);
+        if (alone) swapBoth(1);
     }
-    void stTurbulence() {
+    void stTurbulence(bool alone) {
         const Scn<R>* S = dS;
-        launch("k_turb_center", D_CELLS, TPB, k_turb_center<R>, S, dom[D_CELLS]);
-        launch("k_turb_filter", D_CELLS, TPB, k_turb_filter<R, 0>, S, dom[D_CELLS]);
-        launch("k_turb_filter", D_CELLS, TPB, k_turb_filter<R, 1>, S, dom[D_CELLS]);
-        launch("k_turb_filter", D_CELLS, TPB, k_turb_filter<R, 2>, S, dom[D_CELLS]);
+        launch("k_turb_x", D_CELLS, TPB, k_turb_x<R>, S, dom[D_CELLS], alone ? nullptr : dS);
+        if (!alone) swapHost(1);
+        launch("k_turb_y", D_CELLS, TPB, k_turb_y<R>, S, dom[D_CELLS]);
         launch("k_turb_nu", D_CELLS, TPB, k_turb_nu<R>, S, dom[D_CELLS]);
     }
     void stHeat() {
@@ -1241,16 +1243,14 @@ public:
     void stDensity() {
         if (!kMixed) launch("k_rho", D_CELLS, TPB, k_rho<R>, (const Scn<R>*)dS, dom[D_CELLS]);
     }
-    void stEnergy() { launch("k_energy", D_CELLS, TPB, k_energy<R>, (const Scn<R>*)dS, dom[D_CELLS]); }
-    void stMomentum() {
-        const Scn<R>* S = dS;
-        launch("k_momentum", D_FX, TPB, k_momentum<R, 0>, S, dom[D_FX]);
-        launch("k_momentum", D_FY, TPB, k_momentum<R, 1>, S, dom[D_FY]);
-        launch("k_momentum", D_FZ, TPB, k_momentum<R, 2>, S, dom[D_FZ]);
-        launch("k_mom_bnd", D_BX, TPB, k_mom_bnd<R>, S, dom[D_BX], 0);
-        launch("k_mom_bnd", D_BY, TPB, k_mom_bnd<R>, S, dom[D_BY], 1);
-        launch("k_mom_bnd", D_BZ, TPB, k_mom_bnd<R>, S, dom[D_BZ], 2);
-        swapBoth(2);
+    void stEnergy(bool alone) {
+        launch("k_energy", D_CELLS, TPB, k_energy<R>, (const Scn<R>*)dS, dom[D_CELLS], alone ? nullptr : dS);
+        if (!alone) swapHost(2);
+    }
+    void stMomentum(bool alone) {
+        if (alone) swapBoth(2);
+        launch("k_momentum", D_FACES, TPB, k_momentum<R>, (const Scn<R>*)dS, dom[D_FACES]);
+        launch("k_mom_bnd", D_BND, TPB, k_mom_bnd<R>, (const Scn<R>*)dS, dom[D_BND]);
     }
     void stLeakage() {
         launch("k_zone_integral", D_CZ, TPB, k_zone_integral<R>, (const Scn<R>*)dS, dom[D_CZ]);
@@ -1306,9 +1306,7 @@ public:
         const Scn<R>* S = dS;
         launch("k_zone_mean", D_CZ, TPB, k_zone_mean<R>, S, dom[D_CZ]);
         launch("k_zone_mean_sub", D_CC, TPB, k_zone_mean_sub<R>, S, dom[D_CC]);
-        launch("k_velcorr", D_FX, TPB, k_velcorr<R>, S, dom[D_FX], 0);
-        launch("k_velcorr", D_FY, TPB, k_velcorr<R>, S, dom[D_FY], 1);
-        launch("k_velcorr", D_FZ, TPB, k_velcorr<R>, S, dom[D_FZ], 2);
+        launch("k_velcorr", D_FACES, TPB, k_velcorr<R>, S, dom[D_FACES]);
     }
     int maxItersAll() const {
         int m = 0;
@@ -1321,13 +1319,14 @@ public:
         projectEpilogue();
         return PHX_OK;
     }
-    void stAdvect() {
+    void stAdvect(bool alone) {
         launchSplit("k_advect", D_CELLS, TPB / ADV_TPB<R>, ADV_TPB<R>, k_advect<R>, (const Scn<R>*)dS, dom[D_CELLS]);
-        swapBoth(4);
+        if (alone) swapBoth(4);
     }
-    void stEnd() {
+    void stEnd(bool alone) {
         const Scn<R>* S = dS;
-        launch("k_zone_pressure", D_ONE, 32, k_zone_pressure<R>, S, dom[D_ONE]);
+        launch("k_zone_pressure", D_ONE, 32, k_zone_pressure<R>, S, dom[D_ONE], alone ? nullptr : dS);
+        if (!alone) swapHost(4);
         launch("k_zone_pb", D_CC, TPB, k_zone_pb<R>, S, dom[D_CC]);
         launch("k_stats", D_CELLS, TPB, k_stats<R>, S, dom[D_CELLS]);
     }
@@ -1361,15 +1360,15 @@ public:
         PHX_CK(cudaStreamBeginCaptureToGraph(st, graph, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal));
         launches = 0;
         stBegin(true, 0.0);
-        stCombustion();
-        stTurbulence();
+        stCombustion(false);
+        stTurbulence(false);
         stHeat();
-        stEnergy();
-        stMomentum();
+        stEnergy(false);
+        stMomentum(false);
         stLeakage();
         PHX_TRY(stProject());
-        stAdvect();
-        stEnd();
+        stAdvect(false);
+        stEnd(false);
         cudaGraph_t done = nullptr;
         PHX_CK(cudaStreamEndCapture(st, &done));
         graphKernels = launches;
@@ -1392,15 +1391,15 @@ public:
         if (useGraph && !prof) return graphStep(dtMax, per);
         PHX_TRY(setDtMax(dtMax, per));
         stBegin(true, 0.0);
-        stCombustion();
-        stTurbulence();
+        stCombustion(false);
+        stTurbulence(false);
         stHeat();
-        stEnergy();
-        stMomentum();
+        stEnergy(false);
+        stMomentum(false);
         stLeakage();
         PHX_TRY(stProject());
-        stAdvect();
-        stEnd();
+        stAdvect(false);
+        stEnd(false);
         return checkLaunch();
     }
 
@@ -1425,15 +1424,15 @@ public:
         PHX_TRY(ensureTables());
         switch (which) {
         case PHX_STAGE_BEGIN: PHX_TRY(setDtMax(arg, nullptr)); stBegin(true, 0.0); break;
-        case PHX_STAGE_COMBUSTION: stBegin(false, arg); stCombustion(); break;
-        case PHX_STAGE_TURBULENCE: stTurbulence(); break;
+        case PHX_STAGE_COMBUSTION: stBegin(false, arg); stCombustion(true); break;
+        case PHX_STAGE_TURBULENCE: stTurbulence(true); break;
         case PHX_STAGE_HEAT: stBegin(false, arg); stDensity(); stHeat(); break;
-        case PHX_STAGE_ENERGY: stBegin(false, arg); stEnergy(); break;
-        case PHX_STAGE_MOMENTUM: stBegin(false, arg); stDensity(); stMomentum(); break;
+        case PHX_STAGE_ENERGY: stBegin(false, arg); stEnergy(true); break;
+        case PHX_STAGE_MOMENTUM: stBegin(false, arg); stDensity(); stMomentum(true); break;
         case PHX_STAGE_LEAKAGE: stBegin(false, arg); stLeakage(); break;
         case PHX_STAGE_PROJECT: stBegin(false, arg); PHX_TRY(stProject()); break;
-        case PHX_STAGE_ADVECT: stBegin(false, arg); stDensity(); stAdvect(); break;
-        case PHX_STAGE_END: stBegin(false, arg); stEnd(); break;
+        case PHX_STAGE_ADVECT: stBegin(false, arg); stDensity(); stAdvect(true); break;
+        case PHX_STAGE_END: stBegin(false, arg); stEnd(true); break;
         default: err = "unknown stage"; return PHX_ERR_INVALID;
         }
         PHX_TRY(checkLaunch());

@@ -75,6 +75,18 @@ __device__ bool lastCtaSum(const Scn<R>& g, int slot, int tile, int ntiles, V vT
 __device__ __forceinline__ int ntilesOf(const Dom& d, int s) { return __ldg(d.start + s + 1) - __ldg(d.start + s); }
 
 // ---------------------------------------------------------------------------
+// the wind profile's speed at every layer's cell centres, when a scenario's tables are built
+template <class R>
+__global__ void k_wind(const Scn<R>* __restrict__ S, Dom dom) {
+    PHX_PROLOGUE(dom);
+    if (g.windSpeed <= 0) return;
+    for (int k = threadIdx.x; k < g.nz; k += blockDim.x) {
+        const double z = g.oz + (k + 0.5) * g.dx;
+        const_cast<double*>(g.windU)[k] = g.windSpeed * pow(mx(z, 0.05) / 10.0, g.windExp);
+    }
+}
+
+// ---------------------------------------------------------------------------
 // Solver::stableDt (src/sim/gasphase.cpp:63-70) and the injection amounts of
 // injectIgnitions / injectBurners (src/sim/solver.cpp:271-280,
 // src/sim/gasphase.cpp:92-105, Burner::powerAt src/sim/solver.h:122-126).
@@ -256,62 +268,76 @@ __global__ void k_combust(const Scn<R>* __restrict__ S, Dom dom) {
 // ---------------------------------------------------------------------------
 // Solver::turbulence (src/sim/gasphase.cpp:163-218): cell-centre velocities,
 // the blocked-aware 1-2-1 test filter x -> y -> z per component, and the
-// Deardorff viscosity.
+// Deardorff viscosity, in three passes: the x filter forms the centre
+// velocities of its three cells itself, and the z filter goes straight into the
+// viscosity. A pass is one launch, about 3 us of a small building's step.
+//
+// the filtered value from a cell's own and its neighbours' (a missing or solid
+// neighbour counts as the cell itself)
+template <class T>
+__device__ __forceinline__ T turbFilter(T lo, T self, T hi) { return T(0.25) * lo + T(0.5) * self + T(0.25) * hi; }
+
+// Swap: 1 also exchanges the burning flags' buffers (combustion has written the
+// second; nothing here reads either), saving a launch of its own.
 template <class R>
-__global__ void k_turb_center(const Scn<R>* __restrict__ S, Dom dom) {
+__global__ void k_turb_x(const Scn<R>* __restrict__ S, Dom dom, Scn<R>* swap) {
     using T = R;
     PHX_PROLOGUE(dom);
+    if (swap && tile_ == 0 && threadIdx.x == 0) {
+        uint8_t* const l = swap[s_].lit;
+        swap[s_].lit = swap[s_].lit2;
+        swap[s_].lit2 = l;
+    }
     int c = tile_ * TPB + threadIdx.x;
     if (c >= g.N) return;
-    R *uc = g.tmp[0], *vc = g.tmp[1], *wc = g.tmp[2];
-    if (g.blocked[c]) { uc[c] = vc[c] = wc[c] = 0; return; }
+    if (g.blocked[c]) {
+#pragma unroll
+        for (int q = 0; q < 3; ++q) g.tmp[q][c] = g.tmp[3 + q][c] = 0;
+        return;
+    }
     const int nx = g.nx, ny = g.ny;
     int i, j, k;
     ijkOf(g, 0, c, i, j, k);
-    int fx0 = i + (nx + 1) * (j + ny * k);
-    int fy0 = i + nx * (j + (ny + 1) * k);
-    uc[c] = T(0.5) * (g.u[fx0] + g.u[fx0 + 1]);
-    vc[c] = T(0.5) * (g.v[fy0] + g.v[fy0 + nx]);
-    wc[c] = T(0.5) * (g.w[c] + g.w[c + nx * ny]);
+    const int fx0 = i + (nx + 1) * (j + ny * k), fy0 = i + nx * (j + (ny + 1) * k);
+    // the neighbours' faces at clamped places, used through selects
+    const int mL = i > 0 ? 1 : 0, mH = i < nx - 1 ? 1 : 0;
+    const bool hasLo = i > 0 && !g.blocked[c - mL], hasHi = i < nx - 1 && !g.blocked[c + mH];
+    const T u0 = g.u[fx0 - mL], u1 = g.u[fx0], u2 = g.u[fx0 + 1], u3 = g.u[fx0 + 1 + mH];
+    const T v0 = g.v[fy0 - mL], v1 = g.v[fy0], v2 = g.v[fy0 + mH];
+    const T V0 = g.v[fy0 + nx - mL], V1 = g.v[fy0 + nx], V2 = g.v[fy0 + nx + mH];
+    const R* w = g.w;
+    const R* W = g.w + nx * ny;
+    const T w0 = w[c - mL], w1 = w[c], w2 = w[c + mH], W0 = W[c - mL], W1 = W[c], W2 = W[c + mH];
+    const T lo[3] = {T(0.5) * (u0 + u1), T(0.5) * (v0 + V0), T(0.5) * (w0 + W0)};
+    const T self[3] = {T(0.5) * (u1 + u2), T(0.5) * (v1 + V1), T(0.5) * (w1 + W1)};
+    const T hi[3] = {T(0.5) * (u2 + u3), T(0.5) * (v2 + V2), T(0.5) * (w2 + W2)};
+#pragma unroll
+    for (int q = 0; q < 3; ++q) {
+        g.tmp[q][c] = self[q];
+        g.tmp[3 + q][c] = turbFilter<T>(hasLo ? lo[q] : self[q], self[q], hasHi ? hi[q] : self[q]);
+    }
 }
 
-// one pass of the test filter along AXIS for the three velocity components
-// (the reference filters each component x -> y -> z; the components are
-// independent, so one launch per axis covers all three)
-template <class R, int AXIS>
-__global__ void k_turb_filter(const Scn<R>* __restrict__ S, Dom dom) {
+template <class R>
+__global__ void k_turb_y(const Scn<R>* __restrict__ S, Dom dom) {
     using T = R;
     PHX_PROLOGUE(dom);
     int c = tile_ * TPB + threadIdx.x;
     if (c >= g.N) return;
     if (g.blocked[c]) {
 #pragma unroll
-        for (int q = 0; q < 3; ++q) (AXIS == 1 ? g.tmp[6 + q] : g.tmp[3 + q])[c] = 0;
+        for (int q = 0; q < 3; ++q) g.tmp[6 + q][c] = 0;
         return;
     }
-    const int nx = g.nx, ny = g.ny, nz = g.nz;
     int i, j, k;
     ijkOf(g, 0, c, i, j, k);
-    const int id = AXIS == 0 ? i : AXIS == 1 ? j : k, n = AXIS == 0 ? nx : AXIS == 1 ? ny : nz;
-    const int st = AXIS == 0 ? 1 : AXIS == 1 ? nx : nx * ny;
-    // neighbours at clamped indices, loaded together with their solid flags and
-    // used through selects
-    const int cLo = id > 0 ? c - st : c, cHi = id < n - 1 ? c + st : c;
-    const bool hasLo = id > 0 && !g.blocked[cLo], hasHi = id < n - 1 && !g.blocked[cHi];
-    T self[3], lov[3], hiv[3];
+    const int cLo = j > 0 ? c - g.nx : c, cHi = j < g.ny - 1 ? c + g.nx : c;
+    const bool hasLo = j > 0 && !g.blocked[cLo], hasHi = j < g.ny - 1 && !g.blocked[cHi];
 #pragma unroll
     for (int q = 0; q < 3; ++q) {
-        const R* in = AXIS == 0 ? g.tmp[q] : AXIS == 1 ? g.tmp[3 + q] : g.tmp[6 + q];
-        self[q] = in[c];
-        lov[q] = in[cLo];
-        hiv[q] = in[cHi];
-    }
-#pragma unroll
-    for (int q = 0; q < 3; ++q) {
-        R* out = AXIS == 1 ? g.tmp[6 + q] : g.tmp[3 + q];
-        const T lo = hasLo ? lov[q] : self[q];
-        const T hi = hasHi ? hiv[q] : self[q];
-        out[c] = T(0.25) * lo + T(0.5) * self[q] + T(0.25) * hi;
+        const R* in = g.tmp[3 + q];
+        const T self = in[c], lo = in[cLo], hi = in[cHi];
+        g.tmp[6 + q][c] = turbFilter<T>(hasLo ? lo : self, self, hasHi ? hi : self);
     }
 }
 
@@ -348,9 +374,17 @@ __global__ void k_turb_nu(const Scn<R>* __restrict__ S, Dom dom) {
     if (c < g.N) {
         if (g.blocked[c]) g.nu[c] = 0;
         else {
-            T du = g.tmp[0][c] - g.tmp[3][c];
-            T dv = g.tmp[1][c] - g.tmp[4][c];
-            T dw = g.tmp[2][c] - g.tmp[5][c];
+            const int sxy = g.nx * g.ny, kz = (int)divU((unsigned)c, g.dvB[0]);
+            const int cLo = kz > 0 ? c - sxy : c, cHi = kz < g.nz - 1 ? c + sxy : c;
+            const bool hasLo = kz > 0 && !g.blocked[cLo], hasHi = kz < g.nz - 1 && !g.blocked[cHi];
+            T dif[3];
+#pragma unroll
+            for (int q = 0; q < 3; ++q) {
+                const R* in = g.tmp[6 + q];
+                const T self = in[c], lo = in[cLo], hi = in[cHi];
+                dif[q] = g.tmp[q][c] - turbFilter<T>(hasLo ? lo : self, self, hasHi ? hi : self);
+            }
+            const T du = dif[0], dv = dif[1], dw = dif[2];
             T ks = T(0.5) * (du * du + dv * dv + dw * dw);
             const T Tc = tAbs(g.sc[0][c]);
             T nu;
@@ -426,6 +460,18 @@ __global__ void k_heat(const Scn<R>* __restrict__ S, Dom dom) {
     g.Q[c] = g.Q[c] + q * (T)g.sv[SV_DT];
 }
 
+template <class R>
+__device__ __forceinline__ void swapVelocities(Scn<R>& g) {
+    R* t;
+    t = g.u; g.u = g.u2; g.u2 = t;
+    t = g.v; g.v = g.v2; g.v2 = t;
+    t = g.w; g.w = g.w2; g.w2 = t;
+}
+template <class R>
+__device__ __forceinline__ void swapScalars(Scn<R>& g) {
+    for (int q = 0; q < NSC; ++q) { R* t = g.sc[q]; g.sc[q] = g.sc2[q]; g.sc2[q] = t; }
+}
+
 // FP64 path: density of every gas cell, before a stage that runs on its own
 template <class R>
 __global__ void k_rho(const Scn<R>* __restrict__ S, Dom dom) {
@@ -434,11 +480,14 @@ __global__ void k_rho(const Scn<R>* __restrict__ S, Dom dom) {
     if (c < g.N && !g.blocked[c]) g.rho[c] = rhoOf(g, c);
 }
 
-// Solver::energyAndExpansion (src/sim/gasphase.cpp:251-271)
+// Solver::energyAndExpansion (src/sim/gasphase.cpp:251-271). swap (full step): the
+// velocities' buffers are exchanged here, ahead of momentum, which reads the
+// second and writes the first.
 template <class R>
-__global__ void k_energy(const Scn<R>* __restrict__ S, Dom dom) {
+__global__ void k_energy(const Scn<R>* __restrict__ S, Dom dom, Scn<R>* swap) {
     using T = R;
     PHX_PROLOGUE(dom);
+    if (swap && tile_ == 0 && threadIdx.x == 0) swapVelocities(swap[s_]);
     int c = tile_ * TPB + threadIdx.x;
     T md = 0;
     if (c < g.N) {
@@ -466,25 +515,36 @@ __global__ void k_energy(const Scn<R>* __restrict__ S, Dom dom) {
 }
 
 // ---------------------------------------------------------------------------
-// Solver::momentum (src/sim/gasphase.cpp:275-372): one component on its faces,
-// written to the second velocity buffer.
+// Solver::momentum (src/sim/gasphase.cpp:275-372). The velocities' buffers have
+// been exchanged: a face's old value is in the second buffer, its new one goes
+// into the first.
 template <class T>
 __device__ __forceinline__ T vanLeer(T a, T b) { return a * b > T(0) ? T(2) * a * b / (a + b) : T(0); }
 
+// the axis and the tile within it of a tile of a domain over all faces
+template <class R>
+__device__ __forceinline__ int faceAxis(const Scn<R>& g, int& tile) {
+    const int tx = (g.NX + TPB - 1) / TPB, ty = (g.NY + TPB - 1) / TPB;
+    if (tile < tx) return 0;
+    tile -= tx;
+    if (tile < ty) return 1;
+    tile -= ty;
+    return 2;
+}
+
+// the component on one of its faces
 template <class R, int COMP>
-__global__ void k_momentum(const Scn<R>* __restrict__ S, Dom dom) {
+__device__ __forceinline__ void momentumFace(const Scn<R>& g, int f) {
     using T = R;
     constexpr int comp = COMP;   // the face component: compile-time, so the per-axis arrays stay in registers
-    PHX_PROLOGUE(dom);
     const int nx = g.nx, ny = g.ny, nz = g.nz;
     const int dX = nx + (comp == 0), dY = ny + (comp == 1), dZ = nz + (comp == 2);
     const int nf = dX * dY * dZ;
-    int f = tile_ * TPB + threadIdx.x;
     if (f >= nf) return;
-    const R* vel = comp == 0 ? g.u : comp == 1 ? g.v : g.w;
+    const R* vel = comp == 0 ? g.u2 : comp == 1 ? g.v2 : g.w2;
     const R* fo = comp == 0 ? g.fx : comp == 1 ? g.fy : g.fz;
     const uint8_t* lk = comp == 0 ? g.lx : comp == 1 ? g.ly : g.lz;   // null: no crack faces
-    R* out = comp == 0 ? g.u2 : comp == 1 ? g.v2 : g.w2;
+    R* out = comp == 0 ? g.u : comp == 1 ? g.v : g.w;
     if (fo[f] <= T(0)) { out[f] = 0; return; }
     if (lk && lk[f]) { out[f] = vel[f]; return; }   // set by leakage()
     int i, j, k;
@@ -496,8 +556,7 @@ __global__ void k_momentum(const Scn<R>* __restrict__ S, Dom dom) {
     const int lo = id[comp] - 1;
     const bool bnd = lo < 0 || id[comp] >= ncell[comp];
     if (bnd) {
-        const double zc = g.oz + (comp == 2 ? (double)k : k + 0.5) * g.dx;
-        double wv = windAt(g, comp, lo < 0 ? 0 : 1, zc);
+        const double wv = windAt(g, comp, lo < 0 ? 0 : 1, k);
         out[f] = isnan(wv) ? vel[f] : (R)wv;
         return;
     }
@@ -510,7 +569,7 @@ __global__ void k_momentum(const Scn<R>* __restrict__ S, Dom dom) {
     adv[comp] = v0;
     for (int a = 0; a < 3; ++a) {
         if (a == comp) continue;
-        const R* va = a == 0 ? g.u : a == 1 ? g.v : g.w;
+        const R* va = a == 0 ? g.u2 : a == 1 ? g.v2 : g.w2;
         const int aX = nx + (a == 0), aY = ny + (a == 1);
         T s = 0;
         for (int q = 0; q < 4; ++q) {
@@ -550,6 +609,25 @@ __global__ void k_momentum(const Scn<R>* __restrict__ S, Dom dom) {
         // the upwind-biased face values, the limiter arguments chosen by the
         // sign of the advecting velocity (two van Leer evaluations, no branch)
         const bool pos = adv[a] >= T(0);
+        if constexpr (sizeof(T) == 8) {
+            // half the limited differences, ab / (a + b), from one division for both:
+            // a division costs eight FP64 instructions. A product of differences below
+            // 1e-200 counts as no gradient, so the divisors' product cannot vanish.
+            const double dm = v0 - m1, dp = p1 - v0, db = pos ? m1 - m2 : p2 - p1;
+            const double a2 = pos ? db : dp, b2 = pos ? dm : db;
+            const double nA = dm * dp, nB = a2 * b2;
+            auto graded = [](double v) {   // above 1e-200, not a NaN: by the number's upper half
+                return (unsigned)(__double2hiint(v) - 0x16687e93) < 0x7ff00000u - 0x16687e93u;
+            };
+            const bool hA = graded(nA), hB = graded(nB);
+            const double sA = hA ? dm + dp : 1.0, sB = hB ? a2 + b2 : 1.0;
+            const double rinv = 1.0 / (sA * sB);
+            const double lA = hA ? nA * (sB * rinv) : 0.0, lB = hB ? nB * (sA * rinv) : 0.0;
+            const double fp = pos ? v0 + lA : p1 - lB, fm = pos ? m1 + lB : v0 - lA;
+            acc = fma(-adv[a], fp - fm, acc);
+            lap += dp - dm;
+            continue;
+        }
         const T vlA = vanLeer(v0 - m1, p1 - v0);
         const T vlB = vanLeer(pos ? m1 - m2 : p1 - v0, pos ? v0 - m1 : p2 - p1);
         const T fp = pos ? v0 + T(0.5) * vlA : p1 - T(0.5) * vlB;
@@ -557,12 +635,24 @@ __global__ void k_momentum(const Scn<R>* __restrict__ S, Dom dom) {
         acc -= adv[a] * (fp - fm) * idx;
         lap += (m1 - T(2) * v0 + p1) * idx2;
     }
+    if constexpr (sizeof(T) == 8) {
+        const double ra = g.rho[ca], rb = g.rho[cb], rs = ra + rb;   // face density: rs / 2
+        acc = fma(0.5 * (g.nu[ca] + g.nu[cb]) * idx2, lap, acc * idx);
+        if (comp == 2) {
+            const double r0 = (g.Pb[ca] + g.Pb[cb]) * (0.5 / (K_RS * K_T0));
+            acc = fma(K_G, (2.0 * r0 - rs) / rs, acc);
+        }
+        // p rho_f (1 / rb - 1 / ra) / dx
+        acc = fma(0.25 * rs * (g.p[ca] + g.p[cb]) * idx, (ra - rb) / (ra * rb), acc);
+        out[f] = clampd(fma(g.sv[SV_DT], acc, v0), -K_VMAX, K_VMAX);
+        return;
+    }
     T ra = rhoOf(g, ca), rb = rhoOf(g, cb);
     T rf = T(0.5) * (ra + rb);
     T nuf = T(0.5) * (g.nu[ca] + g.nu[cb]);
     acc += nuf * lap;
     T pt;
-    if constexpr (tempIsOffset<T>()) {
+    {
         // The same terms from the temperature offsets th = T - T0, free of the
         // cancellation of two near-equal FP32 densities:
         //   r0 - rf = 0.5 (Pa / (R T0) - ra + Pb / (R T0) - rb) = 0.5 (ra th_a + rb th_b) / T0
@@ -572,23 +662,31 @@ __global__ void k_momentum(const Scn<R>* __restrict__ S, Dom dom) {
         pt = rf * T(0.5) * (g.p[ca] + g.p[cb]);
         const T ipa = T(1) / g.Pb[ca], ipb = T(1) / g.Pb[cb];
         acc += pt * (T(K_RS) * (T(K_T0) * (ipb - ipa) + (thb * ipb - tha * ipa))) * idx;
-    } else {
-        if (comp == 2) {
-            T r0 = T(0.5) * (g.Pb[ca] + g.Pb[cb]) / (T(K_RS) * T(K_T0));
-            acc += T(K_G) * (r0 - rf) / rf;
-        }
-        pt = rf * T(0.5) * (g.p[ca] + g.p[cb]);
-        acc += pt * (T(1) / rb - T(1) / ra) * idx;
     }
     out[f] = clampd(v0 + (T)g.sv[SV_DT] * acc, -T(K_VMAX), T(K_VMAX));
 }
 
-// open boundary faces without wind inflow take the new value of the face one
-// cell inside (src/sim/gasphase.cpp:374-393). One thread per boundary face.
+// all components: a CTA's tile lies on the faces of one axis
 template <class R>
-__global__ void k_mom_bnd(const Scn<R>* __restrict__ S, Dom dom, int comp) {
+__global__ void k_momentum(const Scn<R>* __restrict__ S, Dom dom) {
+    PHX_PROLOGUE(dom);
+    const int comp = faceAxis(g, tile_);
+    const int f = tile_ * TPB + threadIdx.x;
+    if (comp == 0) momentumFace<R, 0>(g, f);
+    else if (comp == 1) momentumFace<R, 1>(g, f);
+    else momentumFace<R, 2>(g, f);
+}
+
+// open boundary faces without wind inflow take the new value of the face one
+// cell inside (src/sim/gasphase.cpp:374-393). One thread per boundary face of
+// the x sides, then the y sides, then the top.
+template <class R>
+__global__ void k_mom_bnd(const Scn<R>* __restrict__ S, Dom dom) {
     PHX_PROLOGUE(dom);
     const int nx = g.nx, ny = g.ny, nz = g.nz;
+    const int tx = (2 * ny * nz + TPB - 1) / TPB, ty = (2 * nx * nz + TPB - 1) / TPB;
+    const int comp = tile_ < tx ? 0 : tile_ < tx + ty ? 1 : 2;
+    tile_ -= comp == 0 ? 0 : comp == 1 ? tx : tx + ty;
     const int dX = nx + (comp == 0), dY = ny + (comp == 1), dZ = nz + (comp == 2);
     const int dim[3] = {dX, dY, dZ};
     const int st[3] = {1, dX, dX * dY};
@@ -607,10 +705,9 @@ __global__ void k_mom_bnd(const Scn<R>* __restrict__ S, Dom dom, int comp) {
     int f = id[0] + dX * (id[1] + dY * id[2]);
     const R* fo = comp == 0 ? g.fx : comp == 1 ? g.fy : g.fz;
     const uint8_t* lk = comp == 0 ? g.lx : comp == 1 ? g.ly : g.lz;
-    R* out = comp == 0 ? g.u2 : comp == 1 ? g.v2 : g.w2;
+    R* out = comp == 0 ? g.u : comp == 1 ? g.v : g.w;
     if (fo[f] <= R(0) || (lk && lk[f])) return;
-    double zc = g.oz + (comp == 2 ? (double)id[2] : id[2] + 0.5) * g.dx;
-    if (!isnan(windAt(g, comp, side, zc))) return;
+    if (!isnan(windAt(g, comp, side, id[2]))) return;
     int gg = f + (side == 0 ? 1 : -1) * st[comp];
     out[f] = fo[gg] > R(0) && !(lk && lk[gg]) ? out[gg] : (R)0;
 }
@@ -848,11 +945,13 @@ __global__ void k_zone_mean_sub(const Scn<R>* __restrict__ S, Dom dom) {
 }
 
 // velocity correction u -= dt/dx grad H on matrix faces, clamp, maxVel
-// (src/sim/gasphase.cpp:641-676). One thread per face of one axis.
+// (src/sim/gasphase.cpp:641-676). One thread per face; a CTA's tile lies on the
+// faces of one axis.
 template <class R>
-__global__ void k_velcorr(const Scn<R>* __restrict__ S, Dom dom, int comp) {
+__global__ void k_velcorr(const Scn<R>* __restrict__ S, Dom dom) {
     using T = R;
     PHX_PROLOGUE(dom);
+    const int comp = faceAxis(g, tile_);
     const int nx = g.nx, ny = g.ny, nz = g.nz;
     const int dX = nx + (comp == 0), dY = ny + (comp == 1), dZ = nz + (comp == 2);
     int f = tile_ * TPB + threadIdx.x;
@@ -884,7 +983,7 @@ __global__ void k_velcorr(const Scn<R>* __restrict__ S, Dom dom, int comp) {
         } else {
             // open boundary faces of x and y take part where the wind profile leaves them open
             const bool side = comp != 2 && (ca == 0 || ca == na);
-            if (amf > T(0) && !(side && !bndOpen(g, comp, ca == 0 ? 0 : 1, g.oz + (k + 0.5) * g.dx))) {
+            if (amf > T(0) && !(side && !bndOpen(g, comp, ca == 0 ? 0 : 1, k))) {
                 const T hi = ca < na ? pHi : (un < T(0) ? T(-0.5) * un * un : T(0));
                 const T lo = ca > 0 ? pLo : (un > T(0) ? T(-0.5) * un * un : T(0));
                 un = clampd(un - s * (hi - lo), -T(K_VMAX), T(K_VMAX));
@@ -1167,10 +1266,13 @@ __global__ void __launch_bounds__(ADV_TPB<R>, sizeof(R) == 4 ? 3 : 6) k_advect(c
 // ---------------------------------------------------------------------------
 // End of step (src/sim/solver.cpp:258-268): closed-zone background pressure,
 // Pb of closed-zone cells, gatherStats (:884-915), time += dt.
+// swap (full step): the scalars' buffers, which the transport has written, are
+// exchanged here.
 template <class R>
-__global__ void k_zone_pressure(const Scn<R>* __restrict__ S, Dom dom) {
+__global__ void k_zone_pressure(const Scn<R>* __restrict__ S, Dom dom, Scn<R>* swap) {
     PHX_PROLOGUE(dom);
     if (threadIdx.x != 0) return;
+    if (swap) swapScalars(swap[s_]);
     const double dt = g.sv[SV_DT];
     for (int zi = 0; zi < g.nClosed; ++zi) {
         int z = g.closedZone[zi];
@@ -1256,14 +1358,8 @@ __global__ void k_swap(Scn<R>* S, Dom dom, int what) {
     if (threadIdx.x != 0) return;
     Scn<R>& g = S[s_];
     if (what & 1) { uint8_t* t = g.lit; g.lit = g.lit2; g.lit2 = t; }
-    if (what & 2) {
-        R* t;
-        t = g.u; g.u = g.u2; g.u2 = t;
-        t = g.v; g.v = g.v2; g.v2 = t;
-        t = g.w; g.w = g.w2; g.w2 = t;
-    }
-    if (what & 4)
-        for (int q = 0; q < NSC; ++q) { R* t = g.sc[q]; g.sc[q] = g.sc2[q]; g.sc2[q] = t; }
+    if (what & 2) swapVelocities(g);
+    if (what & 4) swapScalars(g);
 }
 
 #undef PHX_PROLOGUE
