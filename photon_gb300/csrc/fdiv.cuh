@@ -14,8 +14,8 @@
 // RN(x y): for d = 1, 2, 4 it is exact; for d = 3, 5, 6, 7, RN(1/d) is within
 // 2^-54 relative of 1/d, so |q - x/d| < 0.5 ulp + 2^53 * 2^-54 ulp = 1 ulp.
 // The theorem assumes no underflow or overflow: zeros (whose sign the FMAs
-// would not keep), values below 2^-960, infinities and NaNs take the plain
-// division. A GPU test compares the two forms bit for bit over random and
+// would not keep) are returned; values below 2^-960, infinities and NaNs take the
+// plain division. A GPU test compares the two forms bit for bit over random and
 // constructed inputs for every d.
 #pragma once
 
@@ -34,7 +34,8 @@ __device__ __forceinline__ double recipSmall(int d) {
 // x / d for d = 1..7, bit-identical to the IEEE quotient
 __device__ __forceinline__ double divSmall(double x, int d) {
     const unsigned ex = ((unsigned)__double2hiint(x) >> 20) & 0x7ffu;
-    if (ex < 63u || ex == 0x7ffu) return x / (double)d;
+    if (ex < 63u || ex == 0x7ffu)   // a zero is its own quotient
+        return (__double_as_longlong(x) << 1) == 0 ? x : x / (double)d;
     const double y = recipSmall(d);
     const double q = x * y;
     const double e = fma(-q, (double)d, x);

@@ -48,65 +48,53 @@ __device__ __forceinline__ T l0Div(T a, unsigned cd, T dg) {
     return gsDiv(a, dg);
 }
 
-// the general-cell form of the stencil: coefficients and diagonal from the arrays
-template <class R>
-struct L0Coef {
-    R dg, xm, xp, ym, yp, zm, zp;
-};
-template <class R>
-__device__ __forceinline__ L0Coef<R> l0General(const Scn<R>& g, int i, int j, int k) {
-    const int nx = g.nx, ny = g.ny;
-    const long long c = (long long)k * nx * ny + (long long)j * nx + i;
-    const long long fx = i + (long long)(nx + 1) * (j + (long long)ny * k);
-    const long long fy = i + (long long)nx * (j + (long long)(ny + 1) * k);
-    L0Coef<R> o;
-    o.dg = g.diag[c];
-    o.xm = g.a0x[fx];
-    o.xp = g.a0x[fx + 1];
-    o.ym = g.a0y[fy];
-    o.yp = g.a0y[fy + nx];
-    o.zm = g.a0z[c];
-    o.zp = g.a0z[c + (long long)nx * ny];
-    return o;
-}
-
 // neighbour values of one cell in the reference's term order
 template <class R>
 struct L0Nb {
     R xm, xp, ym, yp, zm, zp;
 };
 
-// sacc plus (SIGN > 0) or minus (SIGN < 0) the neighbour terms in the order
-// x-, x+, y-, y+, z-, z+: for a coded cell every set bit adds its neighbour
-// (coefficient 1); a general cell multiplies by the arrays' coefficients its
-// interior neighbours
+// the general-cell form of the stencil: the interior neighbours times the arrays'
+// coefficients. Out of line: few cells take it, and its code would stand in the
+// instruction stream of every pass.
 template <int SIGN, class R>
-__device__ __forceinline__ R l0Sum(R sacc, unsigned cd, const L0Coef<R>& a, const L0Nb<R>& n, int i, int j, int k,
-                                   int nx, int ny, int nz) {
-    if (!(cd & CODE_GENERAL)) {
-        if (cd & 1u) sacc = SIGN > 0 ? sacc + n.xm : sacc - n.xm;
-        if (cd & 2u) sacc = SIGN > 0 ? sacc + n.xp : sacc - n.xp;
-        if (cd & 4u) sacc = SIGN > 0 ? sacc + n.ym : sacc - n.ym;
-        if (cd & 8u) sacc = SIGN > 0 ? sacc + n.yp : sacc - n.yp;
-        if (cd & 16u) sacc = SIGN > 0 ? sacc + n.zm : sacc - n.zm;
-        if (cd & 32u) sacc = SIGN > 0 ? sacc + n.zp : sacc - n.zp;
-        return sacc;
-    }
+__device__ __noinline__ R l0SumGeneral(const Scn<R>& g, R sacc, L0Nb<R> n, int i, int j, int k) {
+    const int nx = g.nx, ny = g.ny, nz = g.nz;
+    const long long c = (long long)k * nx * ny + (long long)j * nx + i;
+    const long long fx = i + (long long)(nx + 1) * (j + (long long)ny * k);
+    const long long fy = i + (long long)nx * (j + (long long)(ny + 1) * k);
+    const R xm = g.a0x[fx], xp = g.a0x[fx + 1], ym = g.a0y[fy], yp = g.a0y[fy + nx], zm = g.a0z[c],
+            zp = g.a0z[c + (long long)nx * ny];
     if (SIGN > 0) {
-        if (i > 0) sacc += a.xm * n.xm;
-        if (i < nx - 1) sacc += a.xp * n.xp;
-        if (j > 0) sacc += a.ym * n.ym;
-        if (j < ny - 1) sacc += a.yp * n.yp;
-        if (k > 0) sacc += a.zm * n.zm;
-        if (k < nz - 1) sacc += a.zp * n.zp;
+        if (i > 0) sacc += xm * n.xm;
+        if (i < nx - 1) sacc += xp * n.xp;
+        if (j > 0) sacc += ym * n.ym;
+        if (j < ny - 1) sacc += yp * n.yp;
+        if (k > 0) sacc += zm * n.zm;
+        if (k < nz - 1) sacc += zp * n.zp;
     } else {
-        if (i > 0) sacc -= a.xm * n.xm;
-        if (i < nx - 1) sacc -= a.xp * n.xp;
-        if (j > 0) sacc -= a.ym * n.ym;
-        if (j < ny - 1) sacc -= a.yp * n.yp;
-        if (k > 0) sacc -= a.zm * n.zm;
-        if (k < nz - 1) sacc -= a.zp * n.zp;
+        if (i > 0) sacc -= xm * n.xm;
+        if (i < nx - 1) sacc -= xp * n.xp;
+        if (j > 0) sacc -= ym * n.ym;
+        if (j < ny - 1) sacc -= yp * n.yp;
+        if (k > 0) sacc -= zm * n.zm;
+        if (k < nz - 1) sacc -= zp * n.zp;
     }
+    return sacc;
+}
+
+// sacc plus (SIGN > 0) or minus the neighbour terms of cell (i, j, k) in the order
+// x-, x+, y-, y+, z-, z+: for a coded cell every set bit adds its neighbour
+// (coefficient 1)
+template <int SIGN, class R>
+__device__ __forceinline__ R l0Sum(const Scn<R>& g, R sacc, unsigned cd, const L0Nb<R>& n, int i, int j, int k) {
+    if (cd & CODE_GENERAL) return l0SumGeneral<SIGN>(g, sacc, n, i, j, k);
+    if (cd & 1u) sacc = SIGN > 0 ? sacc + n.xm : sacc - n.xm;
+    if (cd & 2u) sacc = SIGN > 0 ? sacc + n.xp : sacc - n.xp;
+    if (cd & 4u) sacc = SIGN > 0 ? sacc + n.ym : sacc - n.ym;
+    if (cd & 8u) sacc = SIGN > 0 ? sacc + n.yp : sacc - n.yp;
+    if (cd & 16u) sacc = SIGN > 0 ? sacc + n.zm : sacc - n.zm;
+    if (cd & 32u) sacc = SIGN > 0 ? sacc + n.zp : sacc - n.zp;
     return sacc;
 }
 

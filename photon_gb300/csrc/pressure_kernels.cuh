@@ -170,70 +170,33 @@ __device__ __forceinline__ void coarseSerialTile(const Scn<R>& g) {
 // The CG scalars of a scenario while it is being solved, one copy per CTA of its team.
 struct CgState {
     double rz, alpha, beta, dq;
-    double rmax, r64max;     // max|r| of the recursion, of the FP64 residual (mixed path)
-    double pres, prel;       // reported residuals: in 1/s, relative to max|b|
-    double tol, tolHalf, relTol, inv, bmax, relStop, relStop2;
-    int haveB, haveRel;      // max|b| > 0, relTol > 0
+    double rmax, r64;        // last max|r| of the recursion; of the FP64 residual where it was formed (mixed path)
+    // bars on max|r|: the absolute one and half of it; the relative one and twice it (-1: none)
+    double absStop, absHalf, relStop, relStop2;
     int it, done, repl;      // repl: the residual is replaced this iteration (mixed path)
     int brk;                 // mixed path: 1 after a breakdown (next update skipped), 2 restart pending
 };
 
-// What closing a CG iteration needs of its FP64 numbers: the quotients and the
-// comparisons, one per lane of a warp (one thread's chain of FP64 divisions and
-// tests took 1.6 to 2.8 us per iteration).
-struct CgTests {
-    double beta, rInv, rRel, r64Inv, r64Rel;
-    unsigned gt;             // CG_* bits
-};
-enum : unsigned {
-    CG_RZ_POS = 1u,          // r.z > 0
-    CG_R_TOL = 2u,           // max|r| above the absolute bar
-    CG_R_REL = 4u,           // max|r| above the relative bar
-    CG_R64_TOL = 8u,         // the FP64 residual above the absolute bar
-    CG_R64_REL = 16u,        // ... above the relative bar
-    CG_R64_POS = 32u,        // ... above 0
-    CG_DRIFT = 64u,          // ... above four times the recursion's
-    CG_R_REL2 = 128u,        // max|r| above twice the relative bar
-    CG_R_TOL2 = 256u         // max|r| above half the absolute bar
-};
-__device__ __forceinline__ CgTests cgTests(const CgState& c, double tot, double rmax, double r64) {
-    const int lane = threadIdx.x & 31;
-    const bool have64 = __double_as_longlong(r64) > 0;   // r64 >= 0: positive as a number
-    // lanes without a quotient of their own divide 1 by 1: a zero numerator would send
-    // the whole warp through the division's slow path
-    const bool used = lane < 3 || (lane < 5 && have64);
-    const double num = lane == 0 ? tot : lane < 3 ? rmax : used ? r64 : 1.0;
-    const double den = lane == 0 ? c.rz : !used ? 1.0 : (lane & 1) ? c.inv : c.bmax;
-    const double v = num / den;
-    CgTests t;
-    t.beta = __shfl_sync(0xffffffffu, v, 0);
-    t.rInv = __shfl_sync(0xffffffffu, v, 1);
-    t.rRel = __shfl_sync(0xffffffffu, v, 2);
-    t.r64Inv = have64 ? __shfl_sync(0xffffffffu, v, 3) : 0.0;
-    t.r64Rel = have64 ? __shfl_sync(0xffffffffu, v, 4) : 0.0;
-    const double a = lane == 0 ? tot : lane == 1 || lane == 8 ? t.rInv : lane == 2 || lane == 7 ? rmax
-                   : lane == 3 ? t.r64Inv : lane == 4 ? t.r64Rel : r64;
-    const double b = lane == 0 || lane == 5 ? 0.0 : lane == 1 || lane == 3 ? c.tol : lane == 2 ? c.relStop
-                   : lane == 4 ? c.relTol : lane == 7 ? c.relStop2 : c.tolHalf;
-    t.gt = __ballot_sync(0xffffffffu, a > (lane == 6 ? rmax * 4.0 : b));
-    return t;
-}
+// a > b for numbers of which b is not a NaN and a is not negative, by their bits:
+// an FP64 comparison takes some hundred cycles here, and closing an iteration is a
+// chain of them on one thread
+__device__ __forceinline__ bool above(double a, double b) { return __double_as_longlong(a) > __double_as_longlong(b); }
 
-// closes a CG iteration once r.z = tot is known: beta, the iteration count and
-// the stop test (src/sim/gasphase.cpp:589-605; the optional relative test is
-// max|r| <= relTol max|b|). phase 0: the first preconditioning before the loop;
-// 1: inside the loop. One thread.
+// closes a CG iteration once r.z = tot is known: the iteration count and the stop
+// test (src/sim/gasphase.cpp:589-605; the optional relative test is max|r| <=
+// relTol max|b|). beta is tot / rz. phase 0: the first preconditioning before the
+// loop; 1: inside the loop. One thread.
 template <class R>
-__device__ __forceinline__ void closeCgIteration(const Scn<R>& g, CgState& c, int phase, double tot, const CgTests& t) {
+__device__ __forceinline__ void closeCgIteration(const Scn<R>& g, CgState& c, int phase, double tot, double beta,
+                                                 double rmax, double r64) {
     const int it = phase == 0 ? 0 : c.it + 1;
-    const bool positive = (t.gt & CG_RZ_POS) != 0;
+    const bool positive = tot > 0;
     c.it = it;
+    c.rmax = rmax;
     if (!g.mixed) {
-        if (phase != 0) c.beta = t.beta;
+        if (phase != 0) c.beta = beta;
         c.rz = tot;
-        c.pres = t.rInv;
-        c.prel = c.haveB ? t.rRel : 0.0;
-        if (!((t.gt & CG_R_TOL) && it < g.maxIters && positive && (t.gt & CG_R_REL))) c.done = 1;
+        if (!(above(rmax, c.absStop) && it < g.maxIters && positive && above(rmax, c.relStop))) c.done = 1;
         return;
     }
     // mixed: the stop test uses the FP64 residual, known where it was just
@@ -242,16 +205,15 @@ __device__ __forceinline__ void closeCgIteration(const Scn<R>& g, CgState& c, in
     const bool replaced = phase == 0 || c.repl != 0;
     bool converged = false, restart = false;
     if (replaced) {
-        c.pres = t.r64Inv;
-        c.prel = c.haveB ? t.r64Rel : 0.0;
-        converged = !(t.gt & CG_R64_TOL) || (c.haveRel && (!c.haveB || !(t.gt & CG_R64_REL))) || !(t.gt & CG_R64_POS);
+        c.r64 = r64;
+        converged = !above(r64, c.absStop) || !above(r64, c.relStop) || !above(r64, 0.0);
         // restart the FP32 CG from the replaced residual (d = z) where it is no
         // longer conjugate to the search direction: closed zones (their
         // operators are singular), and any scenario whose FP32 recursion had
         // drifted below the true residual (a strong preconditioner takes the
         // recursion to FP32's rounding floor within a few iterations; the old
         // direction then carries only rounding noise)
-        restart = phase != 0 && (g.nClosed > 0 || (t.gt & CG_DRIFT));
+        restart = phase != 0 && (g.nClosed > 0 || above(r64, 4.0 * rmax));
     }
     // the first iteration after a breakdown's replacement restarts the FP32 CG (d = z)
     if (phase != 0 && c.brk == 2) {
@@ -264,9 +226,9 @@ __device__ __forceinline__ void closeCgIteration(const Scn<R>& g, CgState& c, in
     const bool recover = !positive && !replaced && phase != 0 && !converged && it < g.maxIters;
     if (recover) c.brk = 1;
     c.rz = recover ? 1.0 : tot;   // any positive value: the skipped update does not use it
-    if (phase != 0) c.beta = restart || recover ? 0.0 : t.beta;
+    if (phase != 0) c.beta = restart || recover ? 0.0 : beta;
     const bool stop = converged || it >= g.maxIters || (!positive && !recover);
-    const bool claims = phase != 0 && ((c.haveRel && !(t.gt & CG_R_REL2)) || !(t.gt & CG_R_TOL2));
+    const bool claims = phase != 0 && (!above(rmax, c.relStop2) || !above(rmax, c.absHalf));
     c.repl = !stop && phase != 0 && ((it % g.replaceEvery) == 0 || claims || recover);
     if (stop) c.done = 1;
 }

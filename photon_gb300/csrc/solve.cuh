@@ -234,14 +234,11 @@ __device__ __forceinline__ void solvePair(const Scn<R>& g, const SolveBufs<R>& B
         pair(live && k < nz - 1 ? c0 + sxy : c0, zp0, zp1);
         const unsigned cd0 = cf[c0], cd1 = cf[c1];
         const L0Nb<T> n0{xm, v1, ym0, yp0, zm0, zp0}, n1{v0, xp, ym1, yp1, zm1, zp1};
-        L0Coef<T> g0{}, g1{};
-        if (live && (cd0 & CODE_GENERAL)) g0 = l0General(g, i0, j, k);
-        if (on1 && (cd1 & CODE_GENERAL)) g1 = l0General(g, i0 + 1, j, k);
-        const T dg0 = (cd0 & CODE_GENERAL) ? g0.dg : codeDiag<T>(cd0), dg1 = (cd1 & CODE_GENERAL) ? g1.dg : codeDiag<T>(cd1);
+        const T dg0 = diagOf(c0, cd0), dg1 = diagOf(c1, cd1);
         if constexpr (MODE == PASS_APPLY) {
             T w0 = T(0), w1 = T(0);
-            if (dg0 > T(0)) w0 = l0Sum<-1>(dg0 * v0, cd0, g0, n0, i0, j, k, nx, ny, nz);
-            if (on1 && dg1 > T(0)) w1 = l0Sum<-1>(dg1 * v1, cd1, g1, n1, i0 + 1, j, k, nx, ny, nz);
+            if (dg0 > T(0)) w0 = l0Sum<-1>(g, dg0 * v0, cd0, n0, i0, j, k);
+            if (on1 && dg1 > T(0)) w1 = l0Sum<-1>(g, dg1 * v1, cd1, n1, i0 + 1, j, k);
             pairStore<T, EVEN>(B.dNew, c0, on1, v0, v1);
             pairStore<T, EVEN>(B.q, c0, on1, w0, w1);
             t0 = f2prod(w0, v0);
@@ -252,8 +249,8 @@ __device__ __forceinline__ void solvePair(const Scn<R>& g, const SolveBufs<R>& B
             const int* af = g.lv[0].agg;
             const int a0 = live ? af[c0] : -1, a1 = on1 ? af[c1] : -1;
             T s0 = T(0), s1 = T(0);
-            if (a0 >= 0) s0 = l0Sum<1>(r0 - dg0 * v0, cd0, g0, n0, i0, j, k, nx, ny, nz);
-            if (a1 >= 0) s1 = l0Sum<1>(r1 - dg1 * v1, cd1, g1, n1, i0 + 1, j, k, nx, ny, nz);
+            if (a0 >= 0) s0 = l0Sum<1>(g, r0 - dg0 * v0, cd0, n0, i0, j, k);
+            if (a1 >= 0) s1 = l0Sum<1>(g, r1 - dg1 * v1, cd1, n1, i0 + 1, j, k);
             // the block's cells in ascending order over its four lanes
             T acc0 = T(0), acc1 = T(0);
 #pragma unroll
@@ -307,13 +304,11 @@ __device__ __forceinline__ void solvePair(const Scn<R>& g, const SolveBufs<R>& B
     n.yp = v[2];
     n.zm = v[3];
     n.zp = v[4];
-    auto sum = [&](auto sign, T start, L0Coef<T>& gen) -> T {
-        if (cd & CODE_GENERAL) gen = l0General(g, i0 + o, j, k);
-        return l0Sum<decltype(sign)::value>(start, cd, gen, n, i0 + o, j, k, nx, ny, nz);
+    auto sum = [&](auto sign, T start) -> T {
+        return l0Sum<decltype(sign)::value>(g, start, cd, n, i0 + o, j, k);
     };
     using Plus = std::integral_constant<int, 1>;
     using Minus = std::integral_constant<int, -1>;
-    L0Coef<T> gen{};
     if constexpr (MODE == PASS_APPLY) {
         T z0, z1, d0 = T(0), d1 = T(0), q0 = T(0), q1 = T(0);
         const T zc = z[c], rr = B.r[cr];
@@ -327,7 +322,7 @@ __device__ __forceinline__ void solvePair(const Scn<R>& g, const SolveBufs<R>& B
         T wb = T(0);
         if (cOn) {
             const T dg = diagOf(c, cd);
-            if (dg > T(0)) wb = sum(Minus{}, dg * zb, gen);
+            if (dg > T(0)) wb = sum(Minus{}, dg * zb);
         }
         const T wr = rOn ? rr : T(0);
         T w0 = ro ? wb : wr, w1 = ro ? wr : wb;
@@ -346,7 +341,7 @@ __device__ __forceinline__ void solvePair(const Scn<R>& g, const SolveBufs<R>& B
         if (cOn) {
             const T dg = diagOf(c, cd);
             T zc = T(0);
-            if (dg > T(0)) zc = l0Div(sum(Plus{}, rv, gen), cd, dg);
+            if (dg > T(0)) zc = l0Div(sum(Plus{}, rv), cd, dg);
             B.z[c] = zc;
         }
     } else if constexpr (MODE == PASS_RED) {
@@ -354,7 +349,7 @@ __device__ __forceinline__ void solvePair(const Scn<R>& g, const SolveBufs<R>& B
         if (cOn) {
             const T dg = diagOf(c, cd);
             T zc = T(0);
-            if (dg > T(0)) zc = l0Div(sum(Plus{}, rv, gen), cd, dg);
+            if (dg > T(0)) zc = l0Div(sum(Plus{}, rv), cd, dg);
             B.z[c] = zc;
             if constexpr (sizeof(R) == 4) (o ? t1 : t0) = f2prod(rv, zc);
             else dot = fma(rv, zc, dot);
@@ -367,7 +362,7 @@ __device__ __forceinline__ void solvePair(const Scn<R>& g, const SolveBufs<R>& B
         const int* af = g.lv[0].agg;
         const int a = cOn ? af[c] : -1, ab = inOn ? af[cIn] : -1;
         T res = T(0);
-        if (a >= 0) res = sum(Plus{}, T(0), gen);
+        if (a >= 0) res = sum(Plus{}, T(0));
         T acc = T(0), accB = T(0);
         const bool apart = __any_sync(0xffffffffu, ab >= 0 && ab != a);   // pieces of a block that are not joined
 #pragma unroll
@@ -433,14 +428,17 @@ __device__ __forceinline__ double warpSumAll(double v) {   // the same value in 
     for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
     return v;
 }
-// FP32: the sum of a scenario's nt tiles, four to a CTA-sized group whose sum is
-// rounded to FP64, in every lane of warp 0. The orders are those of a 128-thread
-// CTA per 128 blocks and one such CTA over their sums.
-__device__ __forceinline__ double teamTotalF2(const double* part, int nt, double* sh) {
+// FP32: the sum of a scenario's nt tiles, four to a group whose sum is rounded to
+// FP64, in every lane of warp 0. The orders are those of a 128-thread CTA per 128
+// blocks and one such CTA over their sums: thread i adds groups i, i + 128, ...
+// All threads form the groups' sums first (sh: a value per thread of the CTA), so that
+// thread i waits for one load, not for one per group.
+__device__ __forceinline__ double teamTotalF2(const double* part, int nt, double* sh, double* sh4) {
     const int tid = (int)threadIdx.x, n4 = (nt + 3) / 4;
-    if (tid < 128) {
-        double acc = 0;
-        for (int i = tid; i < n4; i += 128) {
+    double acc = 0;
+    for (int i0 = 0; i0 < n4; i0 += (int)blockDim.x) {
+        const int i = i0 + tid;
+        if (i < n4) {
             F2 w[4];
 #pragma unroll
             for (int e = 0; e < 4; ++e) {
@@ -451,13 +449,22 @@ __device__ __forceinline__ double teamTotalF2(const double* part, int nt, double
                 }
             }
             const F2 v = f2add(f2add(w[0], w[2]), f2add(w[1], w[3]));
-            acc += widen(v.hi) + widen(v.lo);
+            sh[tid] = widen(v.hi) + widen(v.lo);
         }
+        __syncthreads();
+        if (tid < 128) {
+            const int n = min(n4 - i0, (int)blockDim.x);
+#pragma unroll 1
+            for (int q = tid; q < n; q += 128) acc += sh[q];
+        }
+        if (i0 + (int)blockDim.x < n4) __syncthreads();
+    }
+    if (tid < 128) {
         acc = warpSum(acc);
-        if ((tid & 31) == 0) sh[tid >> 5] = acc;
+        if ((tid & 31) == 0) sh4[tid >> 5] = acc;
     }
     __syncthreads();
-    return (sh[0] + sh[2]) + (sh[1] + sh[3]);
+    return (sh4[0] + sh4[2]) + (sh4[1] + sh4[3]);
 }
 // The sum of a scenario's nt partials, in every lane of warp 0; the whole CTA
 // calls it and may read what other warps wrote to shared memory before the call.
@@ -735,18 +742,12 @@ k_solve(const Scn<R>* __restrict__ S, SolveArgs a) {
                 cg.rz = 1;   // not yet known: a divisor whose quotient is not used
                 cg.alpha = cg.beta = cg.dq = 0;
                 cg.rmax = sv[SV_RMAX];
-                cg.r64max = 0;
-                cg.pres = sv[SV_PRES];
-                cg.prel = sv[SV_PREL];
-                cg.tol = g.tol;
-                cg.relTol = g.relTol;
-                cg.inv = sv[SV_INV];
-                cg.bmax = sv[SV_BMAX];
-                cg.relStop = g.relTol > 0 ? g.relTol * cg.bmax : -1.0;
+                cg.r64 = 0;
+                const double inv = sv[SV_INV], bmax = sv[SV_BMAX];
+                cg.absStop = g.tol * inv;
+                cg.absHalf = 0.5 * cg.absStop;
+                cg.relStop = !(g.relTol > 0) ? -1.0 : kMixed && !(bmax > 0) ? 1e300 : g.relTol * bmax;
                 cg.relStop2 = 2.0 * cg.relStop;
-                cg.tolHalf = 0.5 * g.tol;
-                cg.haveB = cg.bmax > 0;
-                cg.haveRel = g.relTol > 0;
                 cg.it = cg.done = cg.repl = cg.brk = 0;
                 poolUsed = 0;
             }
@@ -962,7 +963,7 @@ k_solve(const Scn<R>* __restrict__ S, SolveArgs a) {
                 }
                 PHX_PASS(PASS_APPLY, partDq, none, false);
                 PHX_TEAM_SYNC();
-                const double total = kMixed ? teamTotalF2(partDq, nt, shSum) : teamTotal(partDq, nt, shSum);
+                const double total = kMixed ? teamTotalF2(partDq, nt, shDot[0], shSum) : teamTotal(partDq, nt, shSum);
                 if (tid == 0) {
                     cg.dq = total;
                     if (cg.brk == 1) {   // the iteration after a breakdown: no update, then a restart
@@ -1047,13 +1048,12 @@ k_solve(const Scn<R>* __restrict__ S, SolveArgs a) {
                 m = warpMaxPos(m);
                 if (lane == 0) shMax[which] = m;
             }
-            const double total = kMixed ? teamTotalF2(partRz, nt, shSum + 4) : teamTotal(partRz, nt, shSum);
+            const double total = kMixed ? teamTotalF2(partRz, nt, shDot[0], shSum + 4) : teamTotal(partRz, nt, shSum);
             if (warp == 0) {
                 const double rmax = phase == 1 ? shMax[0] : cg.rmax;
                 const double r64 = kMixed && (phase == 0 || cg.repl != 0) ? shMax[1] : 0.0;
-                const CgTests ts = cgTests(cg, total, rmax, r64);
                 if (lane == 0) {
-                    closeCgIteration(g, cg, phase, total, ts);
+                    closeCgIteration(g, cg, phase, total, phase == 1 ? total / cg.rz : 0.0, rmax, r64);
                     if (loop >= a.cap) cg.done = 1;
                 }
             }
@@ -1081,8 +1081,9 @@ k_solve(const Scn<R>* __restrict__ S, SolveArgs a) {
             sv[SV_RMAX] = 0;
             sv[SV_IT] = sv[SV_PITERS] = cg.it;
             sv[SV_DONE] = 1;
-            sv[SV_PRES] = cg.pres;
-            sv[SV_PREL] = cg.prel;
+            const double r = kMixed ? cg.r64 : cg.rmax;   // the residual the solve is judged by
+            sv[SV_PRES] = r / sv[SV_INV];
+            sv[SV_PREL] = sv[SV_BMAX] > 0 ? r / sv[SV_BMAX] : 0.0;
             if (kMixed) sv[SV_HAVEPREV] = 1;
         }
 #undef PHX_PASS
