@@ -38,9 +38,6 @@ namespace phx {
     } while (0)
 #define PHX_TRY(x) do { int r_ = (x); if (r_) return r_; } while (0)
 
-// dense coarse operators up to this many unknowns (n^2 reals)
-constexpr int DENSE_MAX = 4096;
-
 // D_FACES, D_BND: the tiles of the x, then the y, then the z faces (boundary sides)
 enum DomId { D_ONE = 0, D_CELLS, D_FACES, D_BND, D_CZ, D_CC, D_LEAK, D_COUNT };
 
@@ -99,6 +96,7 @@ struct Scenario {
     std::vector<Src> ignitions, burners;
     char* arena = nullptr;       // fields, geometry, solve vectors, scalars
     char* mgArena = nullptr;     // the multigrid levels (replaced when the V-cycle schedule changes)
+    static constexpr size_t TAIL_BYTES = 256;   // of the main arena: what a saved state leaves out (tagBase)
     size_t arenaBytes = 0;       // both arenas
     size_t mainBytes = 0, mgBytes = 0;
     Scn<R> h{};                  // host copy of the device descriptor
@@ -192,15 +190,15 @@ struct Scenario {
 
     // device bytes the scenario will take (both arenas' layouts without memory)
     size_t layout(char* base) {
-        if (base) return layoutMain(base) + layoutLevels(mgArena);
-        return layoutMain(nullptr) + layoutLevels(nullptr);
+        if (base) return layoutMain(base) + TAIL_BYTES + layoutLevels(mgArena);
+        return layoutMain(nullptr) + TAIL_BYTES + layoutLevels(nullptr);
     }
 
     size_t layoutMain(char* base) {
         const int N = geo.N(), NX = geo.NX(), NY = geo.NY(), NZ = geo.NZ();
         // one reduction partial per CTA of the cell domain and per tile of the solve
         const int nblk = ((geo.nx + 1) >> 1) * ((geo.ny + 1) >> 1) * ((geo.nz + 1) >> 1);
-        const int partStride = std::max((N + TPB - 1) / TPB, solveTiling<R>(nblk).nt) + 1;
+        const int partStride = std::max((N + TPB - 1) / TPB, 2 * solveTiling<R>(nblk).nt) + 2;
         size_t off = 0;
         Scn<R>& s = h;
         s.blocked = carve<uint8_t>(base, off, N);
@@ -245,7 +243,6 @@ struct Scenario {
         s.p64prev = kMixed ? carve<double>(base, off, N) : nullptr;
         Level<R>& L0 = s.lv[0];
         L0.diag = s.diag;
-        L0.x = s.z; L0.y = nullptr; L0.b = s.r;
         L0.rowStart = nullptr; L0.col = nullptr; L0.val = nullptr;
         L0.childStart = nullptr; L0.child = nullptr;
         s.sv = carve<double>(base, off, SV_COUNT);
@@ -254,7 +251,10 @@ struct Scenario {
         s.windU = carve<double>(base, off, geo.nz);
         s.cnt = carve<unsigned>(base, off, PS_COUNT + 4);
         s.teamBar = carve<unsigned>(base, off, 64);
-        return off + 256;
+        off = (off + 511) & ~(size_t)255;
+        // past the bytes a saved state covers: tags only ever move on
+        s.tagBase = base ? reinterpret_cast<unsigned*>(base + off) : nullptr;
+        return off;
     }
 
     // the coarsest solve: the reference's 20 Gauss-Seidel sweep pairs on the FP64
@@ -290,7 +290,9 @@ struct Scenario {
                 D.val = carve<R>(base, off, L.val.size() + 1);
                 D.diag = carve<R>(base, off, L.n + 1);
                 D.omd = carve<R>(base, off, L.n + 1);
-                D.x = carve<R>(base, off, L.n + 1); D.y = carve<R>(base, off, L.n + 1); D.b = carve<R>(base, off, L.n + 1);
+                D.x = carve<R>(base, off, l == 1 || l == nl - 1 ? L.n + 1 : 1);
+                for (unsigned long long** v : {&D.b, &D.yd, &D.xd, &D.yu, &D.xu})
+                    *v = carve<unsigned long long>(base, off, TAG_WORDS<R> * (size_t)(L.n + 1));
             }
             D.agg = L.agg.empty() ? nullptr : carve<int>(base, off, L.agg.size());
             D.childStart = (l == 0 || L.childStart.empty()) ? nullptr : carve<int>(base, off, L.childStart.size());
@@ -303,8 +305,8 @@ struct Scenario {
     int allocate() {
         mainBytes = layoutMain(nullptr);
         mgBytes = layoutLevels(nullptr);
-        arenaBytes = mainBytes + mgBytes;
-        cudaError_t e = cudaMalloc(&arena, mainBytes);
+        arenaBytes = mainBytes + TAIL_BYTES + mgBytes;
+        cudaError_t e = cudaMalloc(&arena, mainBytes + TAIL_BYTES);
         if (e == cudaSuccess) e = cudaMalloc(&mgArena, mgBytes);
         if (e != cudaSuccess) {
             cudaGetLastError();
@@ -338,7 +340,7 @@ struct Scenario {
             return PHX_ERR_OOM;
         }
         mgArena = fresh;
-        arenaBytes = mainBytes + mgBytes;
+        arenaBytes = mainBytes + TAIL_BYTES + mgBytes;
         layoutLevels(mgArena);
         PHX_TRY(uploadLevels(st));
         if (old) cudaFree(old);
@@ -366,12 +368,12 @@ struct Scenario {
     int upload(cudaStream_t st) {
         const int N = geo.N();
         Scn<R>& s = h;
-        PHX_CK(cudaMemsetAsync(arena, 0, mainBytes, st));
+        PHX_CK(cudaMemsetAsync(arena, 0, mainBytes + TAIL_BYTES, st));
         s.nx = geo.nx; s.ny = geo.ny; s.nz = geo.nz; s.N = N; s.NX = geo.NX(); s.NY = geo.NY(); s.NZ = geo.NZ();
         s.dvA[0] = makeDivU(geo.nx); s.dvB[0] = makeDivU(geo.nx * geo.ny); s.dY[0] = geo.ny;
         s.dvA[1] = makeDivU(geo.nx + 1); s.dvB[1] = makeDivU((geo.nx + 1) * geo.ny); s.dY[1] = geo.ny;
         s.dvA[2] = makeDivU(geo.nx); s.dvB[2] = makeDivU(geo.nx * (geo.ny + 1)); s.dY[2] = geo.ny + 1;
-        s.dvL0[0] = makeDivU((geo.nx + 1) >> 1); s.dvL0[1] = makeDivU(((geo.nx + 1) >> 1) * ((geo.ny + 1) >> 1));
+        s.dvL0[0] = makeDivS((geo.nx + 1) >> 1); s.dvL0[1] = makeDivS(((geo.nx + 1) >> 1) * ((geo.ny + 1) >> 1));
         s.dx = geo.dx; s.ox = geo.ox; s.oy = geo.oy; s.oz = geo.oz;
         {   // IEEE divisions in R: the values of the kernels' R(1) / dx
             const R dxr = (R)geo.dx;
@@ -1052,8 +1054,8 @@ public:
         int dev = 0, sms = 0, occ = 0;
         PHX_CK(cudaGetDevice(&dev));
         PHX_CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-        PHX_CK(cudaFuncSetAttribute(k_solve<R>, cudaFuncAttributeMaxDynamicSharedMemorySize, SolveCfg<R>::POOL));
-        PHX_CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_solve<R>, SolveCfg<R>::T, SolveCfg<R>::POOL));
+        PHX_CK(cudaFuncSetAttribute(k_solve<R>, cudaFuncAttributeMaxDynamicSharedMemorySize, SolveCfg<R>::SMEM));
+        PHX_CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_solve<R>, SolveCfg<R>::T, SolveCfg<R>::SMEM));
         if (occ < 1) { err = "the solve kernel does not fit an SM"; return PHX_ERR_CUDA; }
         solveGrid = std::min(sms * occ, MAX_SOLVE_CTAS);
         if (const char* c = std::getenv("PHX_PERSIST_CTAS")) solveGrid = std::max(1, std::min(solveGrid, std::atoi(c)));
@@ -1269,7 +1271,7 @@ public:
         cudaLaunchConfig_t cfg = {};
         cfg.gridDim = dim3((unsigned)solveGrid);
         cfg.blockDim = dim3(SolveCfg<R>::T);
-        cfg.dynamicSmemBytes = SolveCfg<R>::POOL;
+        cfg.dynamicSmemBytes = SolveCfg<R>::SMEM;
         cfg.stream = st;
         cudaLaunchAttribute at;
         at.id = cudaLaunchAttributeCooperative;

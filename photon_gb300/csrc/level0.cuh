@@ -58,9 +58,10 @@ struct L0Nb {
 // coefficients. Out of line: few cells take it, and its code would stand in the
 // instruction stream of every pass.
 template <int SIGN, class R>
-__device__ __noinline__ R l0SumGeneral(const Scn<R>& g, R sacc, L0Nb<R> n, int i, int j, int k) {
+__device__ __noinline__ R l0SumGeneral(const Scn<R>& g, R sacc, L0Nb<R> n, int c) {
     const int nx = g.nx, ny = g.ny, nz = g.nz;
-    const long long c = (long long)k * nx * ny + (long long)j * nx + i;
+    int i, j, k;
+    ijkOf(g, 0, c, i, j, k);
     const long long fx = i + (long long)(nx + 1) * (j + (long long)ny * k);
     const long long fy = i + (long long)nx * (j + (long long)(ny + 1) * k);
     const R xm = g.a0x[fx], xp = g.a0x[fx + 1], ym = g.a0y[fy], yp = g.a0y[fy + nx], zm = g.a0z[c],
@@ -83,12 +84,12 @@ __device__ __noinline__ R l0SumGeneral(const Scn<R>& g, R sacc, L0Nb<R> n, int i
     return sacc;
 }
 
-// sacc plus (SIGN > 0) or minus the neighbour terms of cell (i, j, k) in the order
+// sacc plus (SIGN > 0) or minus the neighbour terms of cell c in the order
 // x-, x+, y-, y+, z-, z+: for a coded cell every set bit adds its neighbour
 // (coefficient 1)
 template <int SIGN, class R>
-__device__ __forceinline__ R l0Sum(const Scn<R>& g, R sacc, unsigned cd, const L0Nb<R>& n, int i, int j, int k) {
-    if (cd & CODE_GENERAL) return l0SumGeneral<SIGN>(g, sacc, n, i, j, k);
+__device__ __forceinline__ R l0Sum(const Scn<R>& g, R sacc, unsigned cd, const L0Nb<R>& n, int c) {
+    if (cd & CODE_GENERAL) return l0SumGeneral<SIGN>(g, sacc, n, c);
     if (cd & 1u) sacc = SIGN > 0 ? sacc + n.xm : sacc - n.xm;
     if (cd & 2u) sacc = SIGN > 0 ? sacc + n.xp : sacc - n.xp;
     if (cd & 4u) sacc = SIGN > 0 ? sacc + n.ym : sacc - n.ym;

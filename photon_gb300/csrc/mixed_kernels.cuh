@@ -27,13 +27,12 @@ __global__ void k_read_times(const Scn<R>* __restrict__ S, int n, double* out) {
     if (s < n) out[s] = S[s].sv[SV_TIME];
 }
 
-// before a bare V-cycle: no arrivals at the team barrier yet (one thread per
-// scenario; a step's k_begin does it for the solve)
+// before a bare V-cycle (one thread per scenario; k_begin does it for a step's solve)
 template <class R>
 __global__ void k_reset(const Scn<R>* __restrict__ S, Dom dom) {
     int s_, tile_;
     locate(dom, blockIdx.x, s_, tile_);
-    if (threadIdx.x == 0) *S[s_].teamBar = 0;
+    if (threadIdx.x == 0) startSolve(S[s_]);
 }
 
 }  // namespace phx

@@ -117,6 +117,23 @@ __device__ __forceinline__ unsigned divU(unsigned x, const DivU& v) {
     return v.d <= 1 ? x : (unsigned)__umul64hi((unsigned long long)x, v.m);
 }
 
+// the same for x below 2^31: q = x m >> s with m = ceil(2^s / d), s = 31 + ceil(log2 d)
+// (the error x (m - 2^s / d) / 2^s stays below 1 / d), one wide multiply and a shift
+struct DivS {
+    unsigned m, s, d;
+};
+inline DivS makeDivS(unsigned d) {
+    DivS v;
+    v.d = d;
+    v.s = 31;
+    while ((1ull << (v.s - 31)) < d) ++v.s;
+    v.m = (unsigned)(((1ull << v.s) + d - 1) / d);
+    return v;
+}
+__host__ __device__ __forceinline__ unsigned divS(unsigned x, const DivS& v) {
+    return (unsigned)(((unsigned long long)x * v.m) >> v.s);
+}
+
 template <class R>
 struct Level {
     int n;                       // unknowns
@@ -126,7 +143,10 @@ struct Level {
     const R* omd;                // omega / diag (0 without a diagonal): the damped Jacobi factor
     const int* agg;              // unknown -> unknown of the next coarser level (nullptr at the coarsest)
     const int *childStart, *child;   // next coarser unknown -> its unknowns here, ascending
-    R *x, *y, *b;                // iterate, Jacobi scratch, right-hand side
+    R* x;                        // level 1: the V-cycle's correction; coarsest: scratch of its serial solve
+    // the V-cycle's values of the level, each with the cycle's tag (solve.cuh): right-hand
+    // side, first and second iterate on the way down, first and last on the way up
+    unsigned long long *b, *yd, *xd, *yu, *xu;
     const R* dense;              // coarsest only: n x n operator of the reference's coarse solve
 };
 
@@ -137,7 +157,7 @@ struct Scn {
     // row length dvA, plane size dvB, rows per plane dY
     DivU dvA[3], dvB[3];
     int dY[3];
-    DivU dvL0[2];                // 2x2x2 blocks of the pressure solve: blocks per row, per plane
+    DivS dvL0[2];                // 2x2x2 blocks of the pressure solve: blocks per row, per plane
     double dx, ox, oy, oz;
     double cfl, dtMaxP, tol, relTol;
     const double* dtMaxArg;      // this step's dtMax argument (one slot per scenario of the batch)
@@ -199,6 +219,7 @@ struct Scn {
     int partStride;
     unsigned* cnt;               // last-CTA counters, one per reduction kind
     unsigned* teamBar;           // arrivals at the solve's team barrier; zeroed by k_begin and k_reset
+    unsigned* tagBase;           // tag before the solve's first V-cycle; moved on by k_begin and k_reset
 };
 
 // CTA -> (scenario, tile) over a domain

@@ -41,13 +41,19 @@
 
 namespace phx {
 
-constexpr long long TEAM_WAIT_CYCLES = 4000000000LL;       // about two seconds
-constexpr unsigned ERR_TEAM_WAIT = 8u;                     // error-word bit
+// dense coarse operators up to this many unknowns (n^2 reals)
+constexpr int DENSE_MAX = 4096;
 
 template <class R>
 struct SolveCfg {
-    static constexpr int T = sizeof(R) == 8 ? 512 : 1024;  // threads per CTA
-    static constexpr int POOL = 98304;                     // shared memory for the coarse rows, bytes
+    // threads per CTA. FP64 takes 128 registers a thread. FP32 trades registers for warps in
+    // flight: house step 1.25 / 1.27 / 1.31 ms at 768 / 896 / 1024 threads, 24 scenarios 6.25 / 5.98 / 5.93
+    static constexpr int T = sizeof(R) == 8 ? 512 : 896;
+    static constexpr int ROWS = 98304;                     // shared memory for the coarse rows, bytes
+    // dynamic shared memory: coarse rows, then by turns the FP32 dot products' terms and
+    // the coarsest level's right-hand side
+    static constexpr int TERMS = sizeof(R) == 8 ? 0 : 4 * T * 8, DENSE_B = DENSE_MAX * (int)sizeof(R);
+    static constexpr int SMEM = ROWS + (TERMS > DENSE_B ? TERMS : DENSE_B);
 };
 
 // How a scenario's pairs are walked: a warp takes 8 consecutive 2x2x2 blocks (four
@@ -101,6 +107,7 @@ struct SolveBufs {
     R *p, *r, *z, *q, *d;    // d: the direction (FP32: the previous one, dNew the one being formed)
     R* dNew;
     R alpha, beta;
+    unsigned tag;            // of the V-cycle under way
     bool haveD;              // d and q hold the previous direction and its product
 };
 
@@ -135,15 +142,40 @@ __device__ __forceinline__ void pairStore(R* a, int c0, bool on1, R v0, R v1) {
 // coarsest, its first damped Jacobi sweep from x = 0. Every lane writes its
 // cells' aggregates; the lanes of one aggregate write the same value.
 template <class R>
-__device__ __forceinline__ void restrictTo(const Scn<R>& g, int at, R value) {
+__device__ __forceinline__ void restrictTo(const Scn<R>& g, int at, R value, unsigned tag) {
     if (at < 0) return;
     const Level<R>& L = g.lv[1];
-    L.b[at] = value;
-    if (g.nLevels > 2) L.y[at] = jacobiValue(value, R(0), L.diag[at], L.omd[at]);
+    tagStore(L.b, at, value, tag);
+    if (g.nLevels > 2) tagStore(L.yd, at, jacobiValue(value, R(0), L.diag[at], L.omd[at]), tag);
 }
 
-// One pass over the pair of thread-index q (block q / 4, row and plane of the
-// block by q % 4). All loads are issued unconditionally at clamped places and
+// A pair's place: its first cell, whether it exists (live), has a second cell (on1), has
+// its red cell second (red1), and which of its neighbours lie in the grid
+template <class R>
+struct PairPlace {           // the pair of thread-index q: block q / 4, row and plane of the block by q % 4
+    int i0, j, k, c0, nx, ny, nz;
+    bool live, on1;
+    __device__ __forceinline__ PairPlace(const Scn<R>& g, int q, int nblk) : nx(g.nx), ny(g.ny), nz(g.nz) {
+        const int blk = min(q >> 2, nblk - 1);
+        const int bz = (int)divS((unsigned)blk, g.dvL0[1]);
+        const int rem = blk - bz * (int)g.dvL0[1].d;
+        const int by = (int)divS((unsigned)rem, g.dvL0[0]);
+        i0 = 2 * (rem - by * (int)g.dvL0[0].d);
+        j = 2 * by + (q & 1);
+        k = 2 * bz + ((q >> 1) & 1);
+        live = (q >> 2) < nblk && j < ny && k < nz;
+        on1 = live && i0 + 1 < nx;
+        c0 = live ? i0 + nx * (j + ny * k) : 0;
+    }
+    __device__ __forceinline__ int red1() const { return (j ^ k) & 1; }
+    __device__ __forceinline__ bool xm() const { return live && i0 > 0; }
+    __device__ __forceinline__ bool xp() const { return live && i0 + 2 < nx; }
+    __device__ __forceinline__ bool ym() const { return live && j > 0; }
+    __device__ __forceinline__ bool yp() const { return live && j < ny - 1; }
+    __device__ __forceinline__ bool zm() const { return live && k > 0; }
+    __device__ __forceinline__ bool zp() const { return live && k < nz - 1; }
+};
+// One pass over a pair. All loads are issued unconditionally at clamped places and
 // used through the cell's code, so one memory latency covers them. Cells
 // without a diagonal hold 0 in z, d, q and r.
 //
@@ -155,23 +187,16 @@ __device__ __forceinline__ void restrictTo(const Scn<R>& g, int at, R value) {
 // dropping them moved the rounding of its recursion, and with it iteration
 // counts and the pressure's FP32 noise.
 // dot (FP64) or t0, t1 (FP32) take the pair's terms of the pass's dot product.
-template <class R, int MODE, bool EVEN>
-__device__ __forceinline__ void solvePair(const Scn<R>& g, const SolveBufs<R>& B, int q, int nblk, double& dot, F2& t0,
-                                          F2& t1, R& rmax, bool writeZ) {
+template <class R, int MODE, bool EVEN, class Place>
+__device__ __forceinline__ void solvePair(const Scn<R>& g, const SolveBufs<R>& B, const Place& at, double& dot, F2& t0, F2& t1,
+                                          R& rmax, bool writeZ) {
     using T = R;
-    const int nx = g.nx, ny = g.ny, nz = g.nz, sxy = nx * ny;
-    const int blk = min(q >> 2, nblk - 1), sub = q & 3;
-    const int bz = (int)divU((unsigned)blk, g.dvL0[1]);
-    const int rem = blk - bz * (int)g.dvL0[1].d;
-    const int by = (int)divU((unsigned)rem, g.dvL0[0]);
-    const int i0 = 2 * (rem - by * (int)g.dvL0[0].d);
-    const int dj = sub & 1, dk = sub >> 1;
-    const int j = 2 * by + dj, k = 2 * bz + dk;
-    const bool live = (q >> 2) < nblk && j < ny && k < nz;
+    const int nx = g.nx, sxy = nx * g.ny;
+    const bool live = at.live;
     if (MODE != PASS_RES && !live) return;
-    const int c0 = live ? i0 + nx * j + sxy * k : 0;
-    const bool on1 = live && (EVEN || i0 + 1 < nx);
-    const int ro = dj ^ dk;                                  // the red cell of the pair: c0 + ro
+    const int c0 = at.c0;
+    const bool on1 = EVEN ? live : at.on1;
+    const int ro = at.red1();            // the red cell of the pair: c0 + ro
     const bool rOn = ro ? on1 : live, bOn = ro ? live : on1;
     const int cr = rOn ? c0 + ro : c0, cb = bOn ? c0 + 1 - ro : c0;
     const unsigned char* cf = g.code0;
@@ -210,35 +235,35 @@ __device__ __forceinline__ void solvePair(const Scn<R>& g, const SolveBufs<R>& B
         // FP32: both cells of the pair with all their neighbours; q is A d itself and
         // the residual keeps every term (their rounding is what the FP32 recursion
         // is built on: the forms below, exact in real numbers, would let it drift)
-        auto value = [&](int at) -> T {
-            const T zv = B.z[at];
-            if (MODE == PASS_APPLY && B.haveD) return zv + B.beta * B.d[at];
+        auto value = [&](int c) -> T {
+            const T zv = B.z[c];
+            if (MODE == PASS_APPLY && B.haveD) return zv + B.beta * B.d[c];
             return zv;
         };
-        auto pair = [&](int at, T& v0, T& v1) {
-            pairLoad<T, EVEN>(B.z, at, on1, v0, v1);
+        auto pair = [&](int c, T& v0, T& v1) {
+            pairLoad<T, EVEN>(B.z, c, on1, v0, v1);
             if (MODE == PASS_APPLY && B.haveD) {
                 T e0, e1;
-                pairLoad<T, EVEN>(B.d, at, on1, e0, e1);
+                pairLoad<T, EVEN>(B.d, c, on1, e0, e1);
                 v0 = v0 + B.beta * e0;
                 v1 = v1 + B.beta * e1;
             }
         };
         T v0, v1, ym0, ym1, yp0, yp1, zm0, zm1, zp0, zp1;
         const int c1 = on1 ? c0 + 1 : c0;
-        const T xm = value(live && i0 > 0 ? c0 - 1 : c0), xp = value(live && i0 + 2 < nx ? c0 + 2 : c0);
+        const T xm = value(at.xm() ? c0 - 1 : c0), xp = value(at.xp() ? c0 + 2 : c0);
         pair(c0, v0, v1);
-        pair(live && j > 0 ? c0 - nx : c0, ym0, ym1);
-        pair(live && j < ny - 1 ? c0 + nx : c0, yp0, yp1);
-        pair(live && k > 0 ? c0 - sxy : c0, zm0, zm1);
-        pair(live && k < nz - 1 ? c0 + sxy : c0, zp0, zp1);
+        pair(at.ym() ? c0 - nx : c0, ym0, ym1);
+        pair(at.yp() ? c0 + nx : c0, yp0, yp1);
+        pair(at.zm() ? c0 - sxy : c0, zm0, zm1);
+        pair(at.zp() ? c0 + sxy : c0, zp0, zp1);
         const unsigned cd0 = cf[c0], cd1 = cf[c1];
         const L0Nb<T> n0{xm, v1, ym0, yp0, zm0, zp0}, n1{v0, xp, ym1, yp1, zm1, zp1};
         const T dg0 = diagOf(c0, cd0), dg1 = diagOf(c1, cd1);
         if constexpr (MODE == PASS_APPLY) {
             T w0 = T(0), w1 = T(0);
-            if (dg0 > T(0)) w0 = l0Sum<-1>(g, dg0 * v0, cd0, n0, i0, j, k);
-            if (on1 && dg1 > T(0)) w1 = l0Sum<-1>(g, dg1 * v1, cd1, n1, i0 + 1, j, k);
+            if (dg0 > T(0)) w0 = l0Sum<-1>(g, dg0 * v0, cd0, n0, c0);
+            if (on1 && dg1 > T(0)) w1 = l0Sum<-1>(g, dg1 * v1, cd1, n1, c1);
             pairStore<T, EVEN>(B.dNew, c0, on1, v0, v1);
             pairStore<T, EVEN>(B.q, c0, on1, w0, w1);
             t0 = f2prod(w0, v0);
@@ -249,21 +274,36 @@ __device__ __forceinline__ void solvePair(const Scn<R>& g, const SolveBufs<R>& B
             const int* af = g.lv[0].agg;
             const int a0 = live ? af[c0] : -1, a1 = on1 ? af[c1] : -1;
             T s0 = T(0), s1 = T(0);
-            if (a0 >= 0) s0 = l0Sum<1>(g, r0 - dg0 * v0, cd0, n0, i0, j, k);
-            if (a1 >= 0) s1 = l0Sum<1>(g, r1 - dg1 * v1, cd1, n1, i0 + 1, j, k);
+            if (a0 >= 0) s0 = l0Sum<1>(g, r0 - dg0 * v0, cd0, n0, c0);
+            if (a1 >= 0) s1 = l0Sum<1>(g, r1 - dg1 * v1, cd1, n1, c1);
             // the block's cells in ascending order over its four lanes
-            T acc0 = T(0), acc1 = T(0);
+            int whole = max(a0, a1);
+            whole = max(whole, __shfl_xor_sync(0xffffffffu, whole, 1));
+            whole = max(whole, __shfl_xor_sync(0xffffffffu, whole, 2));
+            if (__all_sync(0xffffffffu, (a0 < 0 || a0 == whole) && (a1 < 0 || a1 == whole))) {
+                // one aggregate per block (a cell without one adds 0): its last lane has the sum
+                T acc = s0 + s1;
 #pragma unroll
-            for (int l = 0; l < 4; ++l) {
-                const int b0 = __shfl_sync(0xffffffffu, a0, l, 4), b1 = __shfl_sync(0xffffffffu, a1, l, 4);
-                const T e0 = __shfl_sync(0xffffffffu, s0, l, 4), e1 = __shfl_sync(0xffffffffu, s1, l, 4);
-                if (b0 >= 0 && b0 == a0) acc0 = acc0 + e0;
-                if (b1 >= 0 && b1 == a0) acc0 = acc0 + e1;
-                if (b0 >= 0 && b0 == a1) acc1 = acc1 + e0;
-                if (b1 >= 0 && b1 == a1) acc1 = acc1 + e1;
+                for (int l = 1; l < 4; ++l) {
+                    const T before = __shfl_sync(0xffffffffu, acc, l - 1, 4);
+                    if ((threadIdx.x & 3) == l) acc = (before + s0) + s1;
+                }
+                if ((threadIdx.x & 3) == 3) restrictTo(g, whole, acc, B.tag);
+            } else {
+                T acc0 = T(0), acc1 = T(0);
+#pragma unroll 1
+                for (int l = 0; l < 4; ++l) {
+                    const int b0 = __shfl_sync(0xffffffffu, a0, l, 4), b1 = __shfl_sync(0xffffffffu, a1, l, 4);
+                    const T e0 = __shfl_sync(0xffffffffu, s0, l, 4), e1 = __shfl_sync(0xffffffffu, s1, l, 4);
+                    if (b0 >= 0 && b0 == a0) acc0 = acc0 + e0;
+                    if (b1 >= 0 && b1 == a0) acc0 = acc0 + e1;
+                    if (b0 >= 0 && b0 == a1) acc1 = acc1 + e0;
+                    if (b1 >= 0 && b1 == a1) acc1 = acc1 + e1;
+                }
+#pragma unroll 1
+                for (int h = 0; h < 2; ++h)
+                    if (h == 0 || a1 != a0) restrictTo(g, h == 0 ? a0 : a1, h == 0 ? acc0 : acc1, B.tag);
             }
-            restrictTo(g, a0, acc0);
-            if (a1 != a0) restrictTo(g, a1, acc1);
         }
         return;
     }
@@ -273,14 +313,13 @@ __device__ __forceinline__ void solvePair(const Scn<R>& g, const SolveBufs<R>& B
     const int o = kRed ? ro : 1 - ro;
     const int c = kRed ? cr : cb, cIn = kRed ? cb : cr;
     const bool cOn = kRed ? rOn : bOn, inOn = kRed ? bOn : rOn;
-    const bool hx = o ? i0 + 2 < nx : i0 > 0;
-    const int nb[5] = {hx ? (o ? c + 1 : c - 1) : c, j > 0 ? c - nx : c, j < ny - 1 ? c + nx : c,
-                       k > 0 ? c - sxy : c, k < nz - 1 ? c + sxy : c};
+    const int nb[5] = {(o ? at.xp() : at.xm()) ? (o ? c + 1 : c - 1) : c, at.ym() ? c - nx : c,
+                       at.yp() ? c + nx : c, at.zm() ? c - sxy : c, at.zp() ? c + sxy : c};
     const T* z = B.z;
     T v[5], vIn;
     vIn = z[cIn];
 #pragma unroll
-    for (int f = 0; f < 5; ++f) v[f] = z[live ? nb[f] : 0];
+    for (int f = 0; f < 5; ++f) v[f] = z[nb[f]];
     const unsigned cd = cf[c];
     if constexpr (MODE == PASS_BLACK) {   // red neighbours: z plus the prolongated correction
         const int* af = g.lv[0].agg;
@@ -305,7 +344,7 @@ __device__ __forceinline__ void solvePair(const Scn<R>& g, const SolveBufs<R>& B
     n.zm = v[3];
     n.zp = v[4];
     auto sum = [&](auto sign, T start) -> T {
-        return l0Sum<decltype(sign)::value>(g, start, cd, n, i0 + o, j, k);
+        return l0Sum<decltype(sign)::value>(g, start, cd, n, c);
     };
     using Plus = std::integral_constant<int, 1>;
     using Minus = std::integral_constant<int, -1>;
@@ -363,17 +402,31 @@ __device__ __forceinline__ void solvePair(const Scn<R>& g, const SolveBufs<R>& B
         const int a = cOn ? af[c] : -1, ab = inOn ? af[cIn] : -1;
         T res = T(0);
         if (a >= 0) res = sum(Plus{}, T(0));
-        T acc = T(0), accB = T(0);
-        const bool apart = __any_sync(0xffffffffu, ab >= 0 && ab != a);   // pieces of a block that are not joined
+        int whole = max(a, ab);
+        whole = max(whole, __shfl_xor_sync(0xffffffffu, whole, 1));
+        whole = max(whole, __shfl_xor_sync(0xffffffffu, whole, 2));
+        if (__all_sync(0xffffffffu, (a < 0 || a == whole) && (ab < 0 || ab == whole))) {
+            // one aggregate per block: its last lane has the sum
+            T acc = res;
 #pragma unroll
-        for (int l = 0; l < 4; ++l) {
-            const int al = __shfl_sync(0xffffffffu, a, l, 4);
-            const T rl = __shfl_sync(0xffffffffu, res, l, 4);
-            if (al >= 0 && al == a) acc = acc + rl;
-            if (apart && al >= 0 && al == ab) accB = accB + rl;
+            for (int l = 1; l < 4; ++l) {
+                const T before = __shfl_sync(0xffffffffu, acc, l - 1, 4);
+                if ((threadIdx.x & 3) == l) acc = before + res;
+            }
+            if ((threadIdx.x & 3) == 3) restrictTo(g, whole, acc, B.tag);
+        } else {
+            T acc = T(0), accB = T(0);
+#pragma unroll 1
+            for (int l = 0; l < 4; ++l) {
+                const int al = __shfl_sync(0xffffffffu, a, l, 4);
+                const T rl = __shfl_sync(0xffffffffu, res, l, 4);
+                if (al >= 0 && al == a) acc = acc + rl;
+                if (al >= 0 && al == ab) accB = accB + rl;
+            }
+#pragma unroll 1
+            for (int h = 0; h < 2; ++h)
+                if (h == 0 || ab != a) restrictTo(g, h == 0 ? a : ab, h == 0 ? acc : accB, B.tag);
         }
-        restrictTo(g, a, acc);
-        if (ab != a) restrictTo(g, ab, accB);
     }
 }
 
@@ -389,7 +442,7 @@ struct Team {
 // the kernel has to end. *gaveUp is shared memory, 0 at first.
 __device__ __forceinline__ bool teamSync(Team& t, volatile int* gaveUp) {
     __syncthreads();
-    if (t.size == 1) return true;
+    if (t.size == 1) return *gaveUp == 0;
     t.target += (unsigned)t.size;
     if (threadIdx.x == 0) {
         asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(t.bar) : "memory");
@@ -417,6 +470,19 @@ __device__ __forceinline__ F2 f2Load(const double* p) {
     return F2{v.x, v.y};
 }
 __device__ __forceinline__ void f2Store(double* p, F2 v) { *reinterpret_cast<float2*>(p) = make_float2(v.hi, v.lo); }
+// a double-float as two tagged words
+__device__ __forceinline__ void tagStorePair(double* part, int t, F2 v, unsigned tag) {
+    const unsigned long long w = (unsigned long long)tag << 32;
+    asm volatile("st.relaxed.gpu.global.v2.u64 [%0], {%1, %2};" ::"l"(part + 2 * (size_t)t), "l"(w | __float_as_uint(v.hi)),
+                 "l"(w | __float_as_uint(v.lo))
+                 : "memory");
+}
+__device__ __forceinline__ bool tagLoadPair(const double* part, int t, unsigned tag, F2& v) {
+    unsigned long long hi, lo;
+    asm volatile("ld.relaxed.gpu.global.v2.u64 {%0, %1}, [%2];" : "=l"(hi), "=l"(lo) : "l"(part + 2 * (size_t)t) : "memory");
+    v = F2{__uint_as_float((unsigned)hi), __uint_as_float((unsigned)lo)};
+    return (unsigned)(hi >> 32) == tag && (unsigned)(lo >> 32) == tag;
+}
 // a float as a double by its bits (a conversion instruction takes some hundred
 // cycles here); zeros and numbers below the normal range take the conversion
 __device__ __forceinline__ double widen(float f) {
@@ -433,21 +499,33 @@ __device__ __forceinline__ double warpSumAll(double v) {   // the same value in 
 // blocks and one such CTA over their sums: thread i adds groups i, i + 128, ...
 // All threads form the groups' sums first (sh: a value per thread of the CTA), so that
 // thread i waits for one load, not for one per group.
-__device__ __forceinline__ double teamTotalF2(const double* part, int nt, double* sh, double* sh4) {
+// TAGGED: the partials are tagged words, waited for instead of a team barrier.
+template <bool TAGGED>
+__device__ __forceinline__ double teamTotalF2(const double* part, int nt, double* sh, double* sh4, unsigned tag,
+                                              const TagWait& tw) {
     const int tid = (int)threadIdx.x, n4 = (nt + 3) / 4;
     double acc = 0;
     for (int i0 = 0; i0 < n4; i0 += (int)blockDim.x) {
         const int i = i0 + tid;
         if (i < n4) {
             F2 w[4];
+            auto read = [&] {
+                bool ok = true;
 #pragma unroll
-            for (int e = 0; e < 4; ++e) {
-                w[e] = F2{0.f, 0.f};
-                if (4 * i + e < nt) {
-                    const float2 v = __ldcg(reinterpret_cast<const float2*>(part + 4 * i + e));
-                    w[e] = F2{v.x, v.y};
+                for (int e = 0; e < 4; ++e) {
+                    w[e] = F2{0.f, 0.f};
+                    if (4 * i + e < nt) {
+                        if (TAGGED) {
+                            ok &= tagLoadPair(part, 4 * i + e, tag, w[e]);
+                        } else {
+                            const float2 v = __ldcg(reinterpret_cast<const float2*>(part + 4 * i + e));
+                            w[e] = F2{v.x, v.y};
+                        }
+                    }
                 }
-            }
+                return ok;
+            };
+            waitFor(tw, read);
             const F2 v = f2add(f2add(w[0], w[2]), f2add(w[1], w[3]));
             sh[tid] = widen(v.hi) + widen(v.lo);
         }
@@ -472,18 +550,27 @@ __device__ __forceinline__ double teamTotalF2(const double* part, int nt, double
 // first. What counts here is the chain of FP64 instructions (an addition takes
 // some hundred cycles, an FP32-to-FP64 conversion more): the loads of sixteen
 // values are in flight together, and they are added as a tree.
-__device__ __forceinline__ double teamTotal(const double* part, int nt, double* sh256) {
+template <bool TAGGED>
+__device__ __forceinline__ double teamTotal(const double* part, int nt, double* sh256, unsigned tag, const TagWait& tw) {
     const int tid = (int)threadIdx.x;
     double acc = 0;
     const int step = nt > 512 ? 256 : 32;
     if (tid < step) {
         for (int i0 = tid; i0 < nt; i0 += 16 * step) {
             double v[16];
+            waitFor(tw, [&] {
+                bool ok = true;
 #pragma unroll
-            for (int e = 0; e < 16; ++e) {
-                const int i = i0 + e * step;
-                v[e] = i < nt ? __ldcg(part + i) : 0.0;
-            }
+                for (int e = 0; e < 16; ++e) {
+                    const int i = i0 + e * step;
+                    v[e] = 0.0;
+                    if (i < nt) {
+                        if (TAGGED) ok &= tagLoad(reinterpret_cast<const unsigned long long*>(part), i, tag, v[e]);
+                        else v[e] = __ldcg(part + i);
+                    }
+                }
+                return ok;
+            });
 #pragma unroll
             for (int e = 0; e < 16; e += 4)
                 if ((i0 & ~31) + e * step < nt) acc += (v[e] + v[e + 1]) + (v[e + 2] + v[e + 3]);
@@ -526,6 +613,8 @@ __device__ __forceinline__ void ctaMaxStore(double* dst, V v, V* sh) {
         if (l == 0) *dst = (double)x;
     }
 }
+
+constexpr int RRJ_LANES = 8;   // lanes per unknown of a restriction
 
 // ---- coarse rows in shared memory ---------------------------------------------
 // A warp's rows of a coarse level are the same in every V-cycle, so their
@@ -585,68 +674,139 @@ __device__ __forceinline__ void keepRows(const Level<R>& L, int I, bool toNext, 
     }
     if (lane == 0) *out = s;
 }
-// jacobiRow for a kept row
+// The couplings of a level's row: kept in shared memory, or the level's arrays
 template <class R>
-__device__ __forceinline__ void jacobiKept(const Scn<R>& g, const RowView<R>& v, int width, int I, int l, int mode) {
-    using T = R;
-    const Level<R>& L = g.lv[l];
-    if (I >= L.n) return;
-    const int lane = (int)(threadIdx.x & 31);
-    const bool toX = mode == 1 || mode == 3, prolong = mode == 2 || mode == 3;
-    const R* in = toX ? L.y : L.x;
-    const R* xc = g.lv[l + 1].x;
-    R* out = toX ? L.x : L.y;
-    T s = L.b[I], xI = in[I];
-    T cI = T(0);
-    if (prolong) cI = xc[v.own[lane]];
-    for (int e0 = 0; e0 < width; e0 += 8) {
-        T x[8], c[8];
+struct KeptRow {
+    RowView<R> v;
+    int n, lane;
+    __device__ __forceinline__ int col(int e) const { return v.col[32 * e + lane]; }
+    __device__ __forceinline__ int next(int e, int) const { return v.next[32 * e + lane]; }
+    __device__ __forceinline__ R val(int e) const { return v.val[32 * e + lane]; }
+    static constexpr bool FAR = false;
+};
+template <class R>
+struct StoredRow {
+    const Level<R>& L;
+    int q0, n;
+    __device__ __forceinline__ int col(int e) const { return L.col[q0 + e]; }
+    __device__ __forceinline__ int next(int, int c) const { return L.agg[c]; }
+    __device__ __forceinline__ R val(int e) const { return L.val[q0 + e]; }
+    static constexpr bool FAR = sizeof(R) == 4;   // values loaded with the columns (FP64 has no registers for them)
+};
+// the sums of a sweep and of a residual: s plus the couplings times in[col], eight at a
+// time with their loads in flight together. PROLONG: in plus the coarser level's xc.
+template <class R, bool PROLONG, class Row, class Vec>
+__device__ __forceinline__ R rowSum(R s, const Row& row, Vec in, Vec xc, unsigned tag, const TagWait& w) {
+    for (int e0 = 0; e0 < row.n; e0 += 8) {
+        int col[8], nxt[8];
+        R x[8], c[8], v[8];
 #pragma unroll
         for (int e = 0; e < 8; ++e) {
-            const int at = 32 * min(e0 + e, width - 1) + lane;
-            x[e] = in[v.col[at]];
-            if (prolong) c[e] = xc[v.next[at]];
+            col[e] = row.col(min(e0 + e, row.n - 1));
+            if (Row::FAR) v[e] = row.val(min(e0 + e, row.n - 1));
+            if (PROLONG) nxt[e] = row.next(min(e0 + e, row.n - 1), col[e]);
         }
+        waitFor(w, [&] {
+            bool ok = true;
+#pragma unroll
+            for (int e = 0; e < 8; ++e) {
+                ok &= tagLoad(in, col[e], tag, x[e]);
+                if (PROLONG) ok &= tagLoad(xc, nxt[e], tag, c[e]);
+            }
+            return ok;
+        });
 #pragma unroll
         for (int e = 0; e < 8; ++e)
-            if (e0 + e < width) s = madd(s, v.val[32 * (e0 + e) + lane], prolong ? x[e] + c[e] : x[e]);
+            if (e0 + e < row.n) s = madd(s, Row::FAR ? v[e] : row.val(e0 + e), PROLONG ? x[e] + c[e] : x[e]);
     }
-    if (prolong) xI = xI + cI;
-    out[I] = jacobiValue(s, xI, v.diag[lane], v.diag[lane]);
+    return s;
 }
-// resRestrictJac0Warp for kept rows: lane c of the eight lanes of unknown J has J's
-// child c
+// damped Jacobi sweep of row I of level l (jacobi, pressure_mg.cpp:237-247).
+// SWEEP_DOWN: the second sweep on the way down; SWEEP_UP: the first on the way up, from
+// the iterate plus the coarser level's prolongated x (:290-297); SWEEP_LAST: the second
+// on the way up; SWEEP_ONLY: the one on the way up of the mixed path's one-sweep
+// schedule. The last value of level 1 goes to its plain array, which the black
+// sweep of level 0 reads after a team barrier.
+enum { SWEEP_DOWN = 0, SWEEP_UP, SWEEP_LAST, SWEEP_ONLY };
+template <class R, int SWEEP, class Row>
+__device__ __forceinline__ void jacobiRow(const Scn<R>& g, int l, int I, const Row& row, int own, R dg, R omd, unsigned tag,
+                                          const TagWait& w) {
+    using T = R;
+    const Level<R>& L = g.lv[l];
+    constexpr bool prolong = SWEEP == SWEEP_UP || SWEEP == SWEEP_ONLY;
+    const Level<R>& C = g.lv[l + 1];
+    const auto in = SWEEP == SWEEP_DOWN || SWEEP == SWEEP_ONLY ? L.yd : SWEEP == SWEEP_UP ? L.xd : L.yu;
+    T s, x, c = T(0);
+    waitFor(w, [&] {
+        bool ok = tagLoad(L.b, I, tag, s);
+        ok &= tagLoad(in, I, tag, x);
+        if (prolong) ok &= tagLoad(C.xu, own, tag, c);
+        return ok;
+    });
+    s = rowSum<R, prolong>(s, row, in, C.xu, tag, w);
+    const T v = jacobiValue(s, prolong ? x + c : x, dg, omd);
+    if (SWEEP == SWEEP_DOWN) tagStore(L.xd, I, v, tag);
+    else if (SWEEP == SWEEP_UP) tagStore(L.yu, I, v, tag);
+    else if (l == 1) L.x[I] = v;
+    else tagStore(L.xu, I, v, tag);
+}
+// residual of level l fused with its restriction to level l+1 and the first
+// (from-zero) Jacobi sweep of level l+1 (pressure_mg.cpp:248-257, 285-286,
+// 237-247). Eight lanes serve one unknown J of level l+1: they compute the
+// residuals of J's children eight at a time (children in ascending order), and
+// the group's first lane sums them in that order -- the order of the reference's
+// scatter. Every lane of the warp takes part (warp shuffles).
 template <class R>
-__device__ __forceinline__ void resRestrictKept(const Scn<R>& g, const RowView<R>& v, int width, int jBase, int l) {
+__device__ __forceinline__ void restrictRows(const Scn<R>& g, int l, int jBase, const unsigned* pool, const RowSet& rs,
+                                             unsigned tag, const TagWait& w) {
     using T = R;
     const Level<R>& L = g.lv[l];
     const Level<R>& C = g.lv[l + 1];
-    const int lane = (int)(threadIdx.x & 31), J = jBase + lane / RRJ_LANES;
-    const R* it = g.smooth1 ? L.y : L.x;
-    const int I = v.own[lane];
-    const T dg = v.diag[lane];
-    T bI = T(0), xI = T(0);
-    if (I >= 0) { bI = L.b[I]; xI = it[I]; }
-    T s = madd(bI, -dg, xI);
-    for (int e0 = 0; e0 < width; e0 += 8) {
-        T x[8];
-#pragma unroll
-        for (int e = 0; e < 8; ++e) x[e] = it[v.col[32 * min(e0 + e, width - 1) + lane]];
-#pragma unroll
-        for (int e = 0; e < 8; ++e) if (e0 + e < width) s = madd(s, v.val[32 * (e0 + e) + lane], x[e]);
-    }
-    if (!(dg > 0)) s = T(0);
-    const unsigned valid = __ballot_sync(0xffffffffu, I >= 0);
+    const int lane = (int)(threadIdx.x & 31), J = jBase + lane / RRJ_LANES, c = lane % RRJ_LANES;
     const int lane0 = lane & ~(RRJ_LANES - 1);
+    const auto it = g.smooth1 ? L.yd : L.xd;   // the iterate after the way down
     T acc = T(0);
+    auto residual = [&](int I, T dg, const auto& row) -> T {
+        T bI, xI;
+        waitFor(w, [&] {
+            bool ok = tagLoad(L.b, I, tag, bI);
+            return ok & tagLoad(it, I, tag, xI);
+        });
+        const T s = rowSum<R, false>(madd(bI, -dg, xI), row, it, it, tag, w);
+        return dg > 0 ? s : T(0);
+    };
+    auto addChildren = [&](T s, bool on) {   // the group's eight in ascending order
+        __syncwarp();
+        const unsigned valid = __ballot_sync(0xffffffffu, on);
 #pragma unroll
-    for (int q = 0; q < RRJ_LANES; ++q) {
-        const T rq = __shfl_sync(0xffffffffu, s, lane0 + q);
-        if ((valid >> (lane0 + q)) & 1u) acc = acc + rq;
+        for (int q = 0; q < RRJ_LANES; ++q) {
+            const T rq = __shfl_sync(0xffffffffu, s, lane0 + q);
+            if ((valid >> (lane0 + q)) & 1u) acc = acc + rq;
+        }
+    };
+    if (rs.off >= 0) {
+        const RowView<R> v = rowView<R>(pool, rs);
+        const int I = v.own[lane];
+        T s = T(0);
+        if (I >= 0) s = residual(I, v.diag[lane], KeptRow<R>{v, rs.width, lane});
+        addChildren(s, I >= 0);
+    } else {
+        const int e0 = J < C.n ? L.childStart[J] : 0, nch = J < C.n ? L.childStart[J + 1] - e0 : 0;
+        const int chunks = __reduce_max_sync(0xffffffffu, (nch + RRJ_LANES - 1) / RRJ_LANES);
+#pragma unroll 1
+        for (int ch = 0; ch < chunks; ++ch) {
+            const int I = ch * RRJ_LANES + c < nch ? L.child[e0 + ch * RRJ_LANES + c] : -1;
+            T s = T(0);
+            if (I >= 0) {
+                const int q0 = L.rowStart[I];
+                s = residual(I, L.diag[I], StoredRow<R>{L, q0, L.rowStart[I + 1] - q0});
+            }
+            addChildren(s, I >= 0);
+        }
     }
     if (J < C.n && lane == lane0) {
-        C.b[J] = acc;
-        if (l + 1 < g.nLevels - 1) C.y[J] = jacobiValue(acc, T(0), C.diag[J], C.omd[J]);
+        tagStore(C.b, J, acc, tag);
+        if (l + 1 < g.nLevels - 1) tagStore(C.yd, J, jacobiValue(acc, T(0), C.diag[J], C.omd[J]), tag);
     }
 }
 
@@ -708,7 +868,9 @@ k_solve(const Scn<R>* __restrict__ S, SolveArgs a) {
     __shared__ double shSum[256], shZone[8], shMax[2];
     __shared__ RowSet rowsJ[MAX_LEVELS][TH / 32][ROW_CHUNKS], rowsR[MAX_LEVELS][TH / 32][ROW_CHUNKS];
     __shared__ int poolUsed;
-    __shared__ double shDot[2][TH];   // the tiles' dot products, by turns
+    __shared__ double shDot[2][sizeof(R) == 8 ? TH : TH / 2];   // FP64: the tiles' dot products, by turns; scratch
+    R* const shB = reinterpret_cast<R*>(pool + SolveCfg<R>::ROWS / 4);   // the coarsest right-hand side
+    double* const shTerms = reinterpret_cast<double*>(pool + SolveCfg<R>::ROWS / 4);   // FP32: a tile's terms, by turns
     __shared__ double shMx[32];
     __shared__ int first[MAX_BATCH + 1];
     __shared__ int gaveUp;
@@ -759,7 +921,6 @@ k_solve(const Scn<R>* __restrict__ S, SolveArgs a) {
         const int nblk = (int)g.dvL0[1].d * ((g.nz + 1) >> 1);
         const SolveTiling tl = solveTiling<R>(nblk);
         const int nt = tl.nt;
-        const int t0 = (int)((long long)nt * team.rank / team.size), t1 = (int)((long long)nt * (team.rank + 1) / team.size);
         const int rank = team.rank, size = team.size;
         double* const partDq = g.part + (size_t)PS_DQ * g.partStride;
         double* const partRz = g.part + (size_t)PS_RZ * g.partStride;
@@ -773,32 +934,41 @@ k_solve(const Scn<R>* __restrict__ S, SolveArgs a) {
         // one pass over the team's tiles
         const int slot = warp / tl.warps, slots = TH / 32 / tl.warps, wt = warp - slot * tl.warps;
         int turn = 0;
+        // Tiles are dealt out to the CTAs by turns: neighbouring tiles have like shares of
+        // gas, so this evens out the CTAs' work (FP64 house step 2.93 -> 2.75 ms, 8
+        // scenarios 4.38 -> 4.19; FP32 house 1.25 -> 1.23). An FP32 CTA with several
+        // rounds of tiles takes neighbours instead, which share cached rows (24 scenarios
+        // 6.06 ms against 6.14 dealt out); its many tiles even out by themselves.
+        const bool deal = !kMixed || nt <= slots * team.size;
+        const int tFirst = deal ? team.rank + slot * team.size : (int)((long long)nt * team.rank / team.size) + slot;
+        const int tEnd = deal ? nt : (int)((long long)nt * (team.rank + 1) / team.size), tStep = deal ? slots * team.size : slots;
         auto pairs = [&](auto mode, auto even, double* part, T& rm, bool writeZ) {
             constexpr int MODE = decltype(mode)::value;
             constexpr bool kDot = MODE == PASS_APPLY || MODE == PASS_RED;
-            for (int t = t0 + slot; t < t1; t += slots) {
+            for (int t = tFirst; t < tEnd; t += tStep) {
                 double dot = 0;
                 F2 e0{0.f, 0.f}, e1{0.f, 0.f};
-                for (int q = 0; q < tl.reps; ++q)
-                    solvePair<R, MODE, decltype(even)::value>(g, B, ((t * tl.reps + q) * tl.warps + wt) * 32 + lane, nblk,
-                                                              dot, e0, e1, rm, writeZ);
+                for (int q = 0; q < tl.reps; ++q) {
+                    const PairPlace<R> at(g, ((t * tl.reps + q) * tl.warps + wt) * 32 + lane, nblk);
+                    solvePair<R, MODE, decltype(even)::value>(g, B, at, dot, e0, e1, rm, writeZ);
+                }
                 if constexpr (kDot && kMixed) {
-                    // a block's eight terms in ascending order over its four lanes, the
-                    // 32 blocks of the tile by one warp
-                    F2 acc = f2add(e0, e1);
-#pragma unroll
-                    for (int l = 1; l < 4; ++l) {
-                        const F2 before{__shfl_sync(0xffffffffu, acc.hi, l - 1, 4), __shfl_sync(0xffffffffu, acc.lo, l - 1, 4)};
-                        const F2 next = f2add(f2add(before, e0), e1);
-                        if ((lane & 3) == l) acc = next;
-                    }
-                    double* const sh = shDot[turn] + 32 * slot;
+                    // the tile's terms side by side: the first warp adds each block's eight in
+                    // ascending order (one block a lane), then its 32 blocks
+                    double* const sh = shTerms + 2 * TH * turn + 256 * slot;
                     turn ^= 1;
-                    if ((lane & 3) == 3) f2Store(sh + wt * 8 + (lane >> 2), acc);
+                    f2Store(sh + 64 * wt + 2 * lane, e0);
+                    f2Store(sh + 64 * wt + 2 * lane + 1, e1);
                     asm volatile("bar.sync %0, 128;" ::"r"(slot + 1) : "memory");
                     if (wt == 0) {
-                        acc = warpSum(f2Load(sh + lane));
-                        if (lane == 0) f2Store(part + t, acc);
+                        F2 acc = f2Load(sh + 8 * lane);
+#pragma unroll
+                        for (int u = 1; u < 8; ++u) acc = f2add(acc, f2Load(sh + 8 * lane + u));
+                        acc = warpSum(acc);
+                        if (lane == 0) {
+                            if (MODE == PASS_APPLY) tagStorePair(part, t, acc, B.tag);
+                            else f2Store(part + t, acc);
+                        }
                     }
                 } else if constexpr (kDot) {
                     if (tl.warps > 1) {   // the tile's first warp adds the warps' lanes
@@ -811,7 +981,10 @@ k_solve(const Scn<R>* __restrict__ S, SolveArgs a) {
                     }
                     if (wt == 0) {
                         dot = warpSumAll(dot);
-                        if (lane == 0) part[t] = dot;
+                        if (lane == 0) {
+                            if (MODE == PASS_APPLY) tagStore(reinterpret_cast<unsigned long long*>(part), t, dot, B.tag);
+                            else part[t] = dot;
+                        }
                     }
                 }
             }
@@ -831,30 +1004,59 @@ k_solve(const Scn<R>* __restrict__ S, SolveArgs a) {
                 if (lane == 0) rowsJ[l][warp][m].off = rowsR[l][warp][m].off = -1;
                 __syncwarp();
                 if (chunk * 32 < L.n)
-                    keepRows(L, I < L.n ? I : -1, true, pool, &poolUsed, SolveCfg<R>::POOL / 4, &rowsJ[l][warp][m]);
+                    keepRows(L, I < L.n ? I : -1, true, pool, &poolUsed, SolveCfg<R>::ROWS / 4, &rowsJ[l][warp][m]);
                 if (chunk * (32 / RRJ_LANES) < C.n) {
                     const int J = chunk * (32 / RRJ_LANES) + lane / RRJ_LANES, c = lane % RRJ_LANES;
                     const int e0 = J < C.n ? L.childStart[J] : 0, nch = J < C.n ? L.childStart[J + 1] - e0 : 0;
                     if (__reduce_max_sync(0xffffffffu, nch) <= RRJ_LANES)
-                        keepRows(L, c < nch ? L.child[e0 + c] : -1, false, pool, &poolUsed, SolveCfg<R>::POOL / 4,
+                        keepRows(L, c < nch ? L.child[e0 + c] : -1, false, pool, &poolUsed, SolveCfg<R>::ROWS / 4,
                                  &rowsR[l][warp][m]);
                 }
                 __syncwarp();
             }
-        auto jacobiLevel = [&](int l, int mode) {
-            const int n = g.lv[l].n;
-            for (int m = 0, i = gw * 32; i < n; ++m, i += nw * 32) {
+        const TagWait tw{&gaveUp, g.errWord};
+        auto jacobiLevel = [&](auto sweep, int l) {
+            constexpr int SWEEP = decltype(sweep)::value;
+            const Level<R>& L = g.lv[l];
+            for (int m = 0, i = gw * 32; i < L.n; ++m, i += nw * 32) {
                 const RowSet rs = m < ROW_CHUNKS ? rowsJ[l][warp][m] : RowSet{-1, 0};
-                if (rs.off >= 0) jacobiKept(g, rowView<R>(pool, rs), rs.width, i + lane, l, mode);
-                else jacobiRow(g, i + lane, l, mode);
+                const int I = i + lane;
+                if (I >= L.n) continue;
+                if (rs.off >= 0) {
+                    const RowView<R> v = rowView<R>(pool, rs);
+                    jacobiRow<R, SWEEP>(g, l, I, KeptRow<R>{v, rs.width, lane}, v.own[lane], v.diag[lane], v.diag[lane], B.tag, tw);
+                } else {
+                    const int q0 = L.rowStart[I];
+                    jacobiRow<R, SWEEP>(g, l, I, StoredRow<R>{L, q0, L.rowStart[I + 1] - q0}, L.agg[I], L.diag[I], L.omd[I], B.tag, tw);
+                }
             }
         };
         auto restrictLevel = [&](int l) {
             constexpr int PER = 32 / RRJ_LANES;
-            for (int m = 0, j = gw * PER; j < g.lv[l + 1].n; ++m, j += nw * PER) {
-                const RowSet rs = m < ROW_CHUNKS ? rowsR[l][warp][m] : RowSet{-1, 0};
-                if (rs.off >= 0) resRestrictKept(g, rowView<R>(pool, rs), rs.width, j, l);
-                else resRestrictJac0Warp(g, j, l);
+            for (int m = 0, j = gw * PER; j < g.lv[l + 1].n; ++m, j += nw * PER)
+                restrictRows(g, l, j, pool, m < ROW_CHUNKS ? rowsR[l][warp][m] : RowSet{-1, 0}, B.tag, tw);
+        };
+        auto coarsest = [&]() {
+            const Level<R>& L = g.lv[nl - 1];
+            auto put = [&](int I, T v) {
+                if (nl == 2) L.x[I] = v;
+                else tagStore(L.xu, I, v, B.tag);
+            };
+            if (L.dense) {
+                for (int i = tid; i < L.n; i += TH) {
+                    T v = T(0);
+                    waitFor(tw, [&] { return tagLoad(L.b, i, B.tag, v); });
+                    shB[i] = v;
+                }
+                __syncthreads();
+                for (int row = gw; row < L.n; row += nw) {
+                    const T v = coarseDenseRow(L, row, shB);
+                    if (lane == 0) put(row, v);
+                }
+            } else if (rank == 0 && tid == 0) {
+                R* const x = L.x;
+                coarseSerial(L, B.tag, tw, x);
+                for (int I = 0; I < L.n; ++I) put(I, x[I]);
             }
         };
         // the cells of the grid, elementwise
@@ -951,8 +1153,10 @@ k_solve(const Scn<R>* __restrict__ S, SolveArgs a) {
             PHX_TEAM_SYNC();
         }
 
+        const unsigned tag0 = *g.tagBase;
         T none = T(0);
         for (int phase = a.vcycleOnly ? 2 : 0, loop = 0;; phase = 1, ++loop) {
+            B.tag = tag0 + 1u + (unsigned)loop;
             bool haveRed = false;   // the update has set the red cells of z
             if (phase == 1) {
                 B.beta = (T)cg.beta;
@@ -962,8 +1166,11 @@ k_solve(const Scn<R>* __restrict__ S, SolveArgs a) {
                     B.dNew = cg.it & 1 ? g.d : g.tmp[0];
                 }
                 PHX_PASS(PASS_APPLY, partDq, none, false);
-                PHX_TEAM_SYNC();
-                const double total = kMixed ? teamTotalF2(partDq, nt, shDot[0], shSum) : teamTotal(partDq, nt, shSum);
+                // tagged partial sums take no barrier: a thread updates the cells it has just formed
+                // q and d for, and every read of z was done before the reader's partial sum
+                __syncthreads();
+                const double total = kMixed ? teamTotalF2<true>(partDq, nt, shDot[0], shSum, B.tag, tw)
+                                            : teamTotal<true>(partDq, nt, shSum, B.tag, tw);
                 if (tid == 0) {
                     cg.dq = total;
                     if (cg.brk == 1) {   // the iteration after a breakdown: no update, then a restart
@@ -1009,31 +1216,27 @@ k_solve(const Scn<R>* __restrict__ S, SolveArgs a) {
             PHX_PASS(PASS_BLACK0, nullptr, none, true);
             PHX_TEAM_SYNC();
             PHX_PASS(PASS_RES, nullptr, none, true);
-            PHX_TEAM_SYNC();
+            using Down = std::integral_constant<int, SWEEP_DOWN>;
+            using Up = std::integral_constant<int, SWEEP_UP>;
+            using Last = std::integral_constant<int, SWEEP_LAST>;
+            using Only = std::integral_constant<int, SWEEP_ONLY>;
+            // the coarse levels: with tagged values no barrier until level 1's correction is whole
             for (int l = 1; l < nl - 1; ++l) {
                 if (!g.smooth1) {
-                    jacobiLevel(l, 1);
-                    PHX_TEAM_SYNC();
+                    jacobiLevel(Down{}, l);
                 }
                 restrictLevel(l);
-                PHX_TEAM_SYNC();
             }
-            if (g.lv[nl - 1].dense) {
-                for (int row = gw; row < g.lv[nl - 1].n; row += nw) coarseDenseRow(g, row);
-            } else if (rank == 0) {
-                coarseSerialTile(g);
-            }
-            PHX_TEAM_SYNC();
+            coarsest();
             for (int l = nl - 2; l >= 1; --l) {
                 if (g.smooth1) {
-                    jacobiLevel(l, 3);
+                    jacobiLevel(Only{}, l);
                 } else {
-                    jacobiLevel(l, 2);
-                    PHX_TEAM_SYNC();
-                    jacobiLevel(l, 1);
+                    jacobiLevel(Up{}, l);
+                    jacobiLevel(Last{}, l);
                 }
-                PHX_TEAM_SYNC();
             }
+            PHX_TEAM_SYNC();
             PHX_PASS(PASS_BLACK, nullptr, none, true);
             PHX_TEAM_SYNC();
             PHX_PASS(PASS_RED, partRz, none, true);
@@ -1048,7 +1251,8 @@ k_solve(const Scn<R>* __restrict__ S, SolveArgs a) {
                 m = warpMaxPos(m);
                 if (lane == 0) shMax[which] = m;
             }
-            const double total = kMixed ? teamTotalF2(partRz, nt, shDot[0], shSum + 4) : teamTotal(partRz, nt, shSum);
+            const double total = kMixed ? teamTotalF2<false>(partRz, nt, shDot[0], shSum + 4, B.tag, tw)
+                                        : teamTotal<false>(partRz, nt, shSum, B.tag, tw);
             if (warp == 0) {
                 const double rmax = phase == 1 ? shMax[0] : cg.rmax;
                 const double r64 = kMixed && (phase == 0 || cg.repl != 0) ? shMax[1] : 0.0;

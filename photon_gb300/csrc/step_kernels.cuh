@@ -75,6 +75,14 @@ __device__ bool lastCtaSum(const Scn<R>& g, int slot, int tile, int ntiles, V vT
 __device__ __forceinline__ int ntilesOf(const Dom& d, int s) { return __ldg(d.start + s + 1) - __ldg(d.start + s); }
 
 // ---------------------------------------------------------------------------
+// before a solve or a bare V-cycle: no arrivals at the team barrier yet, and tags
+// that no value of an earlier solve, finished or not, can carry
+template <class R>
+__device__ __forceinline__ void startSolve(const Scn<R>& g) {
+    *g.teamBar = 0;
+    *g.tagBase += (unsigned)max(g.maxIters, 0) + 8u;
+}
+
 // the wind profile's speed at every layer's cell centres, when a scenario's tables are built
 template <class R>
 __global__ void k_wind(const Scn<R>* __restrict__ S, Dom dom) {
@@ -136,7 +144,7 @@ __global__ void k_begin(const Scn<R>* __restrict__ S, Dom dom, int computeDt, do
     }
     sv[SV_FUELIN] = fuelIn;
     sv[SV_WITERS] = sv[SV_PITERS];
-    *g.teamBar = 0;
+    startSolve(g);
     // reductions of this step start from their neutral values
     sv[SV_MAXNU] = 0;
     sv[SV_MAXDIV] = 0;
