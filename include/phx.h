@@ -326,6 +326,11 @@ int phx_rad_trace(struct phx_ctx* ctx, const phx_rad_elem* elems, int n_elems, c
 int phx_batch_rad_trace(struct phx_ctx* ctx, int scenario, const phx_rad_elem* elems, int n_elems,
                         const phx_rad_wall* walls, int n_walls, const double* solid_t, double* rad_abs,
                         double* rad_gas);
+/* the same with each element as a row of 11 numbers: o, n, area, emissivity,
+ * temperature, sphere, skip_own_cell (the last two truncated to int) */
+int phx_batch_rad_trace_rows(struct phx_ctx* ctx, int scenario, const double* rows, int n_elems,
+                             const phx_rad_wall* walls, int n_walls, const double* solid_t, double* rad_abs,
+                             double* rad_gas);
 /* device time (ms, CUDA events) of the last trace's kernels on this context */
 double phx_rad_last_ms(const struct phx_ctx* ctx);
 

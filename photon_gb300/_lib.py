@@ -26,7 +26,7 @@ STAGE_ID = {n: i for i, n in enumerate(STAGES)}
 SYMBOLS = ["phx_create", "phx_destroy", "phx_last_error", "phx_last_global_error", "phx_abi_version", "phx_add_burner",
            "phx_add_ignition", "phx_step", "phx_run", "phx_stage", "phx_precondition", "phx_get_field",
            "phx_set_field", "phx_field_count", "phx_get_stats", "phx_set_scalars", "phx_set_stats", "phx_device_bytes", "phx_sync",
-           "phx_time_steps", "phx_profile_step", "phx_last_step_launches", "phx_rad_trace", "phx_batch_rad_trace", "phx_rad_last_ms", "phx_vol_render", "phx_batch_vol_render", "phx_vol_last_ms", "phx_selftest_wait_timeout", "phx_select_device", "phx_alloc_host",
+           "phx_time_steps", "phx_profile_step", "phx_last_step_launches", "phx_rad_trace", "phx_batch_rad_trace", "phx_batch_rad_trace_rows", "phx_rad_last_ms", "phx_vol_render", "phx_batch_vol_render", "phx_vol_last_ms", "phx_selftest_wait_timeout", "phx_select_device", "phx_alloc_host",
            "phx_free_host", "phx_create_batch", "phx_batch_add", "phx_batch_remove", "phx_batch_size",
            "phx_batch_scenario_bytes", "phx_batch_add_burner", "phx_batch_step", "phx_batch_get_field",
            "phx_batch_set_field", "phx_batch_field_count", "phx_batch_get_stats", "phx_batch_set_stats", "phx_batch_mg_info", "phx_batch_mg_nnz", "phx_batch_tune_vcycle", "phx_gather_stats_noalloc",
@@ -66,6 +66,26 @@ def rad_elements(a) -> np.ndarray:
     r["area"], r["emissivity"], r["temperature"] = a[:, 6], a[:, 7], a[:, 8]
     r["sphere"], r["skip_own_cell"] = a[:, 9].astype(np.int32), a[:, 10].astype(np.int32)
     return r
+
+
+def rad_trace(L, h, s: int, elements, walls, solid_t, gas: bool):
+    """The trace of scenario s as (status, radAbs, radGas or None); solid_t holds a value per
+    cell at least. An (n, 11) array of
+    elements goes to the device as it is: as records it would be written out once more
+    first (210,000 elements: 6.2 ms, the trace itself 2.2 ms)."""
+    rows = not (isinstance(elements, np.ndarray) and elements.dtype == RAD_ELEM_DTYPE)
+    el = np.ascontiguousarray(np.asarray(elements, np.float64).reshape(-1, 11)) if rows else rad_elements(elements)
+    wl = rad_walls(walls)
+    n = L.phx_batch_field_count(h, s, FIELD_ID["T"])
+    st = None if solid_t is None else np.ascontiguousarray(solid_t, np.float64)
+    if st is not None and st.size < n:
+        return PHX_ERR_INVALID, None, None
+    ab = np.zeros(len(el), np.float64)
+    g = np.zeros(n, np.float64) if gas else None
+    trace = L.phx_batch_rad_trace_rows if rows else L.phx_batch_rad_trace
+    r = trace(h, s, el.ctypes.data if len(el) else None, len(el), wl.ctypes.data if len(wl) else None, len(wl),
+              None if st is None else st.ctypes.data, ab.ctypes.data, None if g is None else g.ctypes.data)
+    return r, ab, g
 
 
 def rad_walls(a) -> np.ndarray:
@@ -184,6 +204,7 @@ def load():
     L.phx_batch_tune_vcycle.argtypes = [vp, i, d, vp, i]
     L.phx_rad_trace.argtypes = [vp, vp, i, vp, i, vp, vp, vp]
     L.phx_batch_rad_trace.argtypes = [vp, i, vp, i, vp, i, vp, vp, vp]
+    L.phx_batch_rad_trace_rows.argtypes = [vp, i, vp, i, vp, i, vp, vp, vp]
     L.phx_rad_last_ms.restype = d
     L.phx_rad_last_ms.argtypes = [vp]
     L.phx_vol_render.argtypes = [vp, ctypes.POINTER(PhxVolParams), vp, vp]

@@ -223,7 +223,13 @@ int phx_last_step_launches(const phx_ctx* c) { return c && c->impl ? c->impl->la
 int phx_batch_rad_trace(phx_ctx* c, int s, const phx_rad_elem* elems, int n_elems, const phx_rad_wall* walls,
                         int n_walls, const double* solid_t, double* rad_abs, double* rad_gas) {
     return guarded(c, [&](phx::CtxBase* x) {
-        return x->radTrace(s, elems, n_elems, walls, n_walls, solid_t, rad_abs, rad_gas);
+        return x->radTrace(s, elems, sizeof(phx_rad_elem) / sizeof(double), n_elems, walls, n_walls, solid_t, rad_abs, rad_gas);
+    });
+}
+int phx_batch_rad_trace_rows(phx_ctx* c, int s, const double* rows, int n_elems, const phx_rad_wall* walls, int n_walls,
+                             const double* solid_t, double* rad_abs, double* rad_gas) {
+    return guarded(c, [&](phx::CtxBase* x) {
+        return x->radTrace(s, rows, 11, n_elems, walls, n_walls, solid_t, rad_abs, rad_gas);
     });
 }
 int phx_rad_trace(phx_ctx* c, const phx_rad_elem* elems, int n_elems, const phx_rad_wall* walls, int n_walls,

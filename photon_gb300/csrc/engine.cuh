@@ -610,7 +610,8 @@ public:
     }
     void discard(void* prepared) override { delete static_cast<Scenario<R>*>(prepared); }
     // Solver::traceRadiation (src/sim/radiation.cpp:181-319) for scenario s
-    int radTrace(int s, const phx_rad_elem* el, int nE, const phx_rad_wall* wl, int nW, const double* solidT,
+    // (el: phx_rad_elem records, or rows of 11 doubles; elWords: their doubles)
+    int radTrace(int s, const void* el, int elWords, int nE, const phx_rad_wall* wl, int nW, const double* solidT,
                  double* radAbs, double* radGas) override {
         PHX_TRY(checkScn(s));
         if (nE < 0 || nW < 0 || (nE > 0 && (!el || !radAbs)) || (nW > 0 && !wl)) {
@@ -621,18 +622,21 @@ public:
         const int nx = S.geo.nx, ny = S.geo.ny, nz = S.geo.nz;
         const size_t N = (size_t)nx * ny * nz;
         const size_t NF[3] = {(size_t)(nx + 1) * ny * nz, (size_t)nx * (ny + 1) * nz, (size_t)nx * ny * (nz + 1)};
-        {   // at most one wall per face, every face in range
-            std::vector<size_t> key(nW);
+        const size_t nF = NF[0] + NF[1] + NF[2];
+        {   // at most one wall per face, every face in range (an error of the range comes first)
+            std::vector<uint64_t> seen((nF + 63) / 64);
+            bool two = false;
             for (int w = 0; w < nW; ++w) {
                 if (wl[w].axis < 0 || wl[w].axis > 2 || wl[w].face < 0 || (size_t)wl[w].face >= NF[wl[w].axis]) {
                     err = "radiation wall " + std::to_string(w) + ": axis or face out of range";
                     return PHX_ERR_INVALID;
                 }
-                key[w] = (wl[w].axis == 0 ? 0 : wl[w].axis == 1 ? NF[0] : NF[0] + NF[1]) + (size_t)wl[w].face;
+                const size_t key = (wl[w].axis == 0 ? 0 : wl[w].axis == 1 ? NF[0] : NF[0] + NF[1]) + (size_t)wl[w].face;
+                const uint64_t bit = 1ull << (key & 63);
+                two |= (seen[key >> 6] & bit) != 0;
+                seen[key >> 6] |= bit;
             }
-            std::sort(key.begin(), key.end());
-            for (int w = 1; w < nW; ++w)
-                if (key[w] == key[w - 1]) { err = "two radiation walls on one face"; return PHX_ERR_INVALID; }
+            if (two) { err = "two radiation walls on one face"; return PHX_ERR_INVALID; }
         }
         PHX_TRY(ensureTables());
         PHX_TRY(initStream());
@@ -650,8 +654,8 @@ public:
             rad.cap[b] = bytes;
             return PHX_OK;
         };
-        const size_t nF = NF[0] + NF[1] + NF[2];
-        PHX_TRY(grow(RadWork::EL, nE * sizeof(phx_rad_elem)));
+        const size_t elBytes = (size_t)nE * elWords * sizeof(double);
+        PHX_TRY(grow(RadWork::EL, elBytes));
         PHX_TRY(grow(RadWork::ABS, nE * sizeof(double)));
         PHX_TRY(grow(RadWork::WL, nW * sizeof(phx_rad_wall)));
         PHX_TRY(grow(RadWork::WALLI, nW * 8 * sizeof(R)));
@@ -677,7 +681,7 @@ public:
             PHX_CK(cudaEventCreate(&rad.e0));
             PHX_CK(cudaEventCreate(&rad.e1));
         }
-        phx_rad_elem* dEl = static_cast<phx_rad_elem*>(rad.buf[RadWork::EL]);
+        double* dEl = static_cast<double*>(rad.buf[RadWork::EL]);
         phx_rad_wall* dWl = static_cast<phx_rad_wall*>(rad.buf[RadWork::WL]);
         R* dWallI = static_cast<R*>(rad.buf[RadWork::WALLI]);
         double* dAbs = static_cast<double*>(rad.buf[RadWork::ABS]);
@@ -692,7 +696,7 @@ public:
         R* dRayVal = static_cast<R*>(rad.buf[RadWork::RAYVAL]);
         int* dRayElem = static_cast<int*>(rad.buf[RadWork::RAYELEM]);
         int* dCnt = static_cast<int*>(rad.buf[RadWork::CNT]);
-        if (nE) PHX_CK(cudaMemcpyAsync(dEl, el, nE * sizeof(phx_rad_elem), cudaMemcpyHostToDevice, st));
+        if (nE) PHX_CK(cudaMemcpyAsync(dEl, el, elBytes, cudaMemcpyHostToDevice, st));
         if (nW) PHX_CK(cudaMemcpyAsync(dWl, wl, nW * sizeof(phx_rad_wall), cudaMemcpyHostToDevice, st));
         if (solidT) PHX_CK(cudaMemcpyAsync(dSolid, solidT, N * sizeof(double), cudaMemcpyHostToDevice, st));
         PHX_CK(cudaMemsetAsync(dGas, 0, N * sizeof(R), st));
@@ -704,7 +708,7 @@ public:
         if (nW) k_rad_walls<R><<<(nW + 127) / 128, 128, 0, st>>>(dWl, nW, nx, ny, nz, dWallOf,
                                                                  reinterpret_cast<unsigned*>(dFlags), dWallI, dKc);
         if (nE) {
-            k_rad_elems<R><<<(nE + RAD_ELEMS - 1) / RAD_ELEMS, RAD_ELEMS, 0, st>>>(dS, s, dEl, nE, dKc, dSources, dRays,
+            k_rad_elems<R><<<(nE + RAD_ELEMS - 1) / RAD_ELEMS, RAD_ELEMS, 0, st>>>(dS, s, dEl, elWords, nE, dKc, dSources, dRays,
                                                                                    dRayElem, dRayVal, dCnt);
             k_rad_march<R><<<rad.marchCtas, 256, 0, st>>>(dS, s, nE, dSources, dCells, dFlags, dWallOf, dWallI, dKc,
                                                           dRays, dRayElem, dRayVal, dCnt, dGas);
@@ -713,17 +717,8 @@ public:
         PHX_CK(cudaGetLastError());
         PHX_CK(cudaEventRecord(rad.e1, st));
         if (nE) PHX_CK(cudaMemcpyAsync(radAbs, dAbs, nE * sizeof(double), cudaMemcpyDeviceToHost, st));
-        std::vector<R> gasHost;
-        if (radGas) {
-            if (std::is_same<R, double>::value)
-                PHX_CK(cudaMemcpyAsync(radGas, dGas, N * sizeof(double), cudaMemcpyDeviceToHost, st));
-            else {
-                gasHost.resize(N);
-                PHX_CK(cudaMemcpyAsync(gasHost.data(), dGas, N * sizeof(R), cudaMemcpyDeviceToHost, st));
-            }
-        }
-        PHX_CK(cudaStreamSynchronize(st));
-        if (!gasHost.empty()) for (size_t c = 0; c < N; ++c) radGas[c] = (double)gasHost[c];
+        if (radGas) PHX_TRY(getReal(dGas, N, radGas));
+        else PHX_CK(cudaStreamSynchronize(st));
         float ms = 0;
         PHX_CK(cudaEventElapsedTime(&ms, rad.e0, rad.e1));
         rad.lastMs = ms;
@@ -1462,11 +1457,25 @@ public:
             PHX_CK(cudaStreamSynchronize(st));
             return PHX_OK;
         }
-        std::vector<R> tmp(n);
-        PHX_CK(cudaMemcpyAsync(tmp.data(), src, n * sizeof(R), cudaMemcpyDeviceToHost, st));
+        PHX_CK(cudaMemcpyAsync(upperHalf(out, n), src, n * sizeof(R), cudaMemcpyDeviceToHost, st));
         PHX_CK(cudaStreamSynchronize(st));
-        for (size_t i = 0; i < n; ++i) out[i] = (double)tmp[i];
+        widenUpperHalf(out, n);
         return PHX_OK;
+    }
+    // A caller's n doubles take the device's n reals in their upper half first and are
+    // widened from the front: number i is read before anything that covers it is written
+    // (8 i + 8 <= 4 n + 4 i + 4 for every i < n), block by block through a copy on the
+    // stack. No second array whose pages are touched for the first time on every call
+    // (a trace's C call over 1.3e6 cells, with the walls' bitmap instead of a sort: 3.1 -> 2.2 ms).
+    static void* upperHalf(double* out, size_t n) { return reinterpret_cast<char*>(out) + n * (sizeof(double) - sizeof(R)); }
+    static void widenUpperHalf(double* out, size_t n) {
+        constexpr size_t B = 1024;
+        R part[B];
+        for (size_t i = 0; i < n; i += B) {
+            const size_t m = std::min(B, n - i);
+            std::memcpy(part, static_cast<char*>(upperHalf(out, n)) + i * sizeof(R), m * sizeof(R));
+            for (size_t q = 0; q < m; ++q) out[i + q] = (double)part[q];
+        }
     }
 
     bool fieldPtr(int s, int f, void** p, size_t* n, int* type) const {

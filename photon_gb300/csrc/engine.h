@@ -55,7 +55,7 @@ public:
     virtual void discard(void* prepared) = 0;
     // simulated time of every scenario, one read-back for the batch
     virtual int readTimes(double* out) = 0;
-    virtual int radTrace(int s, const phx_rad_elem* el, int nE, const phx_rad_wall* wl, int nW, const double* solidT,
+    virtual int radTrace(int s, const void* el, int elWords, int nE, const phx_rad_wall* wl, int nW, const double* solidT,
                          double* radAbs, double* radGas) = 0;
     virtual double radLastMs() const = 0;
     virtual int volRender(int s, const phx_vol_params* p, const float* depth, float* rgb) = 0;

@@ -259,12 +259,12 @@ __global__ void k_rad_cells(const Scn<R>* __restrict__ S, int s, const double* _
 // crossings. A direction that is not emitted into gets its result here: 0.
 template <class R>
 __global__ void __launch_bounds__(RAD_ELEMS)
-k_rad_elems(const Scn<R>* __restrict__ S, int s, const phx_rad_elem* __restrict__ els, int nE,
+k_rad_elems(const Scn<R>* __restrict__ S, int s, const double* __restrict__ els, int elWords, int nE,
             const RadConst<R>* __restrict__ kc, RadSource<R>* __restrict__ sources, RadRay<R>* __restrict__ rays,
             int* __restrict__ rayElem, R* __restrict__ rayVal, int* __restrict__ counts) {
     constexpr int WARPS = RAD_ELEMS / 32;
     __shared__ R dir[RAD_DIRS][3];
-    __shared__ R shN[RAD_ELEMS][3], shP[RAD_ELEMS][3], shW[RAD_ELEMS];
+    __shared__ R shN[RAD_ELEMS][3], shP[RAD_ELEMS][3], shW[RAD_ELEMS], shA[RAD_ELEMS];
     __shared__ int kind[RAD_ELEMS];              // 0 no rays, 1 hemisphere, 2 sphere
     __shared__ int room[WARPS][RAD_DIRS];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -276,10 +276,13 @@ k_rad_elems(const Scn<R>* __restrict__ S, int s, const phx_rad_elem* __restrict_
     __syncthreads();
     kind[tid] = 0;
     if (e0 + tid < nE) {
-        const phx_rad_elem& el = els[e0 + tid];
-        const R eps = (R)el.emissivity, temp = (R)el.temperature, area = (R)el.area;
-        const bool sphere = el.sphere != 0;
-        const R n0 = (R)el.n[0], n1 = (R)el.n[1], n2 = (R)el.n[2];
+        // a phx_rad_elem, or its 11 numbers as doubles
+        static_assert(sizeof(phx_rad_elem) == 80, "nine doubles and two ints");
+        const double* el = els + (size_t)(e0 + tid) * elWords;
+        const R eps = (R)el[7], temp = (R)el[8], area = (R)el[6];
+        const bool sphere = elWords == 11 ? (int)el[9] != 0 : reinterpret_cast<const int*>(el + 9)[0] != 0;
+        const bool skipOwn = elWords == 11 ? (int)el[10] != 0 : reinterpret_cast<const int*>(el + 9)[1] != 0;
+        const R n0 = (R)el[3], n1 = (R)el[4], n2 = (R)el[5];
         RadSource<R> o;
         R f[RAD_NB];
         radBandFractions<R>(temp, f);
@@ -298,18 +301,19 @@ k_rad_elems(const Scn<R>* __restrict__ S, int s, const phx_rad_elem* __restrict_
             }
         }
         const R norm = sphere ? (R)1 : (wsum > 0 ? PI / wsum : (R)0);
-        const R px = ((R)el.o[0] - (R)g.ox) / (R)g.dx, py = ((R)el.o[1] - (R)g.oy) / (R)g.dx,
-                pz = ((R)el.o[2] - (R)g.oz) / (R)g.dx;
+        const R px = ((R)el[0] - (R)g.ox) / (R)g.dx, py = ((R)el[1] - (R)g.oy) / (R)g.dx,
+                pz = ((R)el[2] - (R)g.oz) / (R)g.dx;
         const int ci = (int)radFloor(px), cj = (int)radFloor(py), ck = (int)radFloor(pz);
         const bool inside = !(ci < 0 || cj < 0 || ck < 0 || ci >= g.nx || cj >= g.ny || ck >= g.nz);
         o.eps = eps;
         o.cell = inside ? ci + g.nx * (cj + g.ny * ck) : 0;
-        o.skip = el.skip_own_cell ? o.cell : -1;
+        o.skip = skipOwn ? o.cell : -1;
         sources[e0 + tid] = o;
         kind[tid] = !inside ? 0 : sphere ? 2 : 1;
         shN[tid][0] = n0; shN[tid][1] = n1; shN[tid][2] = n2;
         shP[tid][0] = px; shP[tid][1] = py; shP[tid][2] = pz;
         shW[tid] = sphere ? dW * (R)0.25 * area : norm;
+        shA[tid] = area;
     }
     __syncthreads();
     const R v0 = dir[lane][0], v1 = dir[lane][1], v2 = dir[lane][2];
@@ -346,7 +350,7 @@ k_rad_elems(const Scn<R>* __restrict__ S, int s, const phx_rad_elem* __restrict_
         r.tMx = crossing(px, fx, v0);
         r.tMy = crossing(py, fy, v1);
         r.tMz = crossing(pz, fz, v2);
-        r.w = kind[q] == 2 ? shW[q] : cosine(q) * dW * shW[q] * (R)els[e0 + q].area;
+        r.w = kind[q] == 2 ? shW[q] : cosine(q) * dW * shW[q] * shA[q];
         rays[at] = r;
         rayElem[at] = e0 + q;
         ++at;

@@ -168,17 +168,10 @@ class Solver:
         array), walls (phx_rad_wall records or an (m, 4) array), solid_t (N, K,
         or None for ambient). Returns (radAbs per element, radGas per cell or
         None); rad_last_ms() is the device time of its kernels."""
-        el, wl = _lib.rad_elements(elements), _lib.rad_walls(walls)
-        n = len(self.get("T"))
-        st = None if solid_t is None else np.ascontiguousarray(solid_t, np.float64)
-        if st is not None and st.size != n:
+        if solid_t is not None and np.size(solid_t) != self.L.phx_field_count(self.h, FIELD_ID["T"]):
             raise PhxError(_lib.PHX_ERR_INVALID, "solid_t needs one value per cell")
-        ab = np.zeros(len(el), np.float64)
-        g = np.zeros(n, np.float64) if gas else None
-        self._check(self.L.phx_rad_trace(self.h, el.ctypes.data if len(el) else None, len(el),
-                                         wl.ctypes.data if len(wl) else None, len(wl),
-                                         None if st is None else st.ctypes.data, ab.ctypes.data,
-                                         None if g is None else g.ctypes.data))
+        r, ab, g = _lib.rad_trace(self.L, self.h, 0, elements, walls, solid_t, gas)
+        self._check(r)
         return ab, g
 
     def rad_last_ms(self) -> float:
@@ -345,15 +338,10 @@ class Batch:
 
     def rad_trace(self, s: int, elements, walls, solid_t=None, gas: bool = True):
         """Solver.rad_trace for scenario s of the batch (phx_batch_rad_trace)."""
-        el, wl = _lib.rad_elements(elements), _lib.rad_walls(walls)
-        n = len(self.get(s, "T"))
-        st = None if solid_t is None else np.ascontiguousarray(solid_t, np.float64)
-        ab = np.zeros(len(el), np.float64)
-        g = np.zeros(n, np.float64) if gas else None
-        self._check(self.L.phx_batch_rad_trace(self.h, s, el.ctypes.data if len(el) else None, len(el),
-                                               wl.ctypes.data if len(wl) else None, len(wl),
-                                               None if st is None else st.ctypes.data, ab.ctypes.data,
-                                               None if g is None else g.ctypes.data))
+        r, ab, g = _lib.rad_trace(self.L, self.h, s, elements, walls, solid_t, gas)
+        if ab is None:
+            raise PhxError(r, "solid_t needs one value per cell")
+        self._check(r)
         return ab, g
 
     def vol_render(self, s: int, params, depth=None) -> np.ndarray:

@@ -60,3 +60,15 @@ def test_trace_at_the_edges_of_its_kernels(n_el, precision, tol):
     oab, ogain = oraclepy.rad_trace((c.nx, c.ny, c.nz), (c.dx, c.ox, c.oy, c.oz), c.blocked, gas, el, wl, solid)
     assert rel_l2(ab, oab) <= tol
     assert rel_l2(gain, ogain) <= tol
+
+
+@pytest.mark.parametrize("precision", [_lib.PREC_FP64, _lib.PREC_MIXED])
+def test_records_and_rows_are_the_same_elements(precision):
+    """Elements as an (n, 11) array and as phx_rad_elem records: the same bits."""
+    c, gas, el, wl, solid = scene(130, 7)
+    g = Solver(c, precision)
+    for f, a in gas.items():
+        g.set(f, a)
+    ab1, _ = g.rad_trace(el, wl, solid)
+    ab2, _ = g.rad_trace(_lib.rad_elements(el), _lib.rad_walls(wl), solid)
+    np.testing.assert_array_equal(ab1, ab2)
