@@ -867,6 +867,8 @@ public:
     struct VolWork {
         float4* vol = nullptr;
         size_t capVol = 0;
+        uint8_t* bricks = nullptr;
+        size_t capBricks = 0;
         float* depth = nullptr;
         float* rgb = nullptr;
         size_t capPix = 0;
@@ -874,6 +876,7 @@ public:
         double lastMs = 0;
         void release() {
             if (vol) cudaFree(vol);
+            if (bricks) cudaFree(bricks);
             if (depth) cudaFree(depth);
             if (rgb) cudaFree(rgb);
             if (e0) cudaEventDestroy(e0);
@@ -906,6 +909,11 @@ public:
             return PHX_OK;
         };
         PHX_TRY(alloc(volw.vol, volw.capVol, N, sizeof(float4)));
+        VolGrid G;
+        G.bx = (S.geo.nx + VOL_BRICK - 1) / VOL_BRICK;
+        G.by = (S.geo.ny + VOL_BRICK - 1) / VOL_BRICK;
+        const size_t nBricks = (size_t)G.bx * G.by * ((S.geo.nz + VOL_BRICK - 1) / VOL_BRICK);
+        PHX_TRY(alloc(volw.bricks, volw.capBricks, nBricks, 1));
         if (volw.capPix < npx || !volw.rgb) {
             size_t c1 = volw.capPix, c2 = volw.capPix;
             PHX_TRY(alloc(volw.rgb, c1, npx, 3 * sizeof(float)));
@@ -914,14 +922,15 @@ public:
         }
         if (!volw.e0) { PHX_CK(cudaEventCreate(&volw.e0)); PHX_CK(cudaEventCreate(&volw.e1)); }
         if (depth) PHX_CK(cudaMemcpyAsync(volw.depth, depth, npx * sizeof(float), cudaMemcpyHostToDevice, st));
-        VolGrid G;
         G.vol = volw.vol;
+        G.bricks = volw.bricks;
         G.nx = S.geo.nx; G.ny = S.geo.ny; G.nz = S.geo.nz;
         const float dxf = (float)S.geo.dx;
         G.bmin = v3((float)S.geo.ox, (float)S.geo.oy, (float)S.geo.oz);
         G.bmax = v3((float)S.geo.ox + G.nx * dxf, (float)S.geo.oy + G.ny * dxf, (float)S.geo.oz + G.nz * dxf);
         PHX_CK(cudaEventRecord(volw.e0, st));
-        k_vol_pack<R><<<(unsigned)((N + 255) / 256), 256, 0, st>>>(dS, s, volw.vol);
+        PHX_CK(cudaMemsetAsync(volw.bricks, 0, nBricks, st));
+        k_vol_pack<R><<<(unsigned)((N + 255) / 256), 256, 0, st>>>(dS, s, volw.vol, volw.bricks, G.bx, G.by, p->smoke_scale);
         dim3 grid((p->width + 15) / 16, (p->height + 7) / 8);
         k_vol_render<R><<<grid, 128, 0, st>>>(G, *p, depth ? volw.depth : nullptr, volw.rgb);
         PHX_CK(cudaGetLastError());
