@@ -142,6 +142,7 @@ struct Scenario {
         Z = computeZones(geo, Pb0);
         if (kMixed) coarseStop = vcycleStopFor(NN);   // the tuned schedule of the scenario's size, if any
         MG = buildMultigrid(geo, DENSE_MAX, coarseStop, coarseSolveFor());
+        buildRowSets();
         buildLeakFaces();
         return PHX_OK;
     }
@@ -204,7 +205,10 @@ struct Scenario {
         s.blocked = carve<uint8_t>(base, off, N);
         s.fx = carve<R>(base, off, NX); s.fy = carve<R>(base, off, NY); s.fz = carve<R>(base, off, NZ);
         s.ax = carve<R>(base, off, NX); s.ay = carve<R>(base, off, NY); s.az = carve<R>(base, off, NZ);
-        s.a0x = carve<R>(base, off, NX); s.a0y = carve<R>(base, off, NY); s.a0z = carve<R>(base, off, NZ);
+        // the same arrays where no wind-inflow boundary face is closed
+        s.a0x = MG.a0x == geo.ax ? s.ax : carve<R>(base, off, NX);
+        s.a0y = MG.a0y == geo.ay ? s.ay : carve<R>(base, off, NY);
+        s.a0z = MG.a0z == geo.az ? s.az : carve<R>(base, off, NZ);
         s.lx = geo.anyLeak ? carve<uint8_t>(base, off, NX) : nullptr;
         s.ly = geo.anyLeak ? carve<uint8_t>(base, off, NY) : nullptr;
         s.lz = geo.anyLeak ? carve<uint8_t>(base, off, NZ) : nullptr;
@@ -235,10 +239,11 @@ struct Scenario {
         s.Pb = carve<R>(base, off, N); s.Q = carve<R>(base, off, N); s.Qr = carve<R>(base, off, N);
         s.hrr = carve<R>(base, off, N); s.massSrc = carve<R>(base, off, N);
         s.lit = carve<uint8_t>(base, off, N); s.lit2 = carve<uint8_t>(base, off, N); s.pilot = carve<uint8_t>(base, off, N);
-        for (int q = 0; q < 9; ++q) s.tmp[q] = carve<R>(base, off, N);
+        for (int q = 0; q < 7; ++q) s.tmp[q] = carve<R>(base, off, N);
         s.rho = kMixed ? nullptr : carve<R>(base, off, N);
         s.b = carve<R>(base, off, N); s.r = carve<R>(base, off, N); s.z = carve<R>(base, off, N);
         s.d = carve<R>(base, off, N); s.q = carve<R>(base, off, N);
+        s.tmp[7] = s.d; s.tmp[8] = s.q;   // a solve's first iteration writes both before it reads them
         s.p64 = kMixed ? carve<double>(base, off, N) : nullptr;
         s.p64prev = kMixed ? carve<double>(base, off, N) : nullptr;
         Level<R>& L0 = s.lv[0];
@@ -275,6 +280,73 @@ struct Scenario {
     // the levels' arrays in their own arena: level 0's aggregation map, and per
     // coarser level its CSR rows, diagonal, iterate and scratch, child lists and,
     // at the coarsest level, the dense operator
+    // A level's rows in sets of 32, each word of a set's rows side by side, so that a warp
+    // reads a coupling of its rows in one access: the rows in their order for the sweeps,
+    // and for the restriction eight lanes per unknown of the next level, a lane per child.
+    // A set holds diag[32] (FP64 sweeps: omega / diag), val[width][32], own[32] (sweeps:
+    // the row's aggregate; restriction: the row, -1 none), col[width][32] and, for the
+    // sweeps, next[width][32], the columns' aggregates. Short rows end in couplings of 0 to
+    // the row itself. Sets with a row of more than ROW_WIDEST couplings or an unknown of
+    // more than eight children are left out.
+    struct RowSets {
+        size_t words = 0, nJ = 0, nR = 0;
+        bool allJ = true, allR = true;   // no set is left out
+        std::vector<unsigned> data;      // dropped once uploaded
+        std::vector<RowSet> j, r;
+    };
+    std::vector<RowSets> rowSets;
+    void buildRowSets() {
+        constexpr int RW = (int)sizeof(R) / 4;
+        rowSets.assign(MG.lv.size(), RowSets());
+        for (size_t l = 1; l + 1 < MG.lv.size(); ++l) {
+            const MgLevel& L = MG.lv[l];
+            RowSets& out = rowSets[l];
+            auto add = [&](const int* own, bool sweep) {   // own[32]: rows, -1 none
+                RowSet s{-1, 0};
+                for (int q = 0; q < 32; ++q)
+                    if (own[q] >= 0) s.width = std::max(s.width, L.rowStart[own[q] + 1] - L.rowStart[own[q]]);
+                if (s.width > ROW_WIDEST) return s;
+                s.off = (int)out.data.size();
+                out.data.resize(out.data.size() + 32 * (size_t)((1 + s.width) * RW + 1 + s.width * (sweep ? 2 : 1)));
+                unsigned* w = out.data.data() + s.off;
+                auto real = [&](int at, double v) { const R x = (R)v; std::memcpy(w + at * RW, &x, sizeof(R)); };
+                unsigned* own1 = w + 32 * (1 + s.width) * RW;
+                for (int q = 0; q < 32; ++q) {
+                    const int I = own[q], q0 = I >= 0 ? L.rowStart[I] : 0, n = I >= 0 ? L.rowStart[I + 1] - q0 : 0;
+                    real(q, I < 0 ? 0.0 : sweep && RW == 2 ? (L.diag[I] > 0 ? OMEGA / L.diag[I] : 0.0) : L.diag[I]);
+                    own1[q] = (unsigned)(I < 0 ? -1 : sweep ? L.agg[I] : I);
+                    for (int e = 0; e < s.width; ++e) {
+                        const int col = e < n ? L.col[q0 + e] : std::max(I, 0);
+                        real(32 * (1 + e) + q, e < n ? L.val[q0 + e] : 0.0);
+                        own1[32 * (1 + e) + q] = (unsigned)col;
+                        if (sweep) own1[32 * (1 + s.width + e) + q] = (unsigned)L.agg[col];
+                    }
+                }
+                return s;
+            };
+            int own[32];
+            for (int i = 0; i < L.n; i += 32) {
+                for (int q = 0; q < 32; ++q) own[q] = i + q < L.n ? i + q : -1;
+                out.j.push_back(add(own, true));
+            }
+            const int nC = MG.lv[l + 1].n;
+            for (int J0 = 0; J0 < nC; J0 += 4) {
+                bool few = true;
+                for (int q = 0; q < 32; ++q) {
+                    const int J = J0 + q / 8, n = J < nC ? L.childStart[J + 1] - L.childStart[J] : 0;
+                    few &= n <= 8;
+                    own[q] = q % 8 < n ? L.child[L.childStart[J] + q % 8] : -1;
+                }
+                out.r.push_back(few ? add(own, false) : RowSet{-1, 0});
+            }
+            for (const RowSet& s : out.j) out.allJ &= s.off >= 0;
+            for (const RowSet& s : out.r) out.allR &= s.off >= 0;
+            out.words = out.data.size();
+            out.nJ = out.j.size();
+            out.nR = out.r.size();
+        }
+    }
+
     size_t layoutLevels(char* base) {
         const int nl = (int)MG.lv.size();
         size_t off = 0;
@@ -284,19 +356,25 @@ struct Scenario {
             const MgLevel& L = MG.lv[l];
             Level<R>& D = s.lv[l];
             D.n = L.n;
+            // the arrays that rows without a set, and a serial solve of the coarsest level, read
+            const bool last = l == nl - 1, sets = rowSets[l].allJ && rowSets[l].allR;
+            const bool csr = l > 0 && (last ? L.dense.empty() : !sets);
             if (l > 0) {
-                D.rowStart = carve<int>(base, off, L.rowStart.size());
-                D.col = carve<int>(base, off, L.col.size() + 1);
-                D.val = carve<R>(base, off, L.val.size() + 1);
+                D.rowStart = csr ? carve<int>(base, off, L.rowStart.size()) : nullptr;
+                D.col = csr ? carve<int>(base, off, L.col.size() + 1) : nullptr;
+                D.val = csr ? carve<R>(base, off, L.val.size() + 1) : nullptr;
                 D.diag = carve<R>(base, off, L.n + 1);
                 D.omd = carve<R>(base, off, L.n + 1);
                 D.x = carve<R>(base, off, l == 1 || l == nl - 1 ? L.n + 1 : 1);
                 for (unsigned long long** v : {&D.b, &D.yd, &D.xd, &D.yu, &D.xu})
-                    *v = carve<unsigned long long>(base, off, TAG_WORDS<R> * (size_t)(L.n + 1));
+                    *v = carve<unsigned long long>(base, off, TAG_WORDS<R> * (v == &D.xu && l == 1 ? 1 : (size_t)(L.n + 1)));
             }
-            D.agg = L.agg.empty() ? nullptr : carve<int>(base, off, L.agg.size());
-            D.childStart = (l == 0 || L.childStart.empty()) ? nullptr : carve<int>(base, off, L.childStart.size());
-            D.child = (l == 0 || L.child.empty()) ? nullptr : carve<int>(base, off, L.child.size() + 1);
+            D.agg = L.agg.empty() || (l > 0 && !csr) ? nullptr : carve<int>(base, off, L.agg.size());
+            D.childStart = (l == 0 || !csr || L.childStart.empty()) ? nullptr : carve<int>(base, off, L.childStart.size());
+            D.child = (l == 0 || !csr || L.child.empty()) ? nullptr : carve<int>(base, off, L.child.size() + 1);
+            D.rows = carve<unsigned>(base, off, rowSets[l].words + 1);
+            D.setsJ = carve<RowSet>(base, off, rowSets[l].nJ + 1);
+            D.setsR = carve<RowSet>(base, off, rowSets[l].nR + 1);
             D.dense = L.dense.empty() ? nullptr : carve<R>(base, off, L.dense.size());
         }
         return off + 256;
@@ -332,6 +410,7 @@ struct Scenario {
         char* old = mgArena;
         MG = std::move(M);
         coarseStop = stop;
+        buildRowSets();
         mgBytes = layoutLevels(nullptr);
         char* fresh = nullptr;
         if (cudaMalloc(&fresh, mgBytes) != cudaSuccess) {
@@ -398,7 +477,9 @@ struct Scenario {
         PHX_TRY(putRaw(st, s.blocked, geo.blocked.data(), N));
         PHX_TRY(put(st, s.fx, geo.fx)); PHX_TRY(put(st, s.fy, geo.fy)); PHX_TRY(put(st, s.fz, geo.fz));
         PHX_TRY(put(st, s.ax, geo.ax)); PHX_TRY(put(st, s.ay, geo.ay)); PHX_TRY(put(st, s.az, geo.az));
-        PHX_TRY(put(st, s.a0x, MG.a0x)); PHX_TRY(put(st, s.a0y, MG.a0y)); PHX_TRY(put(st, s.a0z, MG.a0z));
+        if (s.a0x != s.ax) PHX_TRY(put(st, s.a0x, MG.a0x));
+        if (s.a0y != s.ay) PHX_TRY(put(st, s.a0y, MG.a0y));
+        if (s.a0z != s.az) PHX_TRY(put(st, s.a0z, MG.a0z));
         PHX_TRY(put(st, s.diag, MG.lv[0].diag));
         {
             const std::vector<unsigned char> cd = levelZeroCodes();
@@ -435,9 +516,11 @@ struct Scenario {
         for (int l = 1; l < (int)MG.lv.size(); ++l) {
             const MgLevel& L = MG.lv[l];
             Level<R>& D = s.lv[l];
-            PHX_TRY(putRaw(st, D.rowStart, L.rowStart.data(), L.rowStart.size()));
-            PHX_TRY(putRaw(st, D.col, L.col.data(), L.col.size()));
-            PHX_TRY(put(st, D.val, L.val));
+            if (D.rowStart) {
+                PHX_TRY(putRaw(st, D.rowStart, L.rowStart.data(), L.rowStart.size()));
+                PHX_TRY(putRaw(st, D.col, L.col.data(), L.col.size()));
+                PHX_TRY(put(st, D.val, L.val));
+            }
             PHX_TRY(put(st, D.diag, L.diag));
             std::vector<double> omd(L.n);
             for (int I = 0; I < L.n; ++I) omd[I] = L.diag[I] > 0 ? OMEGA / L.diag[I] : 0.0;
@@ -450,7 +533,11 @@ struct Scenario {
             if (D.childStart) PHX_TRY(putRaw(st, D.childStart, L.childStart.data(), L.childStart.size()));
             if (D.child) PHX_TRY(putRaw(st, D.child, L.child.data(), L.child.size()));
             if (D.dense) PHX_TRY(put(st, D.dense, L.dense));
+            PHX_TRY(putRaw(st, D.rows, rowSets[l].data.data(), rowSets[l].words));
+            PHX_TRY(putRaw(st, D.setsJ, rowSets[l].j.data(), rowSets[l].nJ));
+            PHX_TRY(putRaw(st, D.setsR, rowSets[l].r.data(), rowSets[l].nR));
         }
+        for (RowSets& r : rowSets) { r.data = {}; r.j = {}; r.r = {}; }
         return PHX_OK;
     }
 

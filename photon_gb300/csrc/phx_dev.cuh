@@ -134,6 +134,13 @@ __host__ __device__ __forceinline__ unsigned divS(unsigned x, const DivS& v) {
     return (unsigned)(((unsigned long long)x * v.m) >> v.s);
 }
 
+// 32 rows of a coarse level side by side (solve.cuh)
+constexpr int ROW_WIDEST = 24;   // couplings of a row that is kept so
+struct RowSet {
+    int off;                 // of its words; -1: none
+    int width;               // couplings of the longest row
+};
+
 template <class R>
 struct Level {
     int n;                       // unknowns
@@ -143,6 +150,8 @@ struct Level {
     const R* omd;                // omega / diag (0 without a diagonal): the damped Jacobi factor
     const int* agg;              // unknown -> unknown of the next coarser level (nullptr at the coarsest)
     const int *childStart, *child;   // next coarser unknown -> its unknowns here, ascending
+    const unsigned* rows;        // sets of 32 rows: setsJ in the level's order, setsR by the next level's unknowns
+    const RowSet *setsJ, *setsR;
     R* x;                        // level 1: the V-cycle's correction; coarsest: scratch of its serial solve
     // the V-cycle's values of the level, each with the cycle's tag (solve.cuh): right-hand
     // side, first and second iterate on the way down, first and last on the way up

@@ -49,7 +49,10 @@ struct SolveCfg {
     // threads per CTA. FP64 takes 128 registers a thread. FP32 trades registers for warps in
     // flight: house step 1.25 / 1.27 / 1.31 ms at 768 / 896 / 1024 threads, 24 scenarios 6.25 / 5.98 / 5.93
     static constexpr int T = sizeof(R) == 8 ? 512 : 896;
-    static constexpr int ROWS = 98304;                     // shared memory for the coarse rows, bytes
+    // shared memory for the coarse rows, bytes: what it takes is missing to L1. FP32 house
+    // step 1.217 / 1.222 / 1.238 / 1.254 ms at 32 / 64 / 96 / 128 KiB, 1.3e6 cells 3.69 / 3.61 /
+    // 3.58 / 3.56; FP64 house 2.796 / 2.756 / 2.755 / 2.762
+    static constexpr int ROWS = sizeof(R) == 8 ? 98304 : 65536;
     // dynamic shared memory: coarse rows, then by turns the FP32 dot products' terms and
     // the coarsest level's right-hand side
     static constexpr int TERMS = sizeof(R) == 8 ? 0 : 4 * T * 8, DENSE_B = DENSE_MAX * (int)sizeof(R);
@@ -616,17 +619,15 @@ __device__ __forceinline__ void ctaMaxStore(double* dst, V v, V* sh) {
 
 constexpr int RRJ_LANES = 8;   // lanes per unknown of a restriction
 
-// ---- coarse rows in shared memory ---------------------------------------------
-// A warp's rows of a coarse level are the same in every V-cycle, so their
-// couplings are kept in the CTA's shared memory, transposed over the lanes: a
-// sweep then waits for one memory latency (its neighbours' values) instead of
-// three (row start, column, value). Rows that do not fit the pool, or have more
-// than ROW_WIDEST couplings, are read from the level's arrays every time.
-constexpr int ROW_WIDEST = 24, ROW_CHUNKS = 2;
-struct RowSet {
-    int off;                 // words from the pool's start; -1: not kept
-    int width;               // couplings of the longest row
-};
+// ---- coarse rows ----------------------------------------------------------------
+// A coarse level's rows lie in sets of 32, transposed over a warp's lanes (Level::rows):
+// a coupling of 32 rows is one access. The sets of a warp's first ROW_CHUNKS groups are
+// copied to the CTA's shared memory as far as the pool goes, since they are the same in
+// every V-cycle: a sweep then waits for one memory latency (its neighbours' values); other
+// sets are read from the level each time. Rows without a set take the level's arrays.
+// Against rows read one by one (a lane's own row start, columns and values): house step in
+// FP32 1.26 -> 1.21 ms, 1.3e6 cells 3.64 -> 3.57, 24 scenarios 6.07 -> 5.99.
+constexpr int ROW_CHUNKS = 2;
 template <class R>
 struct RowView {
     const R* diag;           // [32]: the diagonal; FP64 sweeps (toNext): omega / diagonal
@@ -643,46 +644,32 @@ __device__ __forceinline__ RowView<R> rowView(const unsigned* pool, const RowSet
     v.next = v.col + 32 * s.width;
     return v;
 }
-// keep row I of level l in lane's column of a new set (I < 0: none): diagonal, the
-// row's aggregate (toNext) or the row itself, couplings, their columns and
-// (toNext) their aggregates. Short rows end in couplings of 0 to the row itself.
+// a warp's set copied to the pool where it fits, for the whole solve: its place there, in
+// the level (~off, below 0 and above -1), or none (width -1)
 template <class R>
-__device__ __forceinline__ void keepRows(const Level<R>& L, int I, bool toNext, unsigned* pool, int* used, int words,
-                                         RowSet* out) {
+__device__ __forceinline__ RowSet keepRows(const unsigned* rows, RowSet s, bool sweep, unsigned* pool, int* used, int words) {
     const int lane = (int)(threadIdx.x & 31);
-    const int q0 = I >= 0 ? L.rowStart[I] : 0, n = I >= 0 ? L.rowStart[I + 1] - q0 : 0;
-    RowSet s;
-    s.width = __reduce_max_sync(0xffffffffu, n);
+    if (s.off < 0) return RowSet{-1, -1};
     constexpr int RW = (int)sizeof(R) / 4;
-    const int need = 32 * ((1 + s.width) * RW + 1 + s.width * (toNext ? 2 : 1));
-    int off = -1;
-    if (lane == 0 && s.width <= ROW_WIDEST) {
-        off = atomicAdd(used, need);
-        if (off + need > words) off = -1;
-    }
-    s.off = __shfl_sync(0xffffffffu, off, 0);
-    if (s.off >= 0) {
-        const RowView<R> v = rowView<R>(pool, s);
-        const_cast<R*>(v.diag)[lane] = I < 0 ? R(0) : toNext && sizeof(R) == 8 ? L.omd[I] : L.diag[I];
-        const_cast<int*>(v.own)[lane] = I < 0 ? -1 : toNext ? L.agg[I] : I;
-        for (int e = 0; e < s.width; ++e) {
-            const int col = e < n ? L.col[q0 + e] : max(I, 0);
-            const_cast<R*>(v.val)[32 * e + lane] = e < n ? L.val[q0 + e] : R(0);
-            const_cast<int*>(v.col)[32 * e + lane] = col;
-            if (toNext) const_cast<int*>(v.next)[32 * e + lane] = L.agg[col];
-        }
-    }
-    if (lane == 0) *out = s;
+    const int need = 32 * ((1 + s.width) * RW + 1 + s.width * (sweep ? 2 : 1));
+    int off = 0;
+    if (lane == 0) off = atomicAdd(used, need);
+    off = __shfl_sync(0xffffffffu, off, 0);
+    if (off + need > words) return RowSet{~s.off, s.width};
+    const uint4* from = reinterpret_cast<const uint4*>(rows + s.off);
+    uint4* to = reinterpret_cast<uint4*>(pool + off);
+    for (int i = lane; i < need / 4; i += 32) to[i] = from[i];
+    return RowSet{off, s.width};
 }
-// The couplings of a level's row: kept in shared memory, or the level's arrays
-template <class R>
-struct KeptRow {
+// The couplings of a level's row: of a set in shared memory (FAR: in the level), or the level's arrays
+template <class R, bool IN_LEVEL>
+struct SetRow {
     RowView<R> v;
     int n, lane;
     __device__ __forceinline__ int col(int e) const { return v.col[32 * e + lane]; }
     __device__ __forceinline__ int next(int e, int) const { return v.next[32 * e + lane]; }
     __device__ __forceinline__ R val(int e) const { return v.val[32 * e + lane]; }
-    static constexpr bool FAR = false;
+    static constexpr bool FAR = IN_LEVEL && sizeof(R) == 4;
 };
 template <class R>
 struct StoredRow {
@@ -784,12 +771,16 @@ __device__ __forceinline__ void restrictRows(const Scn<R>& g, int l, int jBase, 
             if ((valid >> (lane0 + q)) & 1u) acc = acc + rq;
         }
     };
-    if (rs.off >= 0) {
-        const RowView<R> v = rowView<R>(pool, rs);
+    auto fromSet = [&](const RowView<R>& v, auto inLevel) {
         const int I = v.own[lane];
         T s = T(0);
-        if (I >= 0) s = residual(I, v.diag[lane], KeptRow<R>{v, rs.width, lane});
+        if (I >= 0) s = residual(I, v.diag[lane], SetRow<R, decltype(inLevel)::value>{v, rs.width, lane});
         addChildren(s, I >= 0);
+    };
+    if (rs.off >= 0) {
+        fromSet(rowView<R>(pool, rs), std::false_type{});
+    } else if (rs.width >= 0) {
+        fromSet(rowView<R>(L.rows, RowSet{~rs.off, rs.width}), std::true_type{});
     } else {
         const int e0 = J < C.n ? L.childStart[J] : 0, nch = J < C.n ? L.childStart[J + 1] - e0 : 0;
         const int chunks = __reduce_max_sync(0xffffffffu, (nch + RRJ_LANES - 1) / RRJ_LANES);
@@ -1000,31 +991,34 @@ k_solve(const Scn<R>* __restrict__ S, SolveArgs a) {
             for (int m = 0; m < ROW_CHUNKS; ++m) {
                 const Level<R>& L = g.lv[l];
                 const Level<R>& C = g.lv[l + 1];
-                const int chunk = gw + m * nw, I = chunk * 32 + lane;
-                if (lane == 0) rowsJ[l][warp][m].off = rowsR[l][warp][m].off = -1;
-                __syncwarp();
-                if (chunk * 32 < L.n)
-                    keepRows(L, I < L.n ? I : -1, true, pool, &poolUsed, SolveCfg<R>::ROWS / 4, &rowsJ[l][warp][m]);
-                if (chunk * (32 / RRJ_LANES) < C.n) {
-                    const int J = chunk * (32 / RRJ_LANES) + lane / RRJ_LANES, c = lane % RRJ_LANES;
-                    const int e0 = J < C.n ? L.childStart[J] : 0, nch = J < C.n ? L.childStart[J + 1] - e0 : 0;
-                    if (__reduce_max_sync(0xffffffffu, nch) <= RRJ_LANES)
-                        keepRows(L, c < nch ? L.child[e0 + c] : -1, false, pool, &poolUsed, SolveCfg<R>::ROWS / 4,
-                                 &rowsR[l][warp][m]);
+                const int chunk = gw + m * nw;
+                RowSet j{-1, -1}, r{-1, -1};
+                if (chunk * 32 < L.n) j = keepRows<R>(L.rows, L.setsJ[chunk], true, pool, &poolUsed, SolveCfg<R>::ROWS / 4);
+                if (chunk * (32 / RRJ_LANES) < C.n)
+                    r = keepRows<R>(L.rows, L.setsR[chunk], false, pool, &poolUsed, SolveCfg<R>::ROWS / 4);
+                if (lane == 0) {
+                    rowsJ[l][warp][m] = j;
+                    rowsR[l][warp][m] = r;
                 }
                 __syncwarp();
             }
         const TagWait tw{&gaveUp, g.errWord};
+        auto inLevel = [](RowSet s) { return s.off >= 0 ? RowSet{~s.off, s.width} : RowSet{-1, -1}; };
         auto jacobiLevel = [&](auto sweep, int l) {
             constexpr int SWEEP = decltype(sweep)::value;
             const Level<R>& L = g.lv[l];
             for (int m = 0, i = gw * 32; i < L.n; ++m, i += nw * 32) {
-                const RowSet rs = m < ROW_CHUNKS ? rowsJ[l][warp][m] : RowSet{-1, 0};
+                const RowSet rs = m < ROW_CHUNKS ? rowsJ[l][warp][m] : inLevel(L.setsJ[i / 32]);
                 const int I = i + lane;
                 if (I >= L.n) continue;
+                auto fromSet = [&](const RowView<R>& v, auto far) {
+                    jacobiRow<R, SWEEP>(g, l, I, SetRow<R, decltype(far)::value>{v, rs.width, lane}, v.own[lane], v.diag[lane],
+                                        v.diag[lane], B.tag, tw);
+                };
                 if (rs.off >= 0) {
-                    const RowView<R> v = rowView<R>(pool, rs);
-                    jacobiRow<R, SWEEP>(g, l, I, KeptRow<R>{v, rs.width, lane}, v.own[lane], v.diag[lane], v.diag[lane], B.tag, tw);
+                    fromSet(rowView<R>(pool, rs), std::false_type{});
+                } else if (rs.width >= 0) {
+                    fromSet(rowView<R>(L.rows, RowSet{~rs.off, rs.width}), std::true_type{});
                 } else {
                     const int q0 = L.rowStart[I];
                     jacobiRow<R, SWEEP>(g, l, I, StoredRow<R>{L, q0, L.rowStart[I + 1] - q0}, L.agg[I], L.diag[I], L.omd[I], B.tag, tw);
@@ -1034,7 +1028,7 @@ k_solve(const Scn<R>* __restrict__ S, SolveArgs a) {
         auto restrictLevel = [&](int l) {
             constexpr int PER = 32 / RRJ_LANES;
             for (int m = 0, j = gw * PER; j < g.lv[l + 1].n; ++m, j += nw * PER)
-                restrictRows(g, l, j, pool, m < ROW_CHUNKS ? rowsR[l][warp][m] : RowSet{-1, 0}, B.tag, tw);
+                restrictRows(g, l, j, pool, m < ROW_CHUNKS ? rowsR[l][warp][m] : inLevel(g.lv[l].setsR[j / PER]), B.tag, tw);
         };
         auto coarsest = [&]() {
             const Level<R>& L = g.lv[nl - 1];
