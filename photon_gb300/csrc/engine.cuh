@@ -291,59 +291,64 @@ struct Scenario {
     struct RowSets {
         size_t words = 0, nJ = 0, nR = 0;
         bool allJ = true, allR = true;   // no set is left out
-        std::vector<unsigned> data;      // dropped once uploaded
+        std::unique_ptr<unsigned[]> data;   // dropped once uploaded
         std::vector<RowSet> j, r;
     };
     std::vector<RowSets> rowSets;
     void buildRowSets() {
         constexpr int RW = (int)sizeof(R) / 4;
-        rowSets.assign(MG.lv.size(), RowSets());
+        rowSets = std::vector<RowSets>(MG.lv.size());
         for (size_t l = 1; l + 1 < MG.lv.size(); ++l) {
             const MgLevel& L = MG.lv[l];
-            RowSets& out = rowSets[l];
-            auto add = [&](const int* own, bool sweep) {   // own[32]: rows, -1 none
-                RowSet s{-1, 0};
-                for (int q = 0; q < 32; ++q)
-                    if (own[q] >= 0) s.width = std::max(s.width, L.rowStart[own[q] + 1] - L.rowStart[own[q]]);
-                if (s.width > ROW_WIDEST) return s;
-                s.off = (int)out.data.size();
-                out.data.resize(out.data.size() + 32 * (size_t)((1 + s.width) * RW + 1 + s.width * (sweep ? 2 : 1)));
-                unsigned* w = out.data.data() + s.off;
-                auto real = [&](int at, double v) { const R x = (R)v; std::memcpy(w + at * RW, &x, sizeof(R)); };
-                unsigned* own1 = w + 32 * (1 + s.width) * RW;
-                for (int q = 0; q < 32; ++q) {
-                    const int I = own[q], q0 = I >= 0 ? L.rowStart[I] : 0, n = I >= 0 ? L.rowStart[I + 1] - q0 : 0;
-                    real(q, I < 0 ? 0.0 : sweep && RW == 2 ? (L.diag[I] > 0 ? OMEGA / L.diag[I] : 0.0) : L.diag[I]);
-                    own1[q] = (unsigned)(I < 0 ? -1 : sweep ? L.agg[I] : I);
-                    for (int e = 0; e < s.width; ++e) {
-                        const int col = e < n ? L.col[q0 + e] : std::max(I, 0);
-                        real(32 * (1 + e) + q, e < n ? L.val[q0 + e] : 0.0);
-                        own1[32 * (1 + e) + q] = (unsigned)col;
-                        if (sweep) own1[32 * (1 + s.width + e) + q] = (unsigned)L.agg[col];
-                    }
-                }
-                return s;
-            };
-            int own[32];
-            for (int i = 0; i < L.n; i += 32) {
-                for (int q = 0; q < 32; ++q) own[q] = i + q < L.n ? i + q : -1;
-                out.j.push_back(add(own, true));
-            }
             const int nC = MG.lv[l + 1].n;
-            for (int J0 = 0; J0 < nC; J0 += 4) {
-                bool few = true;
-                for (int q = 0; q < 32; ++q) {
-                    const int J = J0 + q / 8, n = J < nC ? L.childStart[J + 1] - L.childStart[J] : 0;
-                    few &= n <= 8;
-                    own[q] = q % 8 < n ? L.child[L.childStart[J] + q % 8] : -1;
-                }
-                out.r.push_back(few ? add(own, false) : RowSet{-1, 0});
+            RowSets& out = rowSets[l];
+            out.nJ = (size_t)(L.n + 31) / 32;
+            out.nR = (size_t)(nC + 3) / 4;
+            out.j.resize(out.nJ);
+            out.r.resize(out.nR);
+            // widths and places first, so that the words are written once
+            auto place = [&](RowSet& s, int width, bool sweep) {
+                s.width = width;
+                s.off = width > ROW_WIDEST ? -1 : (int)out.words;
+                if (s.off >= 0) out.words += 32 * (size_t)((1 + width) * RW + 1 + width * (sweep ? 2 : 1));
+                (sweep ? out.allJ : out.allR) &= s.off >= 0;
+            };
+            auto length = [&](int I) { return L.rowStart[I + 1] - L.rowStart[I]; };
+            for (size_t c = 0; c < out.nJ; ++c) {
+                int width = 0;
+                for (int I = 32 * (int)c; I < std::min(32 * (int)c + 32, L.n); ++I) width = std::max(width, length(I));
+                place(out.j[c], width, true);
             }
-            for (const RowSet& s : out.j) out.allJ &= s.off >= 0;
-            for (const RowSet& s : out.r) out.allR &= s.off >= 0;
-            out.words = out.data.size();
-            out.nJ = out.j.size();
-            out.nR = out.r.size();
+            for (size_t c = 0; c < out.nR; ++c) {
+                int width = 0;
+                for (int J = 4 * (int)c; J < std::min(4 * (int)c + 4, nC); ++J) {
+                    if (L.childStart[J + 1] - L.childStart[J] > 8) width = ROW_WIDEST + 1;
+                    for (int q = L.childStart[J]; q < L.childStart[J + 1]; ++q) width = std::max(width, length(L.child[q]));
+                }
+                place(out.r[c], width, false);
+            }
+            out.data.reset(new unsigned[out.words + 1]);
+            auto fill = [&](const RowSet& s, int q, int I, bool sweep) {   // lane q's row I, -1 none
+                unsigned* const w = out.data.get() + s.off;
+                R* const val = reinterpret_cast<R*>(w);
+                unsigned* const own = w + 32 * (1 + s.width) * RW;
+                const int q0 = I >= 0 ? L.rowStart[I] : 0, n = I >= 0 ? length(I) : 0;
+                val[q] = (R)(I < 0 ? 0.0 : sweep && RW == 2 ? (L.diag[I] > 0 ? OMEGA / L.diag[I] : 0.0) : L.diag[I]);
+                own[q] = (unsigned)(I < 0 ? -1 : sweep ? L.agg[I] : I);
+                for (int e = 0; e < s.width; ++e) {
+                    const int col = e < n ? L.col[q0 + e] : std::max(I, 0);
+                    val[32 * (1 + e) + q] = (R)(e < n ? L.val[q0 + e] : 0.0);
+                    own[32 * (1 + e) + q] = (unsigned)col;
+                    if (sweep) own[32 * (1 + s.width + e) + q] = (unsigned)L.agg[col];
+                }
+            };
+            for (size_t c = 0; c < out.nJ; ++c)
+                for (int q = 0; q < 32 && out.j[c].off >= 0; ++q) fill(out.j[c], q, 32 * (int)c + q < L.n ? 32 * (int)c + q : -1, true);
+            for (size_t c = 0; c < out.nR; ++c)
+                for (int q = 0; q < 32 && out.r[c].off >= 0; ++q) {
+                    const int J = 4 * (int)c + q / 8, n = J < nC ? L.childStart[J + 1] - L.childStart[J] : 0;
+                    fill(out.r[c], q, q % 8 < n ? L.child[L.childStart[J] + q % 8] : -1, false);
+                }
         }
     }
 
@@ -533,11 +538,11 @@ struct Scenario {
             if (D.childStart) PHX_TRY(putRaw(st, D.childStart, L.childStart.data(), L.childStart.size()));
             if (D.child) PHX_TRY(putRaw(st, D.child, L.child.data(), L.child.size()));
             if (D.dense) PHX_TRY(put(st, D.dense, L.dense));
-            PHX_TRY(putRaw(st, D.rows, rowSets[l].data.data(), rowSets[l].words));
+            PHX_TRY(putRaw(st, D.rows, rowSets[l].data.get(), rowSets[l].words));
             PHX_TRY(putRaw(st, D.setsJ, rowSets[l].j.data(), rowSets[l].nJ));
             PHX_TRY(putRaw(st, D.setsR, rowSets[l].r.data(), rowSets[l].nR));
         }
-        for (RowSets& r : rowSets) { r.data = {}; r.j = {}; r.r = {}; }
+        for (RowSets& r : rowSets) { r.data.reset(); r.j = {}; r.r = {}; }
         return PHX_OK;
     }
 
@@ -614,6 +619,7 @@ public:
     double* dTimes = nullptr;    // simulated time of each scenario (read-back staging)
     double* dMaxPart = nullptr;  // k_solve: two maxima per CTA
     int solveGrid = 0;           // k_solve: CTAs resident at once
+    int solvePer = 1;            // ... per SM
     bool smoothOne = false;            // mixed path: one Jacobi sweep per coarse level and leg (vcycleSweeps)
     double* hPin = nullptr;      // pinned scratch for read-backs
     Dom dom[D_COUNT];
@@ -1142,13 +1148,20 @@ public:
     // another. PHX_PERSIST_CTAS caps it (tests: several scenarios per CTA)
     static constexpr int MAX_SOLVE_CTAS = 1024;
     int setupSolve() {
-        int dev = 0, sms = 0, occ = 0;
+        int dev = 0, sms = 0, occ[2] = {0, 0};
         PHX_CK(cudaGetDevice(&dev));
         PHX_CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-        PHX_CK(cudaFuncSetAttribute(k_solve<R>, cudaFuncAttributeMaxDynamicSharedMemorySize, SolveCfg<R>::SMEM));
-        PHX_CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_solve<R>, SolveCfg<R>::T, SolveCfg<R>::SMEM));
-        if (occ < 1) { err = "the solve kernel does not fit an SM"; return PHX_ERR_CUDA; }
-        solveGrid = std::min(sms * occ, MAX_SOLVE_CTAS);
+        auto fit = [&](auto per) -> cudaError_t {
+            constexpr int PER = decltype(per)::value;
+            using Cfg = SolveCfg<R, PER>;
+            const cudaError_t e = cudaFuncSetAttribute(k_solve<R, PER>, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::SMEM);
+            return e != cudaSuccess ? e : cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ[PER - 1], k_solve<R, PER>, Cfg::T, Cfg::SMEM);
+        };
+        PHX_CK(fit(std::integral_constant<int, 1>{}));
+        if constexpr (kMixed) PHX_CK(fit(std::integral_constant<int, 2>{}));
+        if (occ[0] < 1) { err = "the solve kernel does not fit an SM"; return PHX_ERR_CUDA; }
+        solvePer = occ[1] >= 2 ? solvePerSm<R>(nscn(), sms) : 1;
+        solveGrid = std::min(sms * (solvePer == 2 ? 2 : occ[0]), MAX_SOLVE_CTAS);
         if (const char* c = std::getenv("PHX_PERSIST_CTAS")) solveGrid = std::max(1, std::min(solveGrid, std::atoi(c)));
         return PHX_OK;
     }
@@ -1361,8 +1374,10 @@ public:
         a.maxPart = dMaxPart;
         cudaLaunchConfig_t cfg = {};
         cfg.gridDim = dim3((unsigned)solveGrid);
-        cfg.blockDim = dim3(SolveCfg<R>::T);
-        cfg.dynamicSmemBytes = SolveCfg<R>::SMEM;
+        constexpr int PER2 = kMixed ? 2 : 1;
+        const bool two = solvePer == 2;
+        cfg.blockDim = dim3(two ? SolveCfg<R, PER2>::T : SolveCfg<R, 1>::T);
+        cfg.dynamicSmemBytes = two ? SolveCfg<R, PER2>::SMEM : SolveCfg<R, 1>::SMEM;
         cfg.stream = st;
         cudaLaunchAttribute at;
         at.id = cudaLaunchAttributeCooperative;
@@ -1379,7 +1394,7 @@ public:
             evNext += 2;
             cudaEventRecord(evPool[e0], st);
         }
-        PHX_CK(cudaLaunchKernelEx(&cfg, k_solve<R>, S, a));
+        PHX_CK(two ? cudaLaunchKernelEx(&cfg, k_solve<R, PER2>, S, a) : cudaLaunchKernelEx(&cfg, k_solve<R, 1>, S, a));
         if (prof) {
             cudaEventRecord(evPool[e0 + 1], st);
             evUse.push_back({"k_solve", e0});

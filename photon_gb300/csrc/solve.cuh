@@ -44,20 +44,30 @@ namespace phx {
 // dense coarse operators up to this many unknowns (n^2 reals)
 constexpr int DENSE_MAX = 4096;
 
-template <class R>
+// PER: CTAs of the kernel per SM
+template <class R, int PER>
 struct SolveCfg {
     // threads per CTA. FP64 takes 128 registers a thread. FP32 trades registers for warps in
     // flight: house step 1.25 / 1.27 / 1.31 ms at 768 / 896 / 1024 threads, 24 scenarios 6.25 / 5.98 / 5.93
-    static constexpr int T = sizeof(R) == 8 ? 512 : 896;
+    static constexpr int T = sizeof(R) == 8 ? 512 : PER == 1 ? 896 : 512;
     // shared memory for the coarse rows, bytes: what it takes is missing to L1. FP32 house
     // step 1.217 / 1.222 / 1.238 / 1.254 ms at 32 / 64 / 96 / 128 KiB, 1.3e6 cells 3.69 / 3.61 /
     // 3.58 / 3.56; FP64 house 2.796 / 2.756 / 2.755 / 2.762
-    static constexpr int ROWS = sizeof(R) == 8 ? 98304 : 65536;
+    static constexpr int ROWS = PER > 1 ? 32768 : sizeof(R) == 8 ? 98304 : 65536;
     // dynamic shared memory: coarse rows, then by turns the FP32 dot products' terms and
     // the coarsest level's right-hand side
     static constexpr int TERMS = sizeof(R) == 8 ? 0 : 4 * T * 8, DENSE_B = DENSE_MAX * (int)sizeof(R);
     static constexpr int SMEM = ROWS + (TERMS > DENSE_B ? TERMS : DENSE_B);
 };
+
+// CTAs per SM. Two of 512 threads divide the GPU more finely among scenarios than one of
+// 896 (teams of whole CTAs, each as slow as its most loaded scenario) and wait at barriers
+// in turn, but have fewer registers a thread and twice the arrivals. FP32 steps, one / two,
+// ms: 8 scenarios 2.73 / 2.71, 12 3.58 / 3.59, 16 4.43 / 4.29, 24 6.54 / 6.35, 40 9.32 / 8.69,
+// 60 small ones 2.45 / 2.24; 4 scenarios 2.29 / 2.46. So two where a team would have fewer
+// than ten CTAs. FP64 (two of 256 threads) is slower throughout: 24 scenarios 11.46 / 11.55.
+template <class R>
+inline int solvePerSm(int nscn, int sms) { return sizeof(R) == 4 && nscn * 10 > sms ? 2 : 1; }
 
 // How a scenario's pairs are walked: a warp takes 8 consecutive 2x2x2 blocks (four
 // lanes a block) at a time; `warps` warps side by side are a tile, which walks
@@ -847,11 +857,11 @@ __device__ void divideTeams(const Scn<R>* S, int n, int G, int* first) {
 }
 
 // ---- the kernel ----------------------------------------------------------------------
-template <class R>
-__global__ void __launch_bounds__(SolveCfg<R>::T, 1)
+template <class R, int PER>
+__global__ void __launch_bounds__(SolveCfg<R, PER>::T, PER)
 k_solve(const Scn<R>* __restrict__ S, SolveArgs a) {
     using T = R;
-    constexpr int TH = SolveCfg<R>::T;
+    constexpr int TH = SolveCfg<R, PER>::T;
     constexpr bool kMixed = sizeof(R) == 4;
     __shared__ __align__(16) unsigned long long graw[sizeof(Scn<R>) / 8];
     extern __shared__ __align__(16) unsigned pool[];
@@ -860,8 +870,8 @@ k_solve(const Scn<R>* __restrict__ S, SolveArgs a) {
     __shared__ RowSet rowsJ[MAX_LEVELS][TH / 32][ROW_CHUNKS], rowsR[MAX_LEVELS][TH / 32][ROW_CHUNKS];
     __shared__ int poolUsed;
     __shared__ double shDot[2][sizeof(R) == 8 ? TH : TH / 2];   // FP64: the tiles' dot products, by turns; scratch
-    R* const shB = reinterpret_cast<R*>(pool + SolveCfg<R>::ROWS / 4);   // the coarsest right-hand side
-    double* const shTerms = reinterpret_cast<double*>(pool + SolveCfg<R>::ROWS / 4);   // FP32: a tile's terms, by turns
+    R* const shB = reinterpret_cast<R*>(pool + SolveCfg<R, PER>::ROWS / 4);   // the coarsest right-hand side
+    double* const shTerms = reinterpret_cast<double*>(pool + SolveCfg<R, PER>::ROWS / 4);   // FP32: a tile's terms, by turns
     __shared__ double shMx[32];
     __shared__ int first[MAX_BATCH + 1];
     __shared__ int gaveUp;
@@ -993,9 +1003,9 @@ k_solve(const Scn<R>* __restrict__ S, SolveArgs a) {
                 const Level<R>& C = g.lv[l + 1];
                 const int chunk = gw + m * nw;
                 RowSet j{-1, -1}, r{-1, -1};
-                if (chunk * 32 < L.n) j = keepRows<R>(L.rows, L.setsJ[chunk], true, pool, &poolUsed, SolveCfg<R>::ROWS / 4);
+                if (chunk * 32 < L.n) j = keepRows<R>(L.rows, L.setsJ[chunk], true, pool, &poolUsed, SolveCfg<R, PER>::ROWS / 4);
                 if (chunk * (32 / RRJ_LANES) < C.n)
-                    r = keepRows<R>(L.rows, L.setsR[chunk], false, pool, &poolUsed, SolveCfg<R>::ROWS / 4);
+                    r = keepRows<R>(L.rows, L.setsR[chunk], false, pool, &poolUsed, SolveCfg<R, PER>::ROWS / 4);
                 if (lane == 0) {
                     rowsJ[l][warp][m] = j;
                     rowsR[l][warp][m] = r;
@@ -1026,9 +1036,9 @@ k_solve(const Scn<R>* __restrict__ S, SolveArgs a) {
             }
         };
         auto restrictLevel = [&](int l) {
-            constexpr int PER = 32 / RRJ_LANES;
-            for (int m = 0, j = gw * PER; j < g.lv[l + 1].n; ++m, j += nw * PER)
-                restrictRows(g, l, j, pool, m < ROW_CHUNKS ? rowsR[l][warp][m] : inLevel(g.lv[l].setsR[j / PER]), B.tag, tw);
+            constexpr int GROUP = 32 / RRJ_LANES;
+            for (int m = 0, j = gw * GROUP; j < g.lv[l + 1].n; ++m, j += nw * GROUP)
+                restrictRows(g, l, j, pool, m < ROW_CHUNKS ? rowsR[l][warp][m] : inLevel(g.lv[l].setsR[j / GROUP]), B.tag, tw);
         };
         auto coarsest = [&]() {
             const Level<R>& L = g.lv[nl - 1];

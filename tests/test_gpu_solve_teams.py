@@ -93,6 +93,24 @@ def test_teams_do_not_change_the_result(precision, ctas, monkeypatch):
             assert np.array_equal(batch.get(s, f), g.get(f)), (s, f)
 
 
+@pytest.mark.gpu
+@pytest.mark.parametrize("precision", [_lib.PREC_FP64, _lib.PREC_MIXED])
+def test_a_large_batch_equals_its_scenarios_alone(precision):
+    """24 scenarios: the FP32 solve runs two CTAs per SM instead of one."""
+    shapes = [(13, 11, 9), (10, 8, 8), (9, 7, 5), (16, 12, 8), (21, 10, 9), (33, 12, 10), (12, 12, 12), (40, 9, 7)]
+    cs = [casegen.tiny_room(*d, 0.2) for d in shapes]
+    for c in cs:
+        c.profile.tol, c.profile.rel_tol = 0.0, 1e-8
+    batch = Batch([cs[q % len(cs)] for q in range(24)], precision)
+    batch.run(3, 0.02)
+    for s, c in enumerate(cs):
+        alone = Solver(c, precision)
+        alone.run(3, 0.02)
+        for f in STATE:
+            for q in range(s, 24, len(cs)):
+                assert np.array_equal(batch.get(q, f), alone.get(f)), (q, f)
+
+
 @pytest.mark.parametrize("precision,widest", [(_lib.PREC_FP64, 410), (_lib.PREC_MIXED, 776)])
 def test_rows_past_the_widest_are_refused(precision, widest):
     """Rejected on the host, before any device call."""
