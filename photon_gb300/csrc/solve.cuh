@@ -8,10 +8,10 @@
 // its size (a launch, a chain of dependent loads for its tables and
 // descriptor, and a drained GPU); a team barrier costs 1.0 us between 2 CTAs
 // and 1.2 to 1.5 us between 152 with stores in flight, and tables, scalars and
-// coarse rows stay on the SM. Measured, ms per step, launches / this kernel:
-// 36x24x24 room 2.17 / 1.06 in FP64 and 1.13 / 0.55 mixed, 72x52x44 house
-// 6.8 / 4.3 and 2.77 / 1.30, 1.3 M cells mixed 5.66 / 4.1, 24 houses of 2.9 M
-// cells mixed 8.1 / 5.9.
+// coarse rows stay on the SM. Measured, ms per step, launches / this kernel (the other
+// stages' changes included): 36x24x24 room 2.15 / 0.72 in FP64 and 1.13 / 0.45 mixed,
+// 72x52x44 house 6.8 / 2.75 and 2.77 / 1.21, 1.3 M cells mixed 5.66 / 3.58, 24 houses of
+// 2.9 M cells mixed 8.1 / 5.6.
 //
 // What bounds it. One building: latency. Per pass a barrier, one L2 round trip
 // (286 cycles) and the pass's own instructions, 2 to 3 us together; per
@@ -33,9 +33,9 @@
 // its size alone (SolveTiling). Neither depends on the teams, so a scenario's
 // result is the same bits alone, in any batch and with any number of CTAs.
 //
-// Waits: a team barrier gives up after TEAM_WAIT_CYCLES, records it in the
-// context's error word and ends the kernel; the launch is cooperative, so all
-// CTAs of a team are resident.
+// Waits: a team barrier and the reader of a tagged value give up after
+// TEAM_WAIT_CYCLES, record it in the context's error word and end the kernel; the
+// launch is cooperative, so all CTAs of a team are resident.
 #pragma once
 #include "mixed_kernels.cuh"
 

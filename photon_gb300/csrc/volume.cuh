@@ -82,29 +82,31 @@ __device__ __forceinline__ float vNoise(V3 x) {
     return vMix(vMix(line(y0, z0), line(y1, z0), f.y), vMix(line(y0, z1), line(y1, z1), f.y), f.z);
 }
 template <bool SMALL>
-__device__ __forceinline__ float vFlameNoiseAt(V3 q, float time) {
+__device__ __forceinline__ float vFlameNoiseAt(V3 p, float time) {
+    const V3 q = p * v3(5.0f, 5.0f, 2.6f) - v3(0.0f, 0.0f, time * 3.2f);
     return 0.55f * vNoise<SMALL>(q) + 0.30f * vNoise<SMALL>(q * 2.1f + v3(0.0f, 0.0f, -time * 2.0f)) + 0.15f * vNoise<SMALL>(q * 4.3f);
 }
 template <bool SMALL>
-__device__ __forceinline__ float vSmokeNoiseAt(V3 q) {
+__device__ __forceinline__ float vSmokeNoiseAt(V3 p, float time) {
+    V3 q = p * 1.6f - v3(0.0f, 0.0f, time * 0.35f);
     q = q + (v3(vNoise<SMALL>(q + v3(5.2f, 1.3f, 0.0f)), vNoise<SMALL>(q + v3(1.7f, 9.2f, 3.1f)), vNoise<SMALL>(q + v3(8.3f, 2.8f, 4.7f))) * 0.6f -
              v3(0.3f, 0.3f, 0.3f));
     float n = 0.5f * vNoise<SMALL>(q) + 0.3f * vNoise<SMALL>(q * 2.03f + v3(1.7f, 1.7f, 1.7f)) + 0.2f * vNoise<SMALL>(q * 4.1f + v3(3.3f, 3.3f, 3.3f));
     return vSmooth(0.2f, 0.8f, n);
 }
 // far from the origin or late: floorf
-inline __device__ __noinline__ float vFlameNoiseFar(V3 q, float time) { return vFlameNoiseAt<false>(q, time); }
-inline __device__ __noinline__ float vSmokeNoiseFar(V3 q) { return vSmokeNoiseAt<false>(q); }
-__device__ __forceinline__ bool vNear(V3 q, float s) {   // every multiple of it below stays within V_SMALL
-    return fmaxf(fmaxf(fabsf(q.x), fabsf(q.y)), fmaxf(fabsf(q.z), fabsf(s))) < V_SMALL / 8.0f;
+inline __device__ __noinline__ float vFlameNoiseFar(V3 p, float time) { return vFlameNoiseAt<false>(p, time); }
+inline __device__ __noinline__ float vSmokeNoiseFar(V3 p, float time) { return vSmokeNoiseAt<false>(p, time); }
+// every coordinate above stays within V_SMALL: at most 21.5 |p| + 14 |time| + 20. The test is on
+// p and not on q, whose products are contracted into the noise's own additions
+__device__ __forceinline__ bool vNear(V3 p, float time) {
+    return fmaxf(fmaxf(fabsf(p.x), fabsf(p.y)), fmaxf(fabsf(p.z), fabsf(time))) < V_SMALL / 64.0f;
 }
 __device__ __forceinline__ float vFlameNoise(V3 p, float time) {
-    const V3 q = p * v3(5.0f, 5.0f, 2.6f) - v3(0.0f, 0.0f, time * 3.2f);
-    return vNear(q, time * 2.0f) ? vFlameNoiseAt<true>(q, time) : vFlameNoiseFar(q, time);
+    return vNear(p, time) ? vFlameNoiseAt<true>(p, time) : vFlameNoiseFar(p, time);
 }
 __device__ __forceinline__ float vSmokeNoise(V3 p, float time) {
-    const V3 q = p * 1.6f - v3(0.0f, 0.0f, time * 0.35f);
-    return vNear(q, 0.0f) ? vSmokeNoiseAt<true>(q) : vSmokeNoiseFar(q);
+    return vNear(p, time) ? vSmokeNoiseAt<true>(p, time) : vSmokeNoiseFar(p, time);
 }
 __device__ __forceinline__ V3 vFlameColor(float k) {
     return vMix(vMix(v3(0.9f, 0.18f, 0.02f), v3(1.0f, 0.5f, 0.08f), vSmooth(0.0f, 0.4f, k)), v3(1.0f, 0.9f, 0.55f),
