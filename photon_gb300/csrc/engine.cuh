@@ -143,6 +143,9 @@ struct Scenario {
         if (kMixed) coarseStop = vcycleStopFor(NN);   // the tuned schedule of the scenario's size, if any
         MG = buildMultigrid(geo, DENSE_MAX, coarseStop, coarseSolveFor());
         buildRowSets();
+        a0Same[0] = MG.a0x == geo.ax;
+        a0Same[1] = MG.a0y == geo.ay;
+        a0Same[2] = MG.a0z == geo.az;
         buildLeakFaces();
         return PHX_OK;
     }
@@ -206,9 +209,9 @@ struct Scenario {
         s.fx = carve<R>(base, off, NX); s.fy = carve<R>(base, off, NY); s.fz = carve<R>(base, off, NZ);
         s.ax = carve<R>(base, off, NX); s.ay = carve<R>(base, off, NY); s.az = carve<R>(base, off, NZ);
         // the same arrays where no wind-inflow boundary face is closed
-        s.a0x = MG.a0x == geo.ax ? s.ax : carve<R>(base, off, NX);
-        s.a0y = MG.a0y == geo.ay ? s.ay : carve<R>(base, off, NY);
-        s.a0z = MG.a0z == geo.az ? s.az : carve<R>(base, off, NZ);
+        s.a0x = a0Same[0] ? s.ax : carve<R>(base, off, NX);
+        s.a0y = a0Same[1] ? s.ay : carve<R>(base, off, NY);
+        s.a0z = a0Same[2] ? s.az : carve<R>(base, off, NZ);
         s.lx = geo.anyLeak ? carve<uint8_t>(base, off, NX) : nullptr;
         s.ly = geo.anyLeak ? carve<uint8_t>(base, off, NY) : nullptr;
         s.lz = geo.anyLeak ? carve<uint8_t>(base, off, NZ) : nullptr;
@@ -295,6 +298,7 @@ struct Scenario {
         std::vector<RowSet> j, r;
     };
     std::vector<RowSets> rowSets;
+    bool a0Same[3] = {false, false, false};   // level 0's coefficients are the faces' own, per axis
     void buildRowSets() {
         constexpr int RW = (int)sizeof(R) / 4;
         rowSets = std::vector<RowSets>(MG.lv.size());
