@@ -812,7 +812,7 @@ __device__ __forceinline__ void restrictRows(const Scn<R>& g, int l, int jBase, 
 }
 
 // ---- teams ------------------------------------------------------------------------
-// A scenario that has not solved yet counts as this many iterations: a large one that joins
+// A scenario at time 0, which has not solved yet, counts as this many iterations: a large one that joins
 // a running batch would else get a CTA or two for its longest solve (serving 32 requests of
 // 20 k to 1.3 M cells, mixed: 343 M cell-updates/s and 28 ms at the 99th percentile of a
 // step, 292 M and 90 ms with the count of 0).
@@ -829,8 +829,7 @@ __device__ void divideTeams(const Scn<R>* S, int n, int G, int* first) {
         const int nblk = (int)g.dvL0[1].d * ((g.nz + 1) >> 1);
         const SolveTiling tl = solveTiling<R>(nblk);
         most[s] = tl.warps == 1 ? (tl.nt + 1) / 2 : tl.nt;
-        const float its = (float)g.sv[SV_WITERS];
-        work[s] = (float)nblk * (its > 0.0f ? its + 2.0f : SOLVE_FIRST_ITERS);
+        work[s] = (float)nblk * (g.sv[SV_TIME] > 0 ? (float)(g.sv[SV_WITERS] + 2.0) : SOLVE_FIRST_ITERS);
     }
     __syncthreads();
     if (threadIdx.x < 32) {
