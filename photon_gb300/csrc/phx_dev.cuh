@@ -209,7 +209,7 @@ struct Scn {
     R *p, *S, *nu, *Pb, *Q, *Qr, *hrr, *massSrc;
     uint8_t *lit, *lit2, *pilot;
     R* tmp[9];                   // turbulence: cell-centre velocities and filter passes
-    R* rho;                      // FP64 path: gas density of the current T and Pb (k_turb_nu, k_energy; null: mixed)
+    R* rho;                      // FP64 path: every cell's density at its current T and Pb (k_turb_nu, k_energy; null: mixed)
     // pressure solve
     R *b, *r, *z, *d, *q;
     double* p64;                 // mixed path: FP64 pressure; the FP32 iterate p holds the part not yet folded in

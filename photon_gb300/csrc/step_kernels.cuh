@@ -380,8 +380,10 @@ __global__ void k_turb_nu(const Scn<R>* __restrict__ S, Dom dom) {
     int c = tile_ * TPB + threadIdx.x;
     T m = 0;   // the max is taken in the arithmetic type: no FP64 instruction per cell on the mixed path
     if (c < g.N) {
-        if (g.blocked[c]) g.nu[c] = 0;
-        else {
+        if (g.blocked[c]) {
+            g.nu[c] = 0;
+            if constexpr (sizeof(T) == 8) g.rho[c] = rhoOf(g, c);   // read across a face left open beside the solid
+        } else {
             const int sxy = g.nx * g.ny, kz = (int)divU((unsigned)c, g.dvB[0]);
             const int cLo = kz > 0 ? c - sxy : c, cHi = kz < g.nz - 1 ? c + sxy : c;
             const bool hasLo = kz > 0 && !g.blocked[cLo], hasHi = kz < g.nz - 1 && !g.blocked[cHi];
@@ -480,12 +482,12 @@ __device__ __forceinline__ void swapScalars(Scn<R>& g) {
     for (int q = 0; q < NSC; ++q) { R* t = g.sc[q]; g.sc[q] = g.sc2[q]; g.sc2[q] = t; }
 }
 
-// FP64 path: density of every gas cell, before a stage that runs on its own
+// FP64 path: density of every cell, before a stage that runs on its own
 template <class R>
 __global__ void k_rho(const Scn<R>* __restrict__ S, Dom dom) {
     PHX_PROLOGUE(dom);
     const int c = tile_ * TPB + threadIdx.x;
-    if (c < g.N && !g.blocked[c]) g.rho[c] = rhoOf(g, c);
+    if (c < g.N) g.rho[c] = rhoOf(g, c);
 }
 
 // Solver::energyAndExpansion (src/sim/gasphase.cpp:251-271). swap (full step): the
