@@ -32,7 +32,7 @@ UNITS = {
     "server.cpp": [],
 }
 HEADERS = ["phx_dev.cuh", "step_kernels.cuh", "pressure_kernels.cuh", "engine.cuh", "engine.h", "host_setup.h",
-           "mixed_kernels.cuh", "selftest.cuh", "level0.cuh", "solve.cuh", "fdiv.cuh", "radiation.cuh", "volume.cuh"]
+           "mixed_kernels.cuh", "selftest.cuh", "level0.cuh", "teams.cuh", "solve.cuh", "fdiv.cuh", "radiation.cuh", "volume.cuh"]
 
 
 def _newer(target, deps):

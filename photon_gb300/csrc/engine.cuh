@@ -622,6 +622,7 @@ public:
     size_t ownCap = 0;
     double* dTimes = nullptr;    // simulated time of each scenario (read-back staging)
     double* dMaxPart = nullptr;  // k_solve: two maxima per CTA
+    TeamTable teams{};           // ... and which scenario each CTA works on
     int solveGrid = 0;           // k_solve: CTAs resident at once
     int solvePer = 1;            // ... per SM
     bool smoothOne = false;            // mixed path: one Jacobi sweep per coarse level and leg (vcycleSweeps)
@@ -1079,6 +1080,10 @@ public:
                 dErr = carve<unsigned>(base, off, 4);
                 dTimes = carve<double>(base, off, cap);
                 dMaxPart = carve<double>(base, off, 2 * MAX_SOLVE_CTAS);
+                teams.ctas = carve<SolveCta>(base, off, MAX_SOLVE_CTAS);
+                teams.next = carve<int>(base, off, cap);
+                teams.work = carve<float2>(base, off, cap);
+                teams.arrived = carve<unsigned>(base, off, 4);
                 if (pass == 0) {
                     cudaError_t e = cudaMalloc(&tab, off + 256);
                     if (e != cudaSuccess) { tab = nullptr; err = "device allocation of the batch tables failed"; return PHX_ERR_OOM; }
@@ -1167,6 +1172,7 @@ public:
         solvePer = occ[1] >= 2 ? solvePerSm<R>(nscn(), sms) : 1;
         solveGrid = std::min(sms * (solvePer == 2 ? 2 : occ[0]), MAX_SOLVE_CTAS);
         if (const char* c = std::getenv("PHX_PERSIST_CTAS")) solveGrid = std::max(1, std::min(solveGrid, std::atoi(c)));
+        teams.grid = solveGrid;
         return PHX_OK;
     }
 
@@ -1329,7 +1335,7 @@ public:
 
     // ---- stages ---------------------------------------------------------------------
     void stBegin(bool computeDt, double dt) {
-        launch("k_begin", D_ONE, 32, k_begin<R>, (const Scn<R>*)dS, dom[D_ONE], computeDt ? 1 : 0, dt);
+        launch("k_begin", D_ONE, TEAM_TPB, k_begin<R>, (const Scn<R>*)dS, dom[D_ONE], computeDt ? 1 : 0, dt, teams);
     }
     // Stages. In the full step the double buffers are exchanged by kernels that do not
     // read them (turbulence: the burning flags; energy: the velocities, ahead of
@@ -1372,7 +1378,7 @@ public:
     // the whole pressure solve in one cooperative launch (solve.cuh)
     int launchSolve(int vcycleOnly) {
         SolveArgs a;
-        a.nscn = nscn();
+        a.teams = teams;
         a.cap = maxItersAll() + 2;
         a.vcycleOnly = vcycleOnly;
         a.maxPart = dMaxPart;
@@ -1559,7 +1565,7 @@ public:
         Scenario<R>& S = *sc[0];
         const int N = S.geo.N();
         PHX_TRY(S.put(st, S.h.r, std::vector<double>(r, r + N)));
-        launch("k_reset", D_ONE, 32, k_reset<R>, (const Scn<R>*)dS, dom[D_ONE]);
+        k_reset<R><<<1, TEAM_TPB, 0, st>>>(dS, teams);
         PHX_TRY(launchSolve(1));
         PHX_TRY(checkLaunch());
         return getReal(S.h.z, N, z);

@@ -27,12 +27,15 @@ __global__ void k_read_times(const Scn<R>* __restrict__ S, int n, double* out) {
     if (s < n) out[s] = S[s].sv[SV_TIME];
 }
 
-// before a bare V-cycle (one thread per scenario; k_begin does it for a step's solve)
+// before a bare V-cycle of the first scenario (k_begin does it for a step's solves); one CTA
 template <class R>
-__global__ void k_reset(const Scn<R>* __restrict__ S, Dom dom) {
-    int s_, tile_;
-    locate(dom, blockIdx.x, s_, tile_);
-    if (threadIdx.x == 0) startSolve(S[s_]);
+__global__ void __launch_bounds__(TEAM_TPB) k_reset(const Scn<R>* __restrict__ S, TeamTable teams) {
+    if (threadIdx.x == 0) {
+        startSolve(S[0]);
+        offerWork(S[0], 0, teams);
+    }
+    __syncthreads();
+    divideTeams(1, teams);
 }
 
 }  // namespace phx

@@ -83,7 +83,6 @@ enum Slot {
     SV_INV,
     SV_HAVEPREV,                 // mixed path: p64prev holds the previous step's pressure
     SV_SRC_MF = 32,              // MAX_SRC injection amounts of this step (-1 = inactive)
-    SV_WITERS = SV_SRC_MF + MAX_SRC,                     // iterations of the last solve (SV_PITERS), fixed for the coming one: its team's weight
     SV_COUNT = 64
 };
 

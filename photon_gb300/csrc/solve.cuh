@@ -19,12 +19,10 @@
 // Large batches: instruction issue in FP32, the FP64 pipe (a warp's
 // instruction takes it about 19 cycles) in FP64.
 //
-// Teams. The CTAs of the grid are divided into one team per scenario, in
-// proportion to the scenario's work (cells times the iterations of its last
-// solve), at least one CTA each. A team runs its scenario's passes one after
-// the other with a barrier of its own between them, so a scenario never waits
-// for another one's iterations and a stopped scenario costs nothing. With more
-// scenarios than CTAs a team is one CTA that takes several scenarios in turn.
+// Teams. The CTAs of the grid are divided into teams, one per scenario (teams.cuh).
+// A team runs its scenario's passes one after the other with a barrier of its own
+// between them, so a scenario never waits for another one's iterations and a
+// stopped scenario costs nothing. Small scenarios can take turns on a CTA.
 // Every CTA of a team keeps the scenario's scalars in shared memory and
 // computes alpha, beta and the stop test itself from the passes' partial sums,
 // in one fixed order, so all of them take the same decisions.
@@ -69,34 +67,8 @@ struct SolveCfg {
 template <class R>
 inline int solvePerSm(int nscn, int sms) { return sizeof(R) == 4 && nscn * 10 > sms ? 2 : 1; }
 
-// How a scenario's pairs are walked: a warp takes 8 consecutive 2x2x2 blocks (four
-// lanes a block) at a time; `warps` warps side by side are a tile, which walks
-// `reps` such groups. A tile's dot product is one partial sum. The shape follows
-// from the scenario's size alone, so its sums do not depend on the team.
-// FP32: a tile is always the 32 blocks of four warps, whose products are added in
-// the order of one thread per block (the block's cells in ascending order, then
-// a warp's shuffle tree), four tiles to a sum that reaches FP64.
-struct SolveTiling {
-    int warps, reps, nt;
-};
-template <class R>
-__host__ __device__ inline SolveTiling solveTiling(int nblk) {
-    const int groups = (nblk + 7) / 8;
-    SolveTiling t;
-    t.reps = 1;
-    if (sizeof(R) == 4) {
-        t.warps = 4;
-    } else {
-        t.warps = groups <= 512 ? 1 : groups <= 4096 ? 4 : 8;
-        while (groups / (t.warps * t.reps) >= 4096) t.reps *= 2;
-    }
-    const int per = t.warps * t.reps;
-    t.nt = (groups + per - 1) / per;
-    return t;
-}
-
 struct SolveArgs {
-    int nscn;
+    TeamTable teams;
     int cap;                 // iterations after which the loop ends whatever the flags say
     int vcycleOnly;          // 1: one V-cycle z = M r without the CG (phx_precondition)
     double* maxPart;         // 2 per CTA: max |r| of the recursion, max |r| of the FP64 residual
@@ -445,28 +417,28 @@ __device__ __forceinline__ void solvePair(const Scn<R>& g, const SolveBufs<R>& B
 
 // ---- team barrier ---------------------------------------------------------------
 struct Team {
-    unsigned* bar;           // arrivals since the start of the solve
-    unsigned* errWord;
-    unsigned target;
-    int size, rank, first;   // CTAs, this CTA's place, the team's first CTA
+    unsigned target;         // arrivals at g.teamBar since the start of the solve that end the next wait
+    int size, rank;          // CTAs, this CTA's place
 };
 
 // every thread of every CTA of the team calls it; false: the wait ran out and
 // the kernel has to end. *gaveUp is shared memory, 0 at first.
-__device__ __forceinline__ bool teamSync(Team& t, volatile int* gaveUp) {
+template <class R>
+__device__ __forceinline__ bool teamSync(const Scn<R>& g, Team& t, volatile int* gaveUp) {
     __syncthreads();
     if (t.size == 1) return *gaveUp == 0;
     t.target += (unsigned)t.size;
     if (threadIdx.x == 0) {
-        asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(t.bar) : "memory");
+        unsigned* const bar = g.teamBar;
+        asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(bar) : "memory");
         unsigned seen;
-        asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(seen) : "l"(t.bar) : "memory");
+        asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(seen) : "l"(bar) : "memory");
         if ((int)(seen - t.target) < 0) {
             const long long t0 = clock64();
             do {
-                asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(seen) : "l"(t.bar) : "memory");
+                asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(seen) : "l"(bar) : "memory");
                 if (clock64() - t0 > TEAM_WAIT_CYCLES) {
-                    atomicOr(t.errWord, ERR_TEAM_WAIT);
+                    atomicOr(g.errWord, ERR_TEAM_WAIT);
                     *gaveUp = 1;
                     break;
                 }
@@ -811,56 +783,6 @@ __device__ __forceinline__ void restrictRows(const Scn<R>& g, int l, int jBase, 
     }
 }
 
-// ---- teams ------------------------------------------------------------------------
-// A scenario at time 0, which has not solved yet, counts as this many iterations: a large one that joins
-// a running batch would else get a CTA or two for its longest solve (serving 32 requests of
-// 20 k to 1.3 M cells, mixed: 343 M cell-updates/s and 28 ms at the 99th percentile of a
-// step, 292 M and 90 ms with the count of 0).
-constexpr float SOLVE_FIRST_ITERS = 40.0f;
-// CTAs per scenario: the smallest bound on work / CTAs that the grid can meet
-// (bisection on the bound), at least one CTA and at most one per tile. One
-// warp; every CTA computes the same division.
-template <class R>
-__device__ void divideTeams(const Scn<R>* S, int n, int G, int* first) {
-    __shared__ float work[MAX_BATCH];
-    __shared__ int most[MAX_BATCH];
-    for (int s = threadIdx.x; s < n; s += blockDim.x) {
-        const Scn<R>& g = S[s];
-        const int nblk = (int)g.dvL0[1].d * ((g.nz + 1) >> 1);
-        const SolveTiling tl = solveTiling<R>(nblk);
-        most[s] = tl.warps == 1 ? (tl.nt + 1) / 2 : tl.nt;
-        work[s] = (float)nblk * (g.sv[SV_TIME] > 0 ? (float)(g.sv[SV_WITERS] + 2.0) : SOLVE_FIRST_ITERS);
-    }
-    __syncthreads();
-    if (threadIdx.x < 32) {
-        auto ctas = [&](int s, float bound) { return min(most[s], max(1, (int)ceilf(work[s] / bound))); };
-        float hi = 0;
-        for (int s = threadIdx.x; s < n; s += 32) hi = fmaxf(hi, work[s]);
-        hi = warpMax(hi);
-        float lo = 0;
-        for (int it = 0; it < 20; ++it) {
-            const float mid = 0.5f * (lo + hi);
-            int sum = 0;
-            for (int s = threadIdx.x; s < n; s += 32) sum += mid > 0 ? ctas(s, mid) : most[s];
-            sum = __reduce_add_sync(0xffffffffu, sum);
-            if (sum <= G) hi = mid; else lo = mid;
-        }
-        int base = 0;
-        for (int s0 = 0; s0 < n; s0 += 32) {
-            const int s = s0 + (int)threadIdx.x;
-            int v = s < n ? (hi > 0 ? ctas(s, hi) : 1) : 0;
-            for (int o = 1; o < 32; o <<= 1) {
-                const int u = __shfl_up_sync(0xffffffffu, v, o);
-                if ((int)threadIdx.x >= o) v += u;
-            }
-            if (s < n) first[s + 1] = base + v;
-            base += __shfl_sync(0xffffffffu, v, 31);
-        }
-        if (threadIdx.x == 0) first[0] = 0;
-    }
-    __syncthreads();
-}
-
 // ---- the kernel ----------------------------------------------------------------------
 template <class R, int PER>
 __global__ void __launch_bounds__(SolveCfg<R, PER>::T, PER)
@@ -878,28 +800,15 @@ k_solve(const Scn<R>* __restrict__ S, SolveArgs a) {
     R* const shB = reinterpret_cast<R*>(pool + SolveCfg<R, PER>::ROWS / 4);   // the coarsest right-hand side
     double* const shTerms = reinterpret_cast<double*>(pool + SolveCfg<R, PER>::ROWS / 4);   // FP32: a tile's terms, by turns
     __shared__ double shMx[32];
-    __shared__ int first[MAX_BATCH + 1];
     __shared__ int gaveUp;
     static_assert(sizeof(Scn<R>) % 8 == 0, "descriptors are copied as 8-byte words");
     const int tid = (int)threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const int G = (int)gridDim.x, b = (int)blockIdx.x;
+    const int b = (int)blockIdx.x;
     if (tid == 0) gaveUp = 0;
-    Team team;
-    int s = b, sStep = G;
-    team.size = 1; team.rank = 0; team.first = b; team.target = 0; team.bar = nullptr; team.errWord = nullptr;
-    if (a.nscn <= G) {
-        divideTeams(S, a.nscn, G, first);
-        s = a.nscn;
-        for (int q = 0; q < a.nscn; ++q)
-            if (b >= first[q] && b < first[q + 1]) { s = q; break; }
-        if (s >= a.nscn) return;   // no work for this CTA
-        sStep = a.nscn;
-        team.first = first[s];
-        team.size = first[s + 1] - first[s];
-        team.rank = b - team.first;
-    }
+    const SolveCta mine = a.teams.ctas[b];
+    Team team{0, mine.size, mine.rank};
     const Scn<R>& g = *reinterpret_cast<const Scn<R>*>(graw);
-    for (; s < a.nscn; s += sStep) {
+    for (int s = mine.scenario; s >= 0; s = a.teams.next[s]) {
         __syncthreads();
         {   // the scenario's descriptor and scalars
             const unsigned long long* src = reinterpret_cast<const unsigned long long*>(S + s);
@@ -919,12 +828,10 @@ k_solve(const Scn<R>* __restrict__ S, SolveArgs a) {
                 cg.it = cg.done = cg.repl = cg.brk = 0;
                 poolUsed = 0;
             }
-            team.bar = g.teamBar;
-            team.errWord = g.errWord;
             __syncthreads();
         }
         const int N = g.N, nl = g.nLevels;
-        const int nblk = (int)g.dvL0[1].d * ((g.nz + 1) >> 1);
+        const int nblk = solveBlocks(g);
         const SolveTiling tl = solveTiling<R>(nblk);
         const int nt = tl.nt;
         const int rank = team.rank, size = team.size;
@@ -936,7 +843,7 @@ k_solve(const Scn<R>* __restrict__ S, SolveArgs a) {
         B.p = g.p; B.z = g.z; B.q = g.q; B.r = g.r; B.d = g.d;
         B.dNew = nullptr; B.alpha = T(0); B.beta = T(0); B.haveD = false;
 
-#define PHX_TEAM_SYNC() do { if (!teamSync(team, &gaveUp)) return; } while (0)
+#define PHX_TEAM_SYNC() do { if (!teamSync(g, team, &gaveUp)) return; } while (0)
         // one pass over the team's tiles
         const int slot = warp / tl.warps, slots = TH / 32 / tl.warps, wt = warp - slot * tl.warps;
         int turn = 0;
@@ -1249,12 +1156,12 @@ k_solve(const Scn<R>* __restrict__ S, SolveArgs a) {
             PHX_PASS(PASS_BLACK, nullptr, none, true);
             PHX_TEAM_SYNC();
             PHX_PASS(PASS_RED, partRz, none, true);
-            if (phase == 2) return;
+            if (phase == 2) return;   // of one scenario only
             PHX_TEAM_SYNC();
             // r.z, the maxima, beta and the stop test
             if (warp >= TH / 32 - 2) {   // the maxima of the recursion and of the FP64 residual
                 const int which = warp - (TH / 32 - 2);
-                const double* mp = a.maxPart + 2 * team.first + which;
+                const double* mp = a.maxPart + 2 * (b - rank) + which;
                 double m = 0;
                 for (int i = lane; i < size; i += 32) m = mx(m, __ldcg(mp + 2 * i));
                 m = warpMaxPos(m);

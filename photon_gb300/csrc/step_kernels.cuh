@@ -9,7 +9,7 @@
 // per-CTA partials, then the last CTA of a scenario sums the partials in CTA
 // order, so results do not depend on scheduling.
 #pragma once
-#include "phx_dev.cuh"
+#include "teams.cuh"
 
 namespace phx {
 
@@ -98,11 +98,9 @@ __global__ void k_wind(const Scn<R>* __restrict__ S, Dom dom) {
 // Solver::stableDt (src/sim/gasphase.cpp:63-70) and the injection amounts of
 // injectIgnitions / injectBurners (src/sim/solver.cpp:271-280,
 // src/sim/gasphase.cpp:92-105, Burner::powerAt src/sim/solver.h:122-126).
-// One thread per scenario.
+// One thread per scenario; the last CTA then divides the solve's CTAs among all.
 template <class R>
-__global__ void k_begin(const Scn<R>* __restrict__ S, Dom dom, int computeDt, double dtGiven) {
-    PHX_PROLOGUE(dom);
-    if (threadIdx.x != 0) return;
+__device__ __forceinline__ void beginScenario(const Scn<R>& g, int computeDt, double dtGiven) {
     double* sv = g.sv;
     double dt;
     if (computeDt) {
@@ -143,7 +141,6 @@ __global__ void k_begin(const Scn<R>* __restrict__ S, Dom dom, int computeDt, do
         sv[SV_SRC_MF + q] = mf;
     }
     sv[SV_FUELIN] = fuelIn;
-    sv[SV_WITERS] = sv[SV_PITERS];
     startSolve(g);
     // reductions of this step start from their neutral values
     sv[SV_MAXNU] = 0;
@@ -153,6 +150,24 @@ __global__ void k_begin(const Scn<R>* __restrict__ S, Dom dom, int computeDt, do
     sv[SV_BMAX] = 0;
     sv[SV_MAXGAST] = K_T0;
     sv[SV_BURNING] = 0;
+}
+template <class R>
+__global__ void __launch_bounds__(TEAM_TPB) k_begin(const Scn<R>* __restrict__ S, Dom dom, int computeDt, double dtGiven, TeamTable teams) {
+    __shared__ int amLast;
+    PHX_PROLOGUE(dom);
+    if (threadIdx.x == 0) {
+        beginScenario(g, computeDt, dtGiven);
+        offerWork(g, s_, teams);
+        amLast = 1;
+        if (dom.nscn > 1) {
+            __threadfence();
+            amLast = atomicAdd(teams.arrived, 1u) == (unsigned)dom.nscn - 1u;
+            if (amLast) *teams.arrived = 0;
+            __threadfence();
+        }
+    }
+    __syncthreads();
+    if (amLast) divideTeams(dom.nscn, teams);
 }
 
 // ---------------------------------------------------------------------------
