@@ -198,11 +198,13 @@ struct Scenario {
         return layoutMain(nullptr) + TAIL_BYTES + layoutLevels(nullptr);
     }
 
+    // 2x2x2 blocks of the pressure solve
+    int blocks() const { return ((geo.nx + 1) >> 1) * ((geo.ny + 1) >> 1) * ((geo.nz + 1) >> 1); }
+
     size_t layoutMain(char* base) {
         const int N = geo.N(), NX = geo.NX(), NY = geo.NY(), NZ = geo.NZ();
         // one reduction partial per CTA of the cell domain and per tile of the solve
-        const int nblk = ((geo.nx + 1) >> 1) * ((geo.ny + 1) >> 1) * ((geo.nz + 1) >> 1);
-        const int partStride = std::max((N + TPB - 1) / TPB, 2 * solveTiling<R>(nblk).nt) + 2;
+        const int partStride = std::max((N + TPB - 1) / TPB, 2 * solveTiling<R>(blocks()).nt) + 2;
         size_t off = 0;
         Scn<R>& s = h;
         s.blocked = carve<uint8_t>(base, off, N);
@@ -1171,6 +1173,9 @@ public:
         if (occ[0] < 1) { err = "the solve kernel does not fit an SM"; return PHX_ERR_CUDA; }
         solvePer = occ[1] >= 2 ? solvePerSm<R>(nscn(), sms) : 1;
         solveGrid = std::min(sms * (solvePer == 2 ? 2 : occ[0]), MAX_SOLVE_CTAS);
+        long long usable = 0;   // by all scenarios
+        for (auto& S : sc) usable += solveCtas<R>(solveTiling<R>(S->blocks()));
+        solveGrid = (int)std::min<long long>(solveGrid, usable);
         if (const char* c = std::getenv("PHX_PERSIST_CTAS")) solveGrid = std::max(1, std::min(solveGrid, std::atoi(c)));
         teams.grid = solveGrid;
         return PHX_OK;

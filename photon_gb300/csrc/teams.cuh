@@ -32,8 +32,18 @@ __host__ __device__ inline SolveTiling solveTiling(int nblk) {
     t.nt = (groups + per - 1) / per;
     return t;
 }
-// the most CTAs a scenario can use
-__host__ __device__ inline int solveCtas(const SolveTiling& t) { return t.warps == 1 ? (t.nt + 1) / 2 : t.nt; }
+// The CTAs a scenario is given at most: two tiles a CTA cost it nothing where they are a warp
+// each (FP64) or a third of the GPU and more has one (FP32, 36x24x24 room of 81 tiles: 41 / 81 /
+// 152 CTAs 0.476 / 0.482 / 0.494 ms a step; 52x40x32 of 260: 130 / 152 0.526 / 0.537; but 36
+// tiles: 18 / 36 0.403 / 0.383). The grid is no larger than its scenarios can use, so that
+// small contexts run side by side: four closets on four threads 0.10 ms a step, with
+// grids of the whole GPU 0.23, four FP32 rooms 0.12 and 0.30.
+template <class R>
+__host__ __device__ inline int solveCtas(const SolveTiling& t) {
+    const int half = (t.nt + 1) / 2;
+    if (sizeof(R) == 4) return t.nt < 48 ? t.nt : half < 48 ? 48 : half;
+    return t.warps == 1 ? half : t.nt;
+}
 
 // The grid's CTAs among the scenarios. A scenario has a team of CTAs, in proportion to its
 // work (blocks times the iterations of its last solve), at least one. With many scenarios
@@ -67,7 +77,7 @@ __device__ __forceinline__ float solveWork(const Scn<R>& g) {
 // a scenario's share in the division, from the CTA that begins its step
 template <class R>
 __device__ __forceinline__ void offerWork(const Scn<R>& g, int s, const TeamTable& t) {
-    t.work[s] = make_float2(solveWork(g), __int_as_float(solveCtas(solveTiling<R>(solveBlocks(g)))));
+    t.work[s] = make_float2(solveWork(g), __int_as_float(solveCtas<R>(solveTiling<R>(solveBlocks(g)))));
 }
 
 // The division of the first n scenarios' work, by one CTA of TEAM_TPB threads: the smallest bound
