@@ -62,8 +62,8 @@ struct TeamTable {
     int grid;
 };
 
-// A scenario at time 0, which has not solved yet, counts as this many iterations: a large one that joins
-// a running batch would else get a CTA or two for its longest solve (serving 32 requests of
+// A scenario that has not solved yet, new or restored, counts as this many iterations: a large one that
+// joins a running batch would else get a CTA or two for its longest solve (serving 32 requests of
 // 20 k to 1.3 M cells, mixed: 343 M cell-updates/s and 28 ms at the 99th percentile of a
 // step, 292 M and 90 ms with the count of 0).
 constexpr float SOLVE_FIRST_ITERS = 40.0f;
@@ -71,7 +71,7 @@ template <class R>
 __device__ __forceinline__ int solveBlocks(const Scn<R>& g) { return (int)g.dvL0[1].d * ((g.nz + 1) >> 1); }
 template <class R>
 __device__ __forceinline__ float solveWork(const Scn<R>& g) {
-    return (float)solveBlocks(g) * (g.sv[SV_TIME] > 0 ? (float)(g.sv[SV_PITERS] + 2.0) : SOLVE_FIRST_ITERS);
+    return (float)solveBlocks(g) * (g.sv[SV_SOLVED] > 0 ? (float)(g.sv[SV_PITERS] + 2.0) : SOLVE_FIRST_ITERS);
 }
 
 // a scenario's share in the division, from the CTA that begins its step
