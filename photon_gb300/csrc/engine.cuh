@@ -521,8 +521,20 @@ struct Scenario {
         return uploadLevels(st);
     }
 
+    // How long a CTA of the solve waits for its team: two seconds, and where one thread solves the
+    // coarsest level while the others wait, the cycles of its 40 sweeps as well (a row's division
+    // and loads some 1,500, a coupling's load and addition some 700; twice that). The
+    // environment's PHX_TEAM_WAIT_CYCLES takes the place of the two seconds.
+    static long long waitCycles(const MgLevel& coarsest) {
+        const char* e = std::getenv("PHX_TEAM_WAIT_CYCLES");
+        const long long base = e ? std::max(0LL, std::atoll(e)) : 4000000000LL;
+        if (!coarsest.dense.empty() || coarsest.rowStart.empty()) return base;
+        return base + 2LL * MG_COARSE_SWEEPS_REF * (3000LL * coarsest.n + 1400LL * coarsest.rowStart.back());
+    }
+
     int uploadLevels(cudaStream_t st) {
         Scn<R>& s = h;
+        s.waitCycles = waitCycles(MG.lv.back());
         PHX_CK(cudaMemsetAsync(mgArena, 0, mgBytes, st));
         for (int l = 1; l < (int)MG.lv.size(); ++l) {
             const MgLevel& L = MG.lv[l];

@@ -222,6 +222,7 @@ struct Scn {
                                  // of the V-cycle (the reference: two, src/sim/pressure_mg.cpp:281-297)
     Level<R> lv[MAX_LEVELS];
     unsigned* errWord;           // the context's error word (a bounded wait that ran out sets a bit)
+    long long waitCycles;        // after which a wait of the solve's team gives up
     // scalars and reductions
     double* sv;
     double* part;                // PS_COUNT x partStride

@@ -66,21 +66,21 @@ __device__ __forceinline__ bool tagLoad(const unsigned long long* a, int i, unsi
     v = __hiloint2double((int)(unsigned)hi, (int)(unsigned)lo);
     return (unsigned)(lo >> 32) == tag && (unsigned)(hi >> 32) == tag;
 }
-// a thread's wait for tagged values: true while it should read again. After about
-// two seconds it gives up for the whole CTA: *gaveUp (shared memory) ends every
+// a thread's wait for tagged values: true while it should read again. After a scenario's
+// limit it gives up for the whole CTA: *gaveUp (shared memory) ends every
 // later wait at once, and the kernel at its next team barrier.
-constexpr long long TEAM_WAIT_CYCLES = 4000000000LL;       // about two seconds
 constexpr unsigned ERR_TEAM_WAIT = 8u;                     // error-word bit
 struct TagWait {
     volatile int* gaveUp;
-    unsigned* errWord;
+    unsigned* const* errWord;    // the descriptor's, in shared memory
+    const long long* limit;
     __device__ __forceinline__ bool again(int& spins, long long& since) const {
         if (*gaveUp) return false;
         if (++spins < 64) return true;
         const long long now = clock64();
         if (spins == 64) since = now;
-        if (now - since <= TEAM_WAIT_CYCLES) return true;
-        atomicOr(errWord, ERR_TEAM_WAIT);
+        if (now - since <= *limit) return true;
+        atomicOr(*errWord, ERR_TEAM_WAIT);
         *gaveUp = 1;
         return false;
     }
@@ -118,9 +118,9 @@ __device__ __forceinline__ R coarseDenseRow(const Level<R>& L, int row, const R*
 
 // coarsest level solved as the reference does it: 20 forward + backward
 // sweeps, serially in one thread (used when the level is too large for a dense
-// operator); x is the thread's own scratch of the level's size
+// operator); b and x are plain arrays of the CTA's own
 template <class R>
-__device__ __forceinline__ void coarseSerial(const Level<R>& L, unsigned tag, const TagWait& w, R* x) {
+__device__ __forceinline__ void coarseSerial(const Level<R>& L, const R* b, R* x) {
     using T = R;
     for (int I = 0; I < L.n; ++I) x[I] = 0;
     for (int it = 0; it < 20; ++it)
@@ -129,8 +129,7 @@ __device__ __forceinline__ void coarseSerial(const Level<R>& L, unsigned tag, co
                 int I = dir == 0 ? t : L.n - 1 - t;
                 T dg = L.diag[I];
                 if (dg <= 0) { x[I] = 0; continue; }
-                T s = 0;
-                waitFor(w, [&] { return tagLoad(L.b, I, tag, s); });
+                T s = b[I];
                 for (int q = L.rowStart[I]; q < L.rowStart[I + 1]; ++q) s += L.val[q] * x[L.col[q]];
                 x[I] = s / dg;
             }

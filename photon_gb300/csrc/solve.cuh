@@ -32,7 +32,7 @@
 // result is the same bits alone, in any batch and with any number of CTAs.
 //
 // Waits: a team barrier and the reader of a tagged value give up after
-// TEAM_WAIT_CYCLES, record it in the context's error word and end the kernel; the
+// Scn::waitCycles, record it in the context's error word and end the kernel; the
 // launch is cooperative, so all CTAs of a team are resident.
 #pragma once
 #include "mixed_kernels.cuh"
@@ -421,12 +421,12 @@ struct Team {
     int size, rank;          // CTAs, this CTA's place
 };
 
-// every thread of every CTA of the team calls it; false: the wait ran out and
-// the kernel has to end. *gaveUp is shared memory, 0 at first.
+// every thread of every CTA of the team calls it; false, for the whole CTA: a wait ran out
+// and the kernel has to end. *gaveUp and *go are shared memory, *gaveUp 0 at first.
 template <class R>
-__device__ __forceinline__ bool teamSync(const Scn<R>& g, Team& t, volatile int* gaveUp) {
+__device__ __forceinline__ bool teamSync(const Scn<R>& g, Team& t, volatile int* gaveUp, volatile int* go) {
+    if (t.size == 1) return __syncthreads_and(*gaveUp == 0) != 0;
     __syncthreads();
-    if (t.size == 1) return *gaveUp == 0;
     t.target += (unsigned)t.size;
     if (threadIdx.x == 0) {
         unsigned* const bar = g.teamBar;
@@ -437,16 +437,17 @@ __device__ __forceinline__ bool teamSync(const Scn<R>& g, Team& t, volatile int*
             const long long t0 = clock64();
             do {
                 asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(seen) : "l"(bar) : "memory");
-                if (clock64() - t0 > TEAM_WAIT_CYCLES) {
+                if (clock64() - t0 > g.waitCycles) {
                     atomicOr(g.errWord, ERR_TEAM_WAIT);
                     *gaveUp = 1;
                     break;
                 }
             } while ((int)(seen - t.target) < 0);
         }
+        *go = *gaveUp == 0;   // one answer: a fast warp's next wait may run out before a slow one has looked
     }
     __syncthreads();
-    return *gaveUp == 0;
+    return *go != 0;
 }
 
 // ---- sums ----------------------------------------------------------------------
@@ -800,7 +801,7 @@ k_solve(const Scn<R>* __restrict__ S, SolveArgs a) {
     R* const shB = reinterpret_cast<R*>(pool + SolveCfg<R, PER>::ROWS / 4);   // the coarsest right-hand side
     double* const shTerms = reinterpret_cast<double*>(pool + SolveCfg<R, PER>::ROWS / 4);   // FP32: a tile's terms, by turns
     __shared__ double shMx[32];
-    __shared__ int gaveUp;
+    __shared__ int gaveUp, go;
     static_assert(sizeof(Scn<R>) % 8 == 0, "descriptors are copied as 8-byte words");
     const int tid = (int)threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int b = (int)blockIdx.x;
@@ -843,7 +844,7 @@ k_solve(const Scn<R>* __restrict__ S, SolveArgs a) {
         B.p = g.p; B.z = g.z; B.q = g.q; B.r = g.r; B.d = g.d;
         B.dNew = nullptr; B.alpha = T(0); B.beta = T(0); B.haveD = false;
 
-#define PHX_TEAM_SYNC() do { if (!teamSync(g, team, &gaveUp)) return; } while (0)
+#define PHX_TEAM_SYNC() do { if (!teamSync(g, team, &gaveUp, &go)) return; } while (0)
         // one pass over the team's tiles
         const int slot = warp / tl.warps, slots = TH / 32 / tl.warps, wt = warp - slot * tl.warps;
         int turn = 0;
@@ -924,7 +925,7 @@ k_solve(const Scn<R>* __restrict__ S, SolveArgs a) {
                 }
                 __syncwarp();
             }
-        const TagWait tw{&gaveUp, g.errWord};
+        const TagWait tw{&gaveUp, &g.errWord, &g.waitCycles};
         auto inLevel = [](RowSet s) { return s.off >= 0 ? RowSet{~s.off, s.width} : RowSet{-1, -1}; };
         auto jacobiLevel = [&](auto sweep, int l) {
             constexpr int SWEEP = decltype(sweep)::value;
@@ -969,10 +970,17 @@ k_solve(const Scn<R>* __restrict__ S, SolveArgs a) {
                     const T v = coarseDenseRow(L, row, shB);
                     if (lane == 0) put(row, v);
                 }
-            } else if (rank == 0 && tid == 0) {
-                R* const x = L.x;
-                coarseSerial(L, B.tag, tw, x);
-                for (int I = 0; I < L.n; ++I) put(I, x[I]);
+            } else if (rank == 0) {   // yd, which nothing writes at the coarsest level, takes the right-hand side
+                R *const x = L.x, *const rhs = reinterpret_cast<R*>(L.yd);
+                for (int i = tid; i < L.n; i += TH) {
+                    T v = T(0);
+                    waitFor(tw, [&] { return tagLoad(L.b, i, B.tag, v); });
+                    rhs[i] = v;
+                }
+                __syncthreads();
+                if (tid == 0) coarseSerial(L, rhs, x);
+                __syncthreads();
+                for (int I = tid; I < L.n; I += TH) put(I, x[I]);
             }
         };
         // the cells of the grid, elementwise
