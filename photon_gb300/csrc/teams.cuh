@@ -35,9 +35,9 @@ __host__ __device__ inline SolveTiling solveTiling(int nblk) {
 // The CTAs a scenario is given at most: two tiles a CTA cost it nothing where they are a warp
 // each (FP64) or a third of the GPU and more has one (FP32, 36x24x24 room of 81 tiles: 41 / 81 /
 // 152 CTAs 0.476 / 0.482 / 0.494 ms a step; 52x40x32 of 260: 130 / 152 0.526 / 0.537; but 36
-// tiles: 18 / 36 0.403 / 0.383). The grid is no larger than its scenarios can use, so that
-// small contexts run side by side: four closets on four threads 0.10 ms a step, with
-// grids of the whole GPU 0.23, four FP32 rooms 0.12 and 0.30.
+// tiles: 18 / 36 0.403 / 0.383). The rest of the SMs is free for other contexts' solves: four
+// closets on four threads 0.10 ms a step, when every solve bound the whole GPU 0.23; four
+// FP32 rooms 0.15 and 0.30.
 template <class R>
 __host__ __device__ inline int solveCtas(const SolveTiling& t) {
     const int half = (t.nt + 1) / 2;
