@@ -777,10 +777,11 @@ public:
         PHX_TRY(grow(RadWork::SOLIDT, N * sizeof(double)));
         PHX_TRY(grow(RadWork::GAS, N * sizeof(R)));
         PHX_TRY(grow(RadWork::KC, sizeof(RadConst<R>)));
-        PHX_TRY(grow(RadWork::SOURCES, (size_t)nE * sizeof(RadSource<R>)));
-        PHX_TRY(grow(RadWork::RAYS, (size_t)nE * RAD_DIRS * sizeof(RadRay<R>)));
-        PHX_TRY(grow(RadWork::RAYVAL, (size_t)nE * RAD_DIRS * sizeof(R)));
-        PHX_TRY(grow(RadWork::RAYELEM, (size_t)nE * RAD_DIRS * sizeof(int)));
+        const size_t nAt = std::min(nE, RAD_PORTION);   // elements at a time
+        PHX_TRY(grow(RadWork::SOURCES, nAt * sizeof(RadSource<R>)));
+        PHX_TRY(grow(RadWork::RAYS, nAt * RAD_DIRS * sizeof(RadRay<R>)));
+        PHX_TRY(grow(RadWork::RAYVAL, nAt * RAD_DIRS * sizeof(R)));
+        PHX_TRY(grow(RadWork::RAYELEM, nAt * RAD_DIRS * sizeof(int)));
         PHX_TRY(grow(RadWork::CNT, (RAD_DIRS + 1) * sizeof(int)));
         if (!rad.marchCtas) {
             int dev = 0, sms = 0, per = 0;
@@ -819,12 +820,14 @@ public:
                                                                     dKc);
         if (nW) k_rad_walls<R><<<(nW + 127) / 128, 128, 0, st>>>(dWl, nW, nx, ny, nz, dWallOf,
                                                                  reinterpret_cast<unsigned*>(dFlags), dWallI, dKc);
-        if (nE) {
-            k_rad_elems<R><<<(nE + RAD_ELEMS - 1) / RAD_ELEMS, RAD_ELEMS, 0, st>>>(dS, s, dEl, elWords, nE, dKc, dSources, dRays,
-                                                                                   dRayElem, dRayVal, dCnt);
-            k_rad_march<R><<<rad.marchCtas, 256, 0, st>>>(dS, s, nE, dSources, dCells, dFlags, dWallOf, dWallI, dKc,
+        for (long long e0 = 0; e0 < nE; e0 += RAD_PORTION) {
+            const int n = (int)std::min<long long>(nE - e0, RAD_PORTION);
+            if (e0) PHX_CK(cudaMemsetAsync(dCnt, 0, (RAD_DIRS + 1) * sizeof(int), st));
+            k_rad_elems<R><<<(n + RAD_ELEMS - 1) / RAD_ELEMS, RAD_ELEMS, 0, st>>>(dS, s, dEl + e0 * elWords, elWords, n, dKc,
+                                                                                 dSources, dRays, dRayElem, dRayVal, dCnt);
+            k_rad_march<R><<<rad.marchCtas, 256, 0, st>>>(dS, s, n, dSources, dCells, dFlags, dWallOf, dWallI, dKc,
                                                           dRays, dRayElem, dRayVal, dCnt, dGas);
-            k_rad_absorbed<R><<<(nE + 255) / 256, 256, 0, st>>>(dRayVal, nE, dAbs);
+            k_rad_absorbed<R><<<(n + 255) / 256, 256, 0, st>>>(dRayVal, n, dAbs + e0);
         }
         PHX_CK(cudaGetLastError());
         PHX_CK(cudaEventRecord(rad.e1, st));

@@ -36,6 +36,9 @@ namespace phx {
 
 constexpr int RAD_NB = 4, RAD_DIRS = 32;
 constexpr int RAD_ELEMS = 128;      // elements per CTA of k_rad_elems, a thread each
+// elements traced at a time: an element's rays and results take 0.8 KB (FP32) or 1.5 KB of
+// scratch, 420 or 770 MB for this many, however many elements a trace has
+constexpr int RAD_PORTION = 1 << 19;
 constexpr int RAD_EXP_N = 512;      // table of radDecay
 // cells a ray advances before lanes without one take another: an FP64 step costs its warp
 // the same with few lanes as with 32, an FP32 one little against the hand-out (72x52x44
