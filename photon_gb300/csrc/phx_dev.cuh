@@ -82,7 +82,8 @@ enum Slot {
     SV_PITERS, SV_PRES, SV_PREL, SV_HRR, SV_MAXGAST, SV_BURNING, SV_FUELIN, SV_FUELBURNED, SV_FUELINDOMAIN,
     SV_INV,
     SV_HAVEPREV,                 // mixed path: p64prev holds the previous step's pressure
-    SV_SOLVED,                   // a pressure solve has run: SV_PITERS is its iterations
+    SV_SOLVED,                   // a pressure solve has run
+    SV_MEANITERS,                // running mean of the solves' iterations (teams.cuh)
     SV_SRC_MF = 32,              // MAX_SRC injection amounts of this step (-1 = inactive)
     SV_COUNT = 64
 };

@@ -1208,7 +1208,9 @@ k_solve(const Scn<R>* __restrict__ S, SolveArgs a) {
             sv[SV_DQ] = cg.dq;
             sv[SV_RMAX] = 0;
             sv[SV_IT] = sv[SV_PITERS] = cg.it;
-            sv[SV_DONE] = sv[SV_SOLVED] = 1;
+            sv[SV_DONE] = 1;
+            sv[SV_MEANITERS] = sv[SV_SOLVED] > 0 ? sv[SV_MEANITERS] + SOLVE_MEAN_SHARE * (cg.it - sv[SV_MEANITERS]) : cg.it;
+            sv[SV_SOLVED] = 1;
             const double r = kMixed ? cg.r64 : cg.rmax;   // the residual the solve is judged by
             sv[SV_PRES] = r / sv[SV_INV];
             sv[SV_PREL] = sv[SV_BMAX] > 0 ? r / sv[SV_BMAX] : 0.0;

@@ -46,7 +46,7 @@ __host__ __device__ inline int solveCtas(const SolveTiling& t) {
 }
 
 // The grid's CTAs among the scenarios. A scenario has a team of CTAs, in proportion to its
-// work (blocks times the iterations of its last solve), at least one. With many scenarios
+// work (blocks times the iterations its solves take), at least one. With many scenarios
 // beside a large one that would leave the large one a few CTAs, and with more scenarios
 // than CTAs nothing: then scenarios of less work than a CTA's share take turns on a CTA,
 // the largest first. ms per step, a CTA each at least / shared: a 165 k-cell house with 280
@@ -67,11 +67,19 @@ struct TeamTable {
 // 20 k to 1.3 M cells, mixed: 343 M cell-updates/s and 28 ms at the 99th percentile of a
 // step, 292 M and 90 ms with the count of 0).
 constexpr float SOLVE_FIRST_ITERS = 40.0f;
+// After it a running mean of its iterations counts, each solve with this share, and two more.
+// Under the reference's absolute stop counts go up and down (0, 5, 5, 4, 3, 0, ... where the warm
+// start is good enough now and then), and the last one alone gives the solve after a 0 a
+// CTA or two: 64 houses of 20 k to 400 k cells 10.6 ms a step with it, 9.1 with the mean
+// (10.0 when every pass was a launch over all of them), 24 houses 3.80 and 3.55. At a relative
+// stop counts are steady: 24 houses 5.75 ms with either, 8 in FP64 4.31. Mean step of 40
+// to 60; a share of 0.5 and four more are within 1 %.
+constexpr double SOLVE_MEAN_SHARE = 0.3, SOLVE_MORE_ITERS = 2.0;
 template <class R>
 __device__ __forceinline__ int solveBlocks(const Scn<R>& g) { return (int)g.dvL0[1].d * ((g.nz + 1) >> 1); }
 template <class R>
 __device__ __forceinline__ float solveWork(const Scn<R>& g) {
-    return (float)solveBlocks(g) * (g.sv[SV_SOLVED] > 0 ? (float)(g.sv[SV_PITERS] + 2.0) : SOLVE_FIRST_ITERS);
+    return (float)solveBlocks(g) * (g.sv[SV_SOLVED] > 0 ? (float)(g.sv[SV_MEANITERS] + SOLVE_MORE_ITERS) : SOLVE_FIRST_ITERS);
 }
 
 // a scenario's share in the division, from the CTA that begins its step
