@@ -368,7 +368,7 @@ double phx_vol_last_ms(const struct phx_ctx* ctx);
  * kernel records it in the context's device error word and returns, and the
  * next synchronising call reports PHX_ERR_TIMEOUT and clears the word. This
  * call exercises that path on purpose: one thread waits, for limit_ms (at most
- * 1000), on an mbarrier that nothing arrives on. It returns PHX_ERR_TIMEOUT
+ * 1000), for a value that nothing writes. It returns PHX_ERR_TIMEOUT
  * with a message; the context stays usable. No counterpart in the reference. */
 int phx_selftest_wait_timeout(struct phx_ctx* ctx, double limit_ms);
 

@@ -41,7 +41,10 @@ namespace phx {
 // D_FACES, D_BND: the tiles of the x, then the y, then the z faces (boundary sides)
 enum DomId { D_ONE = 0, D_CELLS, D_FACES, D_BND, D_CZ, D_CC, D_LEAK, D_COUNT };
 
-// widest rows the contexts take (nx); wider grids are refused
+// Widest rows the contexts take (nx); wider grids are refused, with PHX_ERR_UNSUPPORTED.
+// What once set these (rows staged in shared memory) is gone, and nothing in the kernels
+// depends on them now; they stay as the limits that callers have been told and that
+// the tests cover, and no wider grid has been run.
 template <class R>
 constexpr int maxRow() { return sizeof(R) == 8 ? 410 : 776; }
 
@@ -631,7 +634,7 @@ public:
     Scn<R>* dS = nullptr;        // descriptors
     int* dDomStart = nullptr;    // D_COUNT x (cap + 1)
     double* dDtMax = nullptr;    // per-scenario dtMax of the step
-    unsigned* dErr = nullptr;    // error word of the device side (bounded waits that ran out)
+    unsigned* dErr = nullptr;    // error word of the device side (bounded waits that ran out); [2..3] stay 0
     unsigned* ownTab = nullptr;  // CTA -> (scenario, tile) of every domain (Dom::owner)
     size_t ownCap = 0;
     double* dTimes = nullptr;    // simulated time of each scenario (read-back staging)
@@ -841,8 +844,6 @@ public:
     }
     double radLastMs() const override { return rad.lastMs; }
 
-    // one bounded wait that nothing satisfies: the failure path a timed-out
-    // copy takes (error word, host report, context still usable)
     // ---- V-cycle schedule autotuner ----------------------------------------------
     // For each size bucket present in the batch (largest total first), every
     // candidate coarsening stop is applied to the bucket's scenarios and the
@@ -964,6 +965,8 @@ public:
         return checkDeviceError();
     }
 
+    // one bounded wait that nothing satisfies: the failure path of a solve's wait that
+    // runs out (error word, host report, context still usable)
     int selftestWait(double limitMs) override {
         if (!(limitMs > 0) || limitMs > 1000) { err = "self-test limit must be in (0, 1000] ms"; return PHX_ERR_INVALID; }
         PHX_TRY(ensureTables());
@@ -972,7 +975,7 @@ public:
         PHX_CK(cudaGetDevice(&dev));
         PHX_CK(cudaDeviceGetAttribute(&khz, cudaDevAttrClockRate, dev));
         const long long cycles = (long long)(limitMs * (double)std::max(khz, 1000000));
-        k_selftest_wait<R><<<1, 32, 0, st>>>(dErr, cycles);
+        k_selftest_wait<R><<<1, 32, 0, st>>>(dErr, reinterpret_cast<const unsigned long long*>(dErr + 2), cycles);
         PHX_CK(cudaGetLastError());
         PHX_CK(cudaStreamSynchronize(st));
         return checkDeviceError();
@@ -1312,9 +1315,9 @@ public:
             // report once and clear, so that the context stays usable
             PHX_CK(cudaMemsetAsync(dErr, 0, sizeof(unsigned), st));
             PHX_CK(cudaStreamSynchronize(st));
-            err = (w & ERR_TEAM_WAIT) ? "a CTA of the pressure solve waited too long for its team; the step's results are not "
-                             "valid (device error word " + std::to_string(w) + ")"
-                                        : "a bounded device wait ran out (self-test, device error word " + std::to_string(w) + ")";
+            err = (w & ERR_SELFTEST) ? "a bounded device wait ran out (self-test, device error word " + std::to_string(w) + ")"
+                                     : "a CTA of the pressure solve waited too long for its team; the step's results are not "
+                                       "valid (device error word " + std::to_string(w) + ")";
             return PHX_ERR_TIMEOUT;
         }
         return PHX_OK;

@@ -8,7 +8,6 @@
 // with CTA b of the launch mapped to (scenario, tile) by a prefix table.
 #pragma once
 #include <cstdint>
-#include <cuda_fp16.h>
 #include <cuda_runtime.h>
 
 namespace phx {
@@ -78,8 +77,7 @@ constexpr int MAX_BATCH = 1024;  // scenarios per batch (the persistent kernels 
 // scalar slots of a scenario (double each)
 enum Slot {
     SV_DTMAX_ARG = 0, SV_DT, SV_TIME, SV_MAXVEL, SV_MAXNU, SV_MAXDIV,
-    SV_RZ, SV_ALPHA, SV_BETA, SV_RMAX, SV_BMAX, SV_IT, SV_DONE, SV_DQ,
-    SV_PITERS, SV_PRES, SV_PREL, SV_HRR, SV_MAXGAST, SV_BURNING, SV_FUELIN, SV_FUELBURNED, SV_FUELINDOMAIN,
+    SV_RMAX, SV_BMAX, SV_IT, SV_PRES, SV_PREL, SV_HRR, SV_MAXGAST, SV_BURNING, SV_FUELIN, SV_FUELBURNED, SV_FUELINDOMAIN,
     SV_INV,
     SV_HAVEPREV,                 // mixed path: p64prev holds the previous step's pressure
     SV_SOLVED,                   // a pressure solve has run
@@ -335,8 +333,6 @@ __device__ __forceinline__ double f2value(F2 v) { return (double)v.hi + (double)
 // one term of a dot product in the accumulator of the arithmetic type
 __device__ __forceinline__ double dotTerm(double a, double b) { return a * b; }
 __device__ __forceinline__ F2 dotTerm(float a, float b) { return f2prod(a, b); }
-__device__ __forceinline__ double accAdd(double a, double b) { return a + b; }
-__device__ __forceinline__ F2 accAdd(F2 a, F2 b) { return f2add(a, b); }
 
 __device__ __forceinline__ F2 warpSum(F2 v) {
     for (int o = 16; o > 0; o >>= 1) {

@@ -1205,13 +1205,7 @@ k_solve(const Scn<R>* __restrict__ S, SolveArgs a) {
             });
         if (rank == 0 && tid == 0) {
             double* sv = g.sv;
-            sv[SV_RZ] = cg.rz;
-            sv[SV_ALPHA] = cg.alpha;
-            sv[SV_BETA] = cg.beta;
-            sv[SV_DQ] = cg.dq;
-            sv[SV_RMAX] = 0;
-            sv[SV_IT] = sv[SV_PITERS] = cg.it;
-            sv[SV_DONE] = 1;
+            sv[SV_IT] = cg.it;
             sv[SV_MEANITERS] = sv[SV_SOLVED] > 0 ? sv[SV_MEANITERS] + SOLVE_MEAN_SHARE * (cg.it - sv[SV_MEANITERS]) : cg.it;
             sv[SV_SOLVED] = 1;
             const double r = kMixed ? cg.r64 : cg.rmax;   // the residual the solve is judged by
