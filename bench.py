@@ -96,23 +96,22 @@ def make_workload(name: str):
     return c
 
 
-# Algorithmic bytes per unit of each kernel's domain for storage width w
-# (8 for FP64 fields, 4 for the mixed path): each input array read once and
-# each output written once per launch; uint8 masks count 1 B, int32 maps 4 B.
-# The mixed path's level-0 kernels read one coefficient-code byte per cell in
-# place of the diagonal and the three coefficient arrays.
+# Algorithmic bytes per cell of each kernel for storage width w (8 for FP64
+# fields, 4 for the mixed path): each input array read once and each output
+# written once per launch; uint8 masks count 1 B. A kernel over the faces of all
+# three axes reads and writes three face arrays per cell.
 def kernel_bytes(name: str, w: int):
     table = {
         "k_advect": 18 * w + 1 + 10 * w,        # 10 scalars + u,v,w + fx,fy,fz + Pb,nu + blocked -> 10 scalars
-        "k_momentum": 9 * w,                    # vel, 2 other components, fo, Pb, T, nu, p -> vel' (per face)
+        "k_momentum": 27 * w,                   # per face: vel, 2 other components, fo, Pb, T, nu, p -> vel'
         "k_rhs": 13 * w + 1,
         "k_heat": 8 * w + 1,
         "k_energy": 6 * w + 1,
         "k_combust": 6 * w + 3,
-        "k_turb_filter": 6 * w + 1,             # three components along one axis -> three components
-        "k_turb_center": 6 * w + 1,
-        "k_turb_nu": 5 * w + 1,
-        "k_velcorr": 5 * w,
+        "k_turb_x": 9 * w + 1,                  # u, v, w -> three centre velocities, three filtered ones
+        "k_turb_y": 6 * w + 1,                  # three filtered components -> three
+        "k_turb_nu": 8 * w + 1,                 # three of either kind, T -> nu
+        "k_velcorr": 15 * w,                    # per face: vel, fo, a, p -> vel'
         "k_stats": 4 * w + 1,
     }
     return table.get(name)

@@ -72,7 +72,7 @@ __host__ __device__ __forceinline__ constexpr double tKFromStoredd(double s) { r
 constexpr int MAX_SRC = 16;      // burners + ignitions per scenario
 constexpr int MAX_LEVELS = 12;   // multigrid levels (the reference's cap)
 constexpr int TPB = 256;         // threads per CTA of the cell/face kernels
-constexpr int MAX_BATCH = 1024;  // scenarios per batch (the persistent kernels keep their table in shared memory)
+constexpr int MAX_BATCH = 1024;  // scenarios per batch (the division into teams keeps their work in shared memory)
 
 // scalar slots of a scenario (double each)
 enum Slot {

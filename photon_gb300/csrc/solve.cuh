@@ -1019,7 +1019,7 @@ k_solve(const Scn<R>* __restrict__ S, SolveArgs a) {
         auto zoneCenter = [&](R* v) {
             zones(v, [&](int c, double mean) { v[c] = (R)((double)v[c] - mean); });
         };
-        // mixed path: r = b - A p64 in FP64 (k_mx_res64's expressions), p = 0; closed
+        // mixed path: r = b - A p64 in FP64 from the FP32 right-hand side and coefficients, p = 0; closed
         // zones: the zone mean of r removed
         auto residual64 = [&](double& rm) {
             const int nx = g.nx, ny = g.ny, nz = g.nz, sxy = nx * ny;

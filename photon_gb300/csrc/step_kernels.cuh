@@ -1,13 +1,15 @@
 // CUDA kernels of the gas-phase step (all stages except the pressure solve).
 //
 // Each kernel is one pass of the reference's step over one domain of every
-// scenario in a launch; the arithmetic of every cell or face restates the
-// reference expression in its own evaluation order (the FP64 build is compiled
-// with --fmad=false so no multiply-add is fused), which keeps the FP64 path
-// within rounding of the reference's own FP64 step. Reductions that the
-// reference sums in a fixed order are summed here in a fixed order as well:
-// per-CTA partials, then the last CTA of a scenario sums the partials in CTA
-// order, so results do not depend on scheduling.
+// scenario in a launch. Combustion, energy, leakage, the right-hand side and the
+// velocity correction restate the reference's expressions in their evaluation order
+// (the FP64 build is compiled with --fmad=false so no multiply-add is fused). FP64
+// momentum, heat diffusion, viscosity and transport, which the FP64 pipe bounds, are in
+// FMA form with reordered terms, shared divisions and short powers, each stated
+// where it stands; a step stays within 5e-14 of the reference order's, relative to a
+// field's norm. Reductions that the reference sums in a fixed order are summed here
+// in a fixed order as well: per-CTA partials, then the last CTA of a scenario sums
+// the partials in CTA order, so results do not depend on scheduling.
 #pragma once
 #include "teams.cuh"
 
