@@ -421,23 +421,28 @@ struct Scenario {
         if (stop == coarseStop && mgArena) return PHX_OK;
         Multigrid M = buildMultigrid(geo, DENSE_MAX, stop, coarseSolveFor());
         PHX_CK(cudaStreamSynchronize(st));
-        char* old = mgArena;
-        MG = std::move(M);
-        coarseStop = stop;
+        std::vector<RowSets> oldSets = std::move(rowSets);
+        std::swap(MG, M);
         buildRowSets();
-        mgBytes = layoutLevels(nullptr);
+        const size_t bytes = layoutLevels(nullptr);
         char* fresh = nullptr;
-        if (cudaMalloc(&fresh, mgBytes) != cudaSuccess) {
+        if (cudaMalloc(&fresh, bytes) != cudaSuccess) {   // the former hierarchy stays
             cudaGetLastError();
+            std::swap(MG, M);
+            rowSets = std::move(oldSets);
+            layoutLevels(mgArena);
             err = "device allocation of the multigrid levels failed";
             return PHX_ERR_OOM;
         }
+        char* const old = mgArena;
+        coarseStop = stop;
         mgArena = fresh;
+        mgBytes = bytes;
         arenaBytes = mainBytes + TAIL_BYTES + mgBytes;
         layoutLevels(mgArena);
-        PHX_TRY(uploadLevels(st));
+        const int r = uploadLevels(st);
         if (old) cudaFree(old);
-        return PHX_OK;
+        return r;
     }
 
     template <class T>
@@ -955,7 +960,8 @@ public:
             std::lock_guard<std::mutex> lock(vcycleMutex());
             vcycleTable()[b] = best;
         }
-        if (r == PHX_OK) r = copyState(false);
+        const int back = copyState(false);   // also after a failure: the trials have stepped the fields
+        if (r == PHX_OK) r = back;
         restoreHost();
         tablesDirty = true;
         cudaStreamSynchronize(st);
