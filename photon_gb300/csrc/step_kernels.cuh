@@ -7,9 +7,10 @@
 // momentum, heat diffusion, viscosity and transport, which the FP64 pipe bounds, are in
 // FMA form with reordered terms, shared divisions and short powers, each stated
 // where it stands; after 6 to 20 steps fields are within 5e-14 of the reference order's,
-// relative to their norm, on buildings, and within 2e-13 on a 200x9x7 duct. Reductions that the reference sums in a fixed order are summed here
-// in a fixed order as well: per-CTA partials, then the last CTA of a scenario sums
-// the partials in CTA order, so results do not depend on scheduling.
+// relative to their norm, on buildings, and within 2e-13 on a 200x9x7 duct.
+// Reductions that the reference sums in a fixed order are summed here in a fixed
+// order as well: per-CTA partials, then the last CTA of a scenario sums the
+// partials in CTA order, so results do not depend on scheduling.
 #pragma once
 #include "teams.cuh"
 
